@@ -18,6 +18,7 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <span>
 #include <stdexcept>
 #include <string>
@@ -33,6 +34,7 @@
 #include "flow.h"
 #include "graph.h"
 #include "kernels.h"
+#include "resident.h"
 #include "solve.h"
 #include "step.h"
 #include "mlp.h"
@@ -548,6 +550,12 @@ struct msb_context {
   msb::DBuf<std::uint32_t> inc_offsets;
   msb::DBuf<float4> inc_a, inc_b, resp_a, resp_b, accepted_a, accepted_b;
   msb::DBuf<float2> inc_constants, inc_sides;  // per row: (offset, compliance), the two side terms
+  msb::DBuf<std::uint32_t> inc_places;         // per side: its entry's place
+  // The resident solve: each entry's slot, and the grid form's words.
+  std::optional<msb::ResidentLimits> resident_limits;
+  msb::DBuf<std::uint32_t> resident_slots;
+  msb::DBuf<unsigned long long> resident_inbox;
+  msb::DBuf<ulonglong2> resident_records;
   msb::DBuf<float> slack;
 
   // A batch of independent colonies (msb_advance_contact_dynamics_batch);
@@ -1188,7 +1196,7 @@ bool use_fused_relaxation(Ctx& c, std::uint32_t items) {
 }
 
 IncidenceArrays incidence_arrays(Ctx& c) {
-  return {c.inc_offsets.p, c.inc_a.p, c.inc_b.p, c.inc_constants.p, c.inc_sides.p};
+  return {c.inc_offsets.p, c.inc_a.p, c.inc_b.p, c.inc_constants.p, c.inc_sides.p, c.inc_places.p};
 }
 
 void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_response& growth, float tolerance,
@@ -1229,6 +1237,7 @@ void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_
     d.barrier_generation = 0;
     d.barrier_abort = 0;
     d.check_status = 0;
+    d.misfit = 0;
     check(cudaMemcpyAsync(c.desc, &d, sizeof(SolveDesc), cudaMemcpyHostToDevice, c.stream), "desc");
     return;
   }
@@ -1243,6 +1252,7 @@ void build_system_incidence(Ctx& c, std::uint32_t row_count) {
   c.inc_b.ensure(entries);
   c.inc_constants.ensure(entries / 2);
   c.inc_sides.ensure(entries / 2);
+  c.inc_places.ensure(entries);
   c.sort_keys.ensure(entries);
   c.sort_values.ensure(entries);
   c.counts.ensure(c.n + 1ull);
@@ -1265,6 +1275,27 @@ void build_row_keys(Ctx& c, RowStore& store) {
 // incidence of c.rows and the bodies.
 SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growth, std::uint32_t max_iterations);
 
+// The solve with the system in shared memory, in one launch; c.host_desc
+// holds its report.  False, with nothing done, when a share does not fit.
+bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_response& growth, float tolerance,
+                    std::uint32_t max_iterations) {
+  c.resident_slots.ensure(2ull * c.rows.count);
+  if (plan.grid) {
+    c.resident_inbox.ensure(std::size_t(resident_stride()) * kResidentMaxCtas);
+    c.resident_records.ensure(2ull * kResidentRecords * kResidentWords);
+  }
+  fill_desc(c, c.rows.count, dt, growth, tolerance, max_iterations, true);
+  const ResidentArrays arrays{c.inc_places.p, c.resident_slots.p, c.resident_inbox.p, c.resident_records.p,
+                              resident_stride()};
+  check(cudaError_t(launch_resident(*c.host_desc, c.desc, arrays, plan, c.stream)), "solve launch");
+  check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
+  sync(c);
+  if (c.host_desc->barrier_abort != 0) throw DeviceCheckError("a wait of the resident solve ran out of time");
+  if (c.host_desc->check_status != 0) throw DeviceCheckError("an index check of the resident solve failed");
+  c.last_blocks = grid_for(std::max(c.rows.count, c.n), kSolveThreads, 4);
+  return c.host_desc->misfit == 0;
+}
+
 SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, float tolerance,
                    std::uint32_t max_iterations) {
   if (c.colonies > 0) return solve_batch(c, dt, growth, max_iterations);
@@ -1277,6 +1308,16 @@ SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, flo
     return {};
   }
   c.partials.ensure(5ull * kMaxPassBlocks);
+  if (c.relaxation == 0) {
+    if (!c.resident_limits) c.resident_limits = resident_limits();
+    const ResidentPlan plan = resident_plan(*c.resident_limits, rows, c.n);
+    if (plan.ctas > 0 && solve_resident(c, plan, dt, growth, tolerance, max_iterations)) {
+      const SolveDesc& d = *c.host_desc;
+      c.solve_log.push_back({rows, d.iterations, d.status, d.residual});
+      if (d.status == 3) throw std::invalid_argument("contact system has no positive diagonal");
+      return {d.status, d.iterations, d.residual};
+    }
+  }
   const bool fused = use_fused_relaxation(c, std::max(rows, c.n));
   if (fused) {
     // One cooperative launch runs the whole solve (relax_kernel).

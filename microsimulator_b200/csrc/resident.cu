@@ -1,0 +1,925 @@
+// The Barzilai-Borwein contact solve with the system resident in shared
+// memory: one launch runs the bound, the initial gaps and every projected
+// iteration, and between iterations nothing but side terms and sums moves.
+//
+// Each CTA holds a contiguous range of bodies and those bodies' incidence
+// entries: the jacobian and lever, the row's offset and compliance, and the
+// row's (multiplier, gap).  Both bodies of a row keep its multiplier and gap
+// and update them with the same operations, so an iteration is
+//   send     per body: project its entries' multipliers, sum their wrenches
+//            in entry order (the reference's row order), respond, and send
+//            each entry's side term of the gap rate to the row's other entry;
+//   receive  per entry: own term + received term -> the new gap; the BB
+//            products and the residual (rows counted on their first side).
+// The arithmetic is that of the two-pass solve (solve.cu), term by term; only
+// the FP64 products are summed in another fixed order.
+//
+// Three forms by size.  One CTA: block barriers.  One cluster: side terms go
+// through distributed shared memory, with two hardware cluster barriers per
+// iteration.  The whole grid (a cooperative launch): a term for another CTA
+// is one 64-bit word (round, value) in that CTA's global inbox, which its
+// owner polls; the sums are words of the same kind that every CTA reads and
+// adds in CTA order, so no CTA waits for another's decision and no grid
+// barrier is needed.  Every wait is bounded (kWaitPolls).
+#include "resident.h"
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <type_traits>
+#include <cstdint>
+
+#include "device.cuh"
+#include "kernels.h"
+#include "solve_math.cuh"
+#include "../../include/msb200.h"
+
+namespace cg = cooperative_groups;
+
+namespace msb {
+namespace {
+
+constexpr int kThreads = 512;
+constexpr int kWarps = kThreads / 32;
+constexpr std::uint32_t kGroup = 8;    // bodies whose entries are interleaved
+constexpr std::uint32_t kClasses = 64;  // degree classes of the stable sort
+// Shared bytes of an entry (jacobian and lever 32, constants and iterate 16,
+// own and received term 8, list of the remote ones 2) and of a body
+// (record 32, index 2, degree 1, share of the group offsets).
+constexpr std::uint32_t kEntryBytes = 58;
+constexpr std::uint32_t kBodyBytes = 36;
+constexpr std::uint32_t kNobody = 0xFFFFFFFFu;  // a constraint row's entry sends nothing
+constexpr std::uint32_t kRemote = 0x80000000u;
+
+enum Form { kSingle, kCluster, kGrid };
+enum Round { kBound, kInitial, kIterate, kFinal };
+
+struct Sums {
+  double v[3];          // ss, sy, yy
+  std::uint32_t bits;   // largest residual (or bound) as float bits; a NaN's when a gap is not finite
+};
+
+struct Shared {
+  std::uint16_t histogram[kWarps][kClasses];
+  std::uint32_t class_base[kClasses];
+  Sums warp[16];   // each warp's sums
+  Sums parts[16];  // the cluster's, written by its CTAs
+  float alpha;
+  int round;
+  std::uint32_t misfit;
+  std::uint32_t remote_count;
+  std::uint32_t slots;
+  std::uint32_t inbox_at;     // shared address of this CTA's inbox
+  std::uint32_t inboxes[16];  // and of every CTA's of the cluster
+};
+
+extern __shared__ __align__(16) unsigned char resident_memory[];
+
+// Where a CTA's arrays lie in its dynamic shared memory.
+struct Layout {
+  std::uint32_t a_at, b_at, c_at, own_at, inbox_at, remote_at;       // by slot
+  std::uint32_t body_a_at, body_b_at, body_at, degree_at, group_at;  // by body, by group
+  std::uint32_t bodies;
+  std::uint32_t slots;
+  std::uint32_t first;  // the CTA's first body
+
+  template <class T>
+  __device__ __forceinline__ static T& at(std::uint32_t offset, std::uint32_t i) {
+    return reinterpret_cast<T*>(resident_memory + offset)[i];
+  }
+  __device__ __forceinline__ float4& a(std::uint32_t j) const { return at<float4>(a_at, j); }
+  // Jacobian 4, 5, lever, where this entry's term goes.
+  __device__ __forceinline__ float4& b(std::uint32_t j) const { return at<float4>(b_at, j); }
+  // Offset, compliance (sign bit: the row's first side), multiplier, gap.
+  __device__ __forceinline__ float4& c(std::uint32_t j) const { return at<float4>(c_at, j); }
+  __device__ __forceinline__ float& own(std::uint32_t j) const { return at<float>(own_at, j); }
+  __device__ __forceinline__ float& inbox(std::uint32_t j) const { return at<float>(inbox_at, j); }
+  __device__ __forceinline__ std::uint16_t& remote(std::uint32_t x) const { return at<std::uint16_t>(remote_at, x); }
+  __device__ __forceinline__ float4& body_a(std::uint32_t q) const { return at<float4>(body_a_at, q); }
+  __device__ __forceinline__ float4& body_b(std::uint32_t q) const { return at<float4>(body_b_at, q); }
+  __device__ __forceinline__ std::uint16_t& body(std::uint32_t q) const { return at<std::uint16_t>(body_at, q); }
+  __device__ __forceinline__ std::uint8_t& degree(std::uint32_t q) const { return at<std::uint8_t>(degree_at, q); }
+  // First slot of each kGroup bodies.
+  __device__ __forceinline__ std::uint32_t& group(std::uint32_t g) const { return at<std::uint32_t>(group_at, g); }
+};
+
+// Body q's slots are base_of(q) + kGroup * k, k below its degree; up to its
+// group's depth they are padding: zeros that send nothing.
+__device__ __forceinline__ std::uint32_t base_of(const Layout& l, std::uint32_t q) {
+  return l.group(q / kGroup) + q % kGroup;
+}
+__device__ __forceinline__ std::uint32_t depth_of(const Layout& l, std::uint32_t q) {
+  return l.degree(q - q % kGroup);
+}
+__device__ __forceinline__ void pad_slot(const Layout& l, std::uint32_t j) {
+  l.a(j) = l.c(j) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  l.b(j) = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(kNobody));
+  l.own(j) = l.inbox(j) = 0.0f;
+}
+
+// A wait gives up after this many polls (each a trip to L2, about half a
+// microsecond: some seconds).
+constexpr std::uint32_t kWaitPolls = 1u << 23;
+__device__ __forceinline__ void put_word(unsigned long long* p, std::uint32_t tag, std::uint32_t value) {
+  const unsigned long long w = (static_cast<unsigned long long>(tag) << 32) | value;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ unsigned long long get_word(const unsigned long long* p) {
+  unsigned long long w;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+  return w;
+}
+// A double and a 32-bit value with their round as one 128-bit word.
+__device__ __forceinline__ void put_wide(ulonglong2* p, std::uint32_t tag, std::uint32_t bits, double v) {
+  const unsigned long long hi = (static_cast<unsigned long long>(tag) << 32) | bits;
+  asm volatile(
+      "{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+      "l"(__double_as_longlong(v)), "l"(hi)
+      : "memory");
+}
+__device__ __forceinline__ ulonglong2 get_wide(const ulonglong2* p) {
+  ulonglong2 w;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+               : "=l"(w.x), "=l"(w.y)
+               : "l"(p)
+               : "memory");
+  return w;
+}
+// Waits until *p carries `tag`; false once the wait has run out.
+__device__ __forceinline__ bool wait_word(const unsigned long long* p, std::uint32_t tag, unsigned long long& word) {
+  for (std::uint32_t polls = 0; std::uint32_t(word >> 32) != tag; ++polls) {
+    if (polls == kWaitPolls) return false;
+    word = get_word(p);
+  }
+  return true;
+}
+
+__device__ __forceinline__ std::uint32_t cluster_address(std::uint32_t local, std::uint32_t rank) {
+  std::uint32_t out;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(local), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ void cluster_store(std::uint32_t address, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(address), "f"(v) : "memory");
+}
+
+__device__ __forceinline__ std::uint64_t weight(const std::uint32_t* offsets, std::uint32_t b0, std::uint32_t b) {
+  return std::uint64_t(kEntryBytes) * (offsets[b] - offsets[b0]) + std::uint64_t(kBodyBytes) * (b - b0);
+}
+// The first body of [b0, b1] whose weight reaches `target` (block-wide).
+__device__ std::uint32_t find_split(const std::uint32_t* offsets, std::uint32_t b0, std::uint32_t b1,
+                                    std::uint64_t target) {
+  std::uint32_t lo = b0, hi = b1;
+  while (lo < hi) {
+    const std::uint32_t step = (hi - lo + kThreads - 1) / kThreads;
+    const std::uint64_t p = std::uint64_t(lo) + std::uint64_t(threadIdx.x) * step;
+    const int below = __syncthreads_count(p < hi && weight(offsets, b0, std::uint32_t(p)) < target);
+    if (below == 0) return lo;
+    const std::uint32_t last = lo + std::uint32_t(below - 1) * step;
+    hi = smin<std::uint64_t>(hi, std::uint64_t(last) + step);
+    lo = last + 1;
+  }
+  return lo;
+}
+
+template <int kForm>
+struct Comm {
+  std::uint32_t rank, size;
+  const ResidentArrays* arrays;
+  std::uint32_t round = 0;
+
+  __device__ void sync_all() const {
+    if constexpr (kForm == kCluster) {
+      cg::this_cluster().sync();
+    } else {
+      __syncthreads();
+    }
+  }
+  // Sends a side term to the entry that meta names.
+  __device__ __forceinline__ void send(const Layout& l, std::uint32_t meta, float value) const {
+    if (meta == kNobody) return;
+    if constexpr (kForm == kSingle) {
+      l.inbox(meta) = value;
+    } else if constexpr (kForm == kCluster) {
+      cluster_store(meta, value);
+    } else {
+      if (meta & kRemote) {
+        put_word(arrays->inbox + (meta & ~kRemote), round, __float_as_uint(value));
+      } else {
+        l.inbox(meta) = value;
+      }
+    }
+  }
+  // Every term sent in this round is in its inbox on return.
+  __device__ bool exchange(const Layout& l, const Shared& s) const {
+    if constexpr (kForm != kGrid) {
+      sync_all();
+      return true;
+    } else {
+      const unsigned long long* words = arrays->inbox + std::size_t(rank) * arrays->stride;
+      bool late = false;
+      constexpr int kFlight = 4;
+      for (std::uint32_t x0 = threadIdx.x; x0 < s.remote_count; x0 += kFlight * kThreads) {
+        unsigned long long w[kFlight];
+        std::uint32_t slot[kFlight];
+#pragma unroll
+        for (int t = 0; t < kFlight; ++t) {
+          const std::uint32_t x = x0 + t * kThreads;
+          if (x < s.remote_count) {
+            slot[t] = l.remote(x);
+            w[t] = get_word(words + slot[t]);
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < kFlight; ++t) {
+          if (x0 + t * kThreads < s.remote_count) {
+            late = !wait_word(words + slot[t], round, w[t]) || late;
+            l.inbox(slot[t]) = __uint_as_float(std::uint32_t(w[t]));
+          }
+        }
+        if (late) break;
+      }
+      return __syncthreads_or(late) == 0;
+    }
+  }
+};
+
+// Sums over a warp in a fixed tree: ss in lanes 0-7, sy in lanes 8-15, yy in
+// lanes 16-23 of the result, and the largest bits in every lane.  Halving the
+// values with the lanes takes 6 double shuffles, not the 15 of three trees.
+__device__ __forceinline__ double fold_warp(const Sums& x, std::uint32_t& bits) {
+  const std::uint32_t lane = threadIdx.x & 31u;
+  const bool upper = (lane & 16u) != 0u, odd = (lane & 8u) != 0u;
+  double p = (upper ? x.v[2] : x.v[0]) + __shfl_xor_sync(0xFFFFFFFFu, upper ? x.v[0] : x.v[2], 16);
+  const double q = __shfl_xor_sync(0xFFFFFFFFu, x.v[1], 16);
+  const double r = upper ? 0.0 : x.v[1] + q;
+  p = (odd ? r : p) + __shfl_xor_sync(0xFFFFFFFFu, odd ? p : r, 8);
+  for (int o = 4; o > 0; o >>= 1) p += __shfl_xor_sync(0xFFFFFFFFu, p, o);
+  bits = __reduce_max_sync(0xFFFFFFFFu, x.bits);
+  return p;
+}
+// The same of 16 records in shared memory, and its totals in every lane.
+__device__ __forceinline__ Sums fold_records(const Sums* records) {
+  const std::uint32_t lane = threadIdx.x & 31u, k = lane >> 3, i = lane & 7u;
+  double p = k < 3u ? records[i].v[k] + records[i + 8].v[k] : 0.0;
+  for (int o = 4; o > 0; o >>= 1) p += __shfl_xor_sync(0xFFFFFFFFu, p, o);
+  const std::uint32_t bits = __reduce_max_sync(0xFFFFFFFFu, lane < 16u ? records[lane].bits : 0u);
+  return {{__shfl_sync(0xFFFFFFFFu, p, 0), __shfl_sync(0xFFFFFFFFu, p, 8), __shfl_sync(0xFFFFFFFFu, p, 16)}, bits};
+}
+
+constexpr std::uint32_t kFan = 12;  // CTAs a group of the grid form's reduction
+static_assert((kResidentMaxCtas + kFan - 1) / kFan <= 32 && kFan <= 32, "a warp reads a group's records, and the groups'");
+static_assert(kWarps <= 16, "fold_records reads 16 records");
+// Records of two alternating sets: a CTA writes a set again only after every
+// CTA has read the other, and so has read this one.
+__device__ __forceinline__ ulonglong2* record_at(const Comm<kGrid>& comm, std::uint32_t index) {
+  return comm.arrays->records + (std::size_t(comm.round & 1u) * kResidentRecords + index) * kResidentWords;
+}
+// fold_warp's sums as the record `index` (the whole warp).
+__device__ __forceinline__ void put_record(const Comm<kGrid>& comm, std::uint32_t index, double p, std::uint32_t bits) {
+  const std::uint32_t lane = threadIdx.x & 31u;
+  if ((lane & 7u) == 0u && lane < 24u) put_wide(record_at(comm, index) + lane / 8, comm.round, bits, p);
+}
+__device__ __forceinline__ bool get_record(const Comm<kGrid>& comm, std::uint32_t index, Sums& x) {
+  const ulonglong2* from = record_at(comm, index);
+  ulonglong2 w[3];
+  const auto there = [&] {
+    bool all = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      w[k] = get_wide(from + k);
+      all = all && std::uint32_t(w[k].y >> 32) == comm.round;
+    }
+    return all;
+  };
+  for (std::uint32_t polls = 0; !there(); ++polls) {
+    if (polls == kWaitPolls) return false;
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) x.v[k] = __longlong_as_double(static_cast<long long>(w[k].x));
+  x.bits = std::uint32_t(w[0].y);
+  return true;
+}
+
+// The sums of every CTA, in a fixed order: in every thread, in the grid form
+// in warp 0.  False (grid form, in some lanes) once a wait has run out.
+template <int kForm>
+__device__ __forceinline__ bool reduce(const Comm<kForm>& comm, Shared& s, Sums& x) {
+  const std::uint32_t lane = threadIdx.x & 31u;
+  std::uint32_t bits;
+  double p = fold_warp(x, bits);
+  if ((lane & 7u) == 0u) {
+    Sums& to = s.warp[threadIdx.x >> 5];
+    if (lane < 24u) {
+      to.v[lane / 8] = p;
+    } else {
+      to.bits = bits;
+    }
+  }
+  __syncthreads();
+  if constexpr (kForm == kSingle) {
+    x = fold_records(s.warp);
+  } else if constexpr (kForm == kCluster) {
+    if (threadIdx.x < 32) {
+      x = fold_records(s.warp);
+      if (lane < comm.size) *cg::this_cluster().map_shared_rank(&s.parts[comm.rank], lane) = x;
+    }
+    comm.sync_all();
+    x = fold_records(s.parts);
+  } else if (threadIdx.x < 32) {
+    // Two hops: every kFan-th CTA adds its group's records, and every CTA
+    // adds the groups' sums.
+    bool late = false;
+    const std::uint32_t groups = (comm.size + kFan - 1) / kFan;
+    const std::uint32_t leader = comm.rank - comm.rank % kFan;
+    const std::uint32_t members = smin<std::uint32_t>(comm.size - leader, kFan);
+    x = fold_records(s.warp);
+    if (comm.rank != leader) {
+      put_record(comm, comm.rank, lane < 8u ? x.v[0] : lane < 16u ? x.v[1] : x.v[2], x.bits);
+    } else {
+      if (lane > 0) x = Sums{{0.0, 0.0, 0.0}, 0u};
+      if (lane > 0 && lane < members) late = !get_record(comm, leader + lane, x);
+      p = fold_warp(x, bits);
+      put_record(comm, kResidentMaxCtas + leader / kFan, p, bits);
+    }
+    x = Sums{{0.0, 0.0, 0.0}, 0u};
+    if (lane < groups) late = !get_record(comm, kResidentMaxCtas + lane, x) || late;
+    p = fold_warp(x, bits);
+    x = Sums{{__shfl_sync(0xFFFFFFFFu, p, 0), __shfl_sync(0xFFFFFFFFu, p, 8), __shfl_sync(0xFFFFFFFFu, p, 16)}, bits};
+    return !late;
+  }
+  return true;
+}
+
+// A body's wrench and load over its entries in entry order, the body's
+// response, and its entries' side terms on their way (kFinal: the response
+// written instead), by P lanes per body.  A padding entry or a zero
+// multiplier adds +-0 to sums that start at +0, which leaves their bits as
+// skipping it would.
+//
+// P = 1: one thread sums all seven components.  P > 1, for CTAs with few
+// bodies: each lane sums 8 / P of the components, each still in entry order,
+// the lanes exchange them, and the side terms are dealt out entry by entry.
+template <int P, int kForm>
+__device__ __forceinline__ void send_sides(const SolveDesc& d, const Layout& l, const Comm<kForm>& comm, int round,
+                                           float alpha) {
+  constexpr std::uint32_t kPass = kThreads / P;  // bodies a pass
+  constexpr int kShare = 8 / P;                  // components a lane
+  const std::uint32_t lane = threadIdx.x % P;
+  const bool project = round == kIterate;
+#pragma unroll 1
+  for (std::uint32_t q0 = 0; q0 < l.bodies; q0 += kPass) {
+    // Lanes past the last body repeat it (P > 1: the warp exchanges sums).
+    const std::uint32_t at = q0 + threadIdx.x / P;
+    if (P == 1 && at >= l.bodies) break;
+    const std::uint32_t q = smin(at, l.bodies - 1);
+    const std::uint32_t depth = depth_of(l, q);
+    const std::uint32_t base = base_of(l, q);
+    const float4 ba = l.body_a(q);
+    const float4 bb = l.body_b(q);
+    float v[6] = {};
+    float rate = 0.0f;
+    if (round != kBound) {
+      float w[8] = {};
+      if constexpr (P == 1) {
+#pragma unroll 1
+        for (std::uint32_t k = 0; k < depth; ++k) {
+          const std::uint32_t j = base + kGroup * k;
+          const float4 ea = l.a(j), eb = l.b(j), c = l.c(j);
+          const float m = project ? smax(0.0f, c.z - alpha * c.w) : c.z;
+          w[0] += m * ea.x;
+          w[1] += m * ea.y;
+          w[2] += m * ea.z;
+          w[3] += m * ea.w;
+          w[4] += m * eb.x;
+          w[5] += m * eb.y;
+          w[6] += eb.z * m;
+        }
+      } else {
+        const std::uint32_t half = lane / (P / 2);              // 0: components 0-3 (a), 1: 4-6 (b)
+        const std::uint32_t part = (lane % (P / 2)) * kShare;   // first component within it
+        const std::uint32_t from = (half != 0u ? l.b_at : l.a_at) / (4 * kShare) + part / kShare;
+        float mine[kShare] = {};
+#pragma unroll 2
+        for (std::uint32_t k = 0; k < depth; ++k) {
+          const std::uint32_t j = base + kGroup * k;
+          const float2 c = Layout::at<float2>(l.c_at, 2 * j + 1);
+          float jac[kShare];
+          if constexpr (P == 4) {
+            const float2 t = Layout::at<float2>(0, from + 2 * j);
+            jac[0] = t.x;
+            jac[1] = t.y;
+          } else {
+            jac[0] = Layout::at<float>(0, from + 4 * j);
+          }
+          const float m = project ? smax(0.0f, c.x - alpha * c.y) : c.x;
+#pragma unroll
+          for (int i = 0; i < kShare; ++i) mine[i] += m * jac[i];
+        }
+#pragma unroll
+        for (int i = 0; i < 7; ++i) w[i] = __shfl_sync(0xFFFFFFFFu, mine[i % kShare], i / kShare, P);
+      }
+      const std::uint32_t b = l.first + l.body(q);
+      const float wrench[6] = {w[0], w[1], w[2], w[3], w[4], w[5]};
+      respond(d, b, ba, bb, wrench, w[6], v, rate);
+      if (round == kFinal) {
+        if (lane == 0 && at < l.bodies) {
+          d.response.a[b] = make_float4(v[0], v[1], v[2], rate);
+          d.response.b[b] = make_float4(v[3], v[4], v[5], w[6]);
+        }
+        continue;
+      }
+    }
+    if (at < l.bodies) {
+#pragma unroll 1
+      for (std::uint32_t k = lane; k < depth; k += P) {
+        const std::uint32_t j = base + kGroup * k;
+        const float4 ea = l.a(j), eb = l.b(j);
+        const float term = round == kBound ? diagonal(ea, eb, ba, bb) : side_term(ea, eb, v, rate);
+        l.own(j) = term;
+        comm.send(l, __float_as_uint(eb.w), term);
+      }
+    }
+  }
+}
+
+// One entry per thread: the row's gap from both terms, and this CTA's share
+// of the sums.  Slots that pad a group hold zeros throughout.
+__device__ __forceinline__ Sums receive_sides(const SolveDesc& d, const Layout& l, int round, float alpha) {
+  Sums s{{0.0, 0.0, 0.0}, 0u};
+  float residual = 0.0f;
+  bool finite = true;
+  const float dt = d.dt;
+  const bool project = round == kIterate;
+#pragma unroll 1
+  for (std::uint32_t j = threadIdx.x; j < l.slots; j += kThreads) {
+    const float4 c = l.c(j);
+    const float rate = l.own(j) + l.inbox(j);
+    const float compliance = fabsf(c.y);
+    if (round == kBound) {
+      residual = smax(residual, dt * rate + compliance);
+    } else {
+      const float m = project ? smax(0.0f, c.z - alpha * c.w) : c.z;
+      const float gn = c.x + dt * rate + compliance * m;
+      residual = smax(residual, row_residual(m, gn));
+      finite = finite && isfinite(gn);
+      if (project && __float_as_int(c.y) < 0) {
+        const double moved = double(m) - double(c.z);
+        const double change = double(gn) - double(c.w);
+        s.v[0] += moved * moved;
+        s.v[1] += moved * change;
+        s.v[2] += change * change;
+      }
+      *reinterpret_cast<float2*>(&l.c(j).z) = make_float2(m, gn);
+    }
+  }
+  s.bits = finite ? __float_as_uint(residual) : 0x7FC00000u;
+  return s;
+}
+
+// Loads this CTA's share of bodies [b0, b1).  False (in every CTA) when some
+// CTA's share does not fit `bytes` of shared memory.
+template <int kForm>
+__device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm, Shared& s, Layout& l,
+                           std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1, SolveDesc* state) {
+  const std::uint32_t* offsets = d.incidence.offsets;
+  const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  std::uint32_t first = b0, last = b1;
+  if constexpr (kForm != kSingle) {
+    const std::uint64_t total = weight(offsets, b0, b1);
+    if (comm.rank > 0) first = find_split(offsets, b0, b1, total * comm.rank / comm.size);
+    if (comm.rank + 1 < comm.size) last = find_split(offsets, b0, b1, total * (comm.rank + 1) / comm.size);
+    __syncthreads();
+  }
+  const std::uint32_t bodies = last - first;
+  l.first = first;
+  l.bodies = bodies;
+  const std::uint32_t groups = (bodies + kGroup - 1) / kGroup;
+  // Carve the parts that depend on the body count.
+  std::uint64_t at = 0;
+  const auto carve = [&](std::uint64_t size) {
+    const std::uint32_t here = std::uint32_t(at);
+    at += (size + 15) & ~std::uint64_t(15);
+    return here;
+  };
+  l.body_a_at = carve(16ull * bodies);
+  l.body_b_at = carve(16ull * bodies);
+  l.group_at = carve(4ull * groups);
+  l.body_at = carve(2ull * bodies);
+  l.degree_at = carve(bodies);
+  for (std::uint32_t i = threadIdx.x; i < 16; i += kThreads) s.warp[i] = s.parts[i] = Sums{{0.0, 0.0, 0.0}, 0u};
+  if (threadIdx.x == 0) {
+    s.misfit = at > bytes || bodies > 0xFFFFu ? 1u : 0u;
+    s.remote_count = 0;
+    s.slots = 0;
+  }
+  for (std::uint32_t i = threadIdx.x; i < kWarps * kClasses; i += kThreads) (&s.histogram[0][0])[i] = 0;
+  __syncthreads();
+  const bool room = s.misfit == 0;
+  __syncthreads();
+  if (room) {
+    // Bodies by falling degree (a stable counting sort, so that the order of
+    // the sums does not depend on scheduling): the 32 bodies of a warp then
+    // have nearly the same number of entries.
+    const std::uint32_t per = ((bodies + kWarps - 1) / kWarps + 31) & ~31u;
+    const std::uint32_t from = smin(bodies, warp * per), to = smin(bodies, from + per);
+    for (std::uint32_t i = from; i < to; i += 32) {
+      const bool live = i + lane < to;
+      std::uint32_t cls = kClasses;
+      if (live) {
+        const std::uint32_t degree = offsets[first + i + lane + 1] - offsets[first + i + lane];
+        if (degree > kResidentDegree) s.misfit = 1u;
+        cls = kClasses - 1 - smin(degree, kResidentDegree);
+      }
+      const std::uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls);
+      if (live && lane == std::uint32_t(__ffs(peers) - 1)) s.histogram[warp][cls] += std::uint16_t(__popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x < kClasses) {
+      std::uint32_t sum = 0;
+      for (int w = 0; w < kWarps; ++w) {
+        const std::uint32_t n = s.histogram[w][threadIdx.x];
+        s.histogram[w][threadIdx.x] = std::uint16_t(sum);
+        sum += n;
+      }
+      s.class_base[threadIdx.x] = sum;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      std::uint32_t x = s.class_base[lane], y = s.class_base[lane + 32], sx = x, sy = y;
+      for (int o = 1; o < 32; o <<= 1) {
+        const std::uint32_t u = __shfl_up_sync(0xFFFFFFFFu, sx, o), v = __shfl_up_sync(0xFFFFFFFFu, sy, o);
+        if (int(lane) >= o) {
+          sx += u;
+          sy += v;
+        }
+      }
+      const std::uint32_t half = __shfl_sync(0xFFFFFFFFu, sx, 31);
+      s.class_base[lane] = sx - x;
+      s.class_base[lane + 32] = half + sy - y;
+    }
+    __syncthreads();
+    for (std::uint32_t i = from; i < to; i += 32) {
+      const bool live = i + lane < to;
+      std::uint32_t cls = kClasses, degree = 0;
+      if (live) {
+        degree = smin(offsets[first + i + lane + 1] - offsets[first + i + lane], kResidentDegree);
+        cls = kClasses - 1 - degree;
+      }
+      const std::uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls);
+      if (live) {
+        const std::uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+        const std::uint32_t q = s.class_base[cls] + s.histogram[warp][cls] + rank;
+        l.body(q) = std::uint16_t(i + lane);
+        l.degree(q) = std::uint8_t(degree);
+      }
+      __syncwarp();
+      if (live && lane == std::uint32_t(__ffs(peers) - 1)) s.histogram[warp][cls] += std::uint16_t(__popc(peers));
+      __syncwarp();
+    }
+    __syncthreads();
+    // Slots of each group: kGroup times the degree of the first, the largest.
+    if (warp == 0) {
+      std::uint32_t sum = 0;
+      for (std::uint32_t g0 = 0; g0 < groups; g0 += 32) {
+        const std::uint32_t n = g0 + lane < groups ? kGroup * l.degree(kGroup * (g0 + lane)) : 0u;
+        std::uint32_t x = n;
+        for (int o = 1; o < 32; o <<= 1) {
+          const std::uint32_t u = __shfl_up_sync(0xFFFFFFFFu, x, o);
+          if (int(lane) >= o) x += u;
+        }
+        if (g0 + lane < groups) l.group(g0 + lane) = sum + x - n;
+        sum += __shfl_sync(0xFFFFFFFFu, x, 31);
+      }
+      if (lane == 0) s.slots = sum;
+    }
+    __syncthreads();
+    const std::uint32_t slots = s.slots;
+    l.slots = slots;
+    l.a_at = carve(16ull * slots);
+    l.b_at = carve(16ull * slots);
+    l.c_at = carve(16ull * slots);
+    l.own_at = carve(4ull * slots);
+    l.inbox_at = carve(4ull * slots);
+    if (threadIdx.x == 0) s.inbox_at = static_cast<std::uint32_t>(__cvta_generic_to_shared(resident_memory)) + l.inbox_at;
+    l.remote_at = carve(kForm == kGrid ? 2ull * slots : 0ull);
+    if (threadIdx.x == 0 && (at > bytes || slots > 0xFFFFu || (kForm == kGrid && slots > r.stride))) s.misfit = 1u;
+    __syncthreads();
+    if (s.misfit == 0) {
+      for (std::uint32_t q = threadIdx.x; q < bodies; q += kThreads) {
+        const std::uint32_t b = first + l.body(q);
+        l.body_a(q) = d.bodies.a[b];
+        l.body_b(q) = d.bodies.b[b];
+        const std::uint32_t degree = l.degree(q), depth = depth_of(l, q);
+        const std::uint32_t base = base_of(l, q);
+        const std::uint32_t begin = offsets[b];
+        for (std::uint32_t k = 0; k < degree; ++k) {
+          const std::uint32_t j = base + kGroup * k;
+          const float4 eb = d.incidence.b[begin + k];
+          const std::uint32_t side = __float_as_uint(eb.w), row = side >> 1;
+          const float2 constants = d.incidence.constants[row];
+          l.a(j) = d.incidence.a[begin + k];
+          l.b(j) = eb;
+          l.c(j) = make_float4(constants.x, (side & 1u) ? constants.y : -constants.y, d.multipliers[row], 0.0f);
+          l.own(j) = 0.0f;
+          l.inbox(j) = 0.0f;
+          r.slot_of[begin + k] = comm.rank << 16 | j;
+        }
+        for (std::uint32_t k = degree; k < depth; ++k) {
+          pad_slot(l, base + kGroup * k);
+        }
+      }
+      // The last group's missing bodies.
+      if (bodies % kGroup != 0) {
+        const std::uint32_t there = bodies % kGroup, missing = kGroup - there, depth = depth_of(l, bodies - there);
+        for (std::uint32_t i = threadIdx.x; i < missing * depth; i += kThreads) {
+          pad_slot(l, l.group(groups - 1) + kGroup * (i / missing) + there + i % missing);
+        }
+      }
+      if constexpr (kForm == kGrid) {
+        unsigned long long* words = r.inbox + std::size_t(comm.rank) * r.stride;
+        for (std::uint32_t j = threadIdx.x; j < slots; j += kThreads) words[j] = 0ull;
+        for (std::uint32_t i = threadIdx.x; i < 2 * kResidentWords; i += kThreads) {
+          const std::size_t set = std::size_t(i / kResidentWords) * kResidentRecords;
+          r.records[(set + comm.rank) * kResidentWords + i % kResidentWords] = make_ulonglong2(0ull, 0ull);
+          if (comm.rank % kFan == 0) {
+            r.records[(set + kResidentMaxCtas + comm.rank / kFan) * kResidentWords + i % kResidentWords] =
+                make_ulonglong2(0ull, 0ull);
+          }
+        }
+      }
+    }
+  }
+  // Every CTA's slots are known (or one does not fit) from here on.
+  if constexpr (kForm == kGrid) {
+    if (threadIdx.x == 0 && s.misfit != 0) atomicExch(&state->misfit, 1u);
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      atomicAdd(&state->barrier_count, 1u);
+      std::uint32_t polls = 0;
+      while (*static_cast<volatile std::uint32_t*>(&state->barrier_count) < comm.size) {
+        if (++polls == kWaitPolls) {
+          atomicExch(&state->barrier_abort, 1u);
+          s.misfit = 1u;
+          break;
+        }
+      }
+      __threadfence();
+      if (*static_cast<volatile std::uint32_t*>(&state->misfit) != 0u) s.misfit = 1u;
+    }
+    __syncthreads();
+  } else if constexpr (kForm == kCluster) {
+    __threadfence();
+    comm.sync_all();
+    const bool misfit = __syncthreads_or(threadIdx.x < comm.size &&
+                                         *cg::this_cluster().map_shared_rank(&s.misfit, threadIdx.x) != 0u) != 0;
+    if (threadIdx.x < comm.size) s.inboxes[threadIdx.x] = *cg::this_cluster().map_shared_rank(&s.inbox_at, threadIdx.x);
+    comm.sync_all();
+    if (misfit) s.misfit = 1u;
+    __syncthreads();
+  } else {
+    __syncthreads();
+  }
+  if (s.misfit != 0) return false;
+  // Where each entry's side terms go: the other entry of its row.
+  for (std::uint32_t q = threadIdx.x; q < bodies; q += kThreads) {
+    const std::uint32_t degree = l.degree(q);
+    const std::uint32_t base = base_of(l, q);
+    for (std::uint32_t k = 0; k < degree; ++k) {
+      const std::uint32_t j = base + kGroup * k;
+      const std::uint32_t side = __float_as_uint(l.b(j).w);
+      std::uint32_t meta = kNobody;
+      if (!index_ok(side >> 1, d.row_count, &state->check_status)) {
+        l.inbox(j) = -0.0f;
+      } else if ((side & 1u) != 0u || d.rows.slots[side >> 1].y != kInvalidSlot) {
+        const std::uint32_t place = r.places[side ^ 1u];
+        const std::uint32_t to =
+            index_ok(place, 2ull * d.row_count, &state->check_status) ? __ldcg(&r.slot_of[place]) : comm.rank << 16 | j;
+        const std::uint32_t cta = to >> 16, slot = to & 0xFFFFu;
+        if constexpr (kForm == kSingle) {
+          meta = slot;
+        } else if constexpr (kForm == kCluster) {
+          meta = cluster_address(s.inboxes[cta] + 4 * slot, cta);
+        } else if (cta == comm.rank) {
+          meta = slot;
+        } else {
+          meta = kRemote | (cta * r.stride + slot);
+          l.remote(atomicAdd(&s.remote_count, 1u)) = std::uint16_t(j);
+        }
+      } else {
+        // A constraint row has no second side: -0.0f adds nothing.
+        l.inbox(j) = -0.0f;
+      }
+      l.b(j).w = __uint_as_float(meta);
+    }
+  }
+  __syncthreads();
+  return true;
+}
+
+// The whole solve of bodies [b0, b1) by the CTAs of `comm`.
+template <int kForm, int P>
+__device__ __forceinline__ void resident_solve(const SolveDesc& d, const ResidentArrays& r, Comm<kForm> comm, Shared& s,
+                               std::uint32_t bytes, SolveDesc* state) {
+  Layout l{};
+  if (!load_share(d, r, comm, s, l, bytes, 0u, d.body_count, state)) {
+    if (kForm != kGrid && comm.rank == 0 && threadIdx.x == 0) state->misfit = 1u;
+    return;
+  }
+  // Every thread takes the same decisions from the same sums (in the grid
+  // form warp 0 does, and the block reads them).  The rounds share one copy
+  // of the code: what a round executes is fetched once per iteration, by few
+  // warps, so its size counts.
+  constexpr bool kBlockDecides = kForm != kGrid;
+  float bound = 0.0f, step = 0.0f, residual = 0.0f;
+  std::uint32_t iterations = 0, status = MSB_SOLVE_ITERATION_LIMIT;
+  int round = kBound;
+#pragma unroll 1
+  for (;;) {
+    ++comm.round;
+    send_sides<P>(d, l, comm, round, step);
+    if (round == kFinal) break;
+    bool arrived = comm.exchange(l, s);
+    if (arrived) {
+      Sums x = receive_sides(d, l, round, step);
+      arrived = reduce(comm, s, x);
+      if (kBlockDecides || threadIdx.x < 32) {
+        const float value = __uint_as_float(x.bits);
+        if (round == kBound) {
+          bound = value;
+          round = kInitial;
+        } else {
+          residual = value;
+          if (round == kInitial && (!isfinite(bound) || !(bound > 0.0f))) {
+            status = 3;  // no positive diagonal: an invalid system
+            round = kFinal;
+          } else if (!isfinite(residual)) {
+            status = MSB_SOLVE_BREAKDOWN;
+            iterations += round == kIterate ? 1u : 0u;
+            round = kFinal;
+          } else if (!(residual > d.tolerance)) {
+            status = MSB_SOLVE_CONVERGED;
+            iterations += round == kIterate ? 1u : 0u;
+            round = kFinal;
+          } else if (round == kInitial) {
+            step = 1.0f / bound;
+            round = d.max_iterations > 0 ? kIterate : kFinal;
+          } else {
+            iterations += 1;
+            step = next_step(step, x.v[0], x.v[1], x.v[2], iterations);
+            round = iterations < d.max_iterations ? kIterate : kFinal;
+          }
+        }
+      }
+    }
+    if constexpr (!kBlockDecides) {
+      if (threadIdx.x == 0) {
+        s.alpha = step;
+        s.round = round;
+      }
+      arrived = __syncthreads_or(!arrived) == 0;
+      step = s.alpha;
+      round = s.round;
+    }
+    if (!arrived) {
+      if (threadIdx.x == 0) atomicExch(&state->barrier_abort, 1u);
+      return;
+    }
+  }
+  // The solution (the last round wrote its response).
+  for (std::uint32_t q = threadIdx.x; q < l.bodies; q += kThreads) {
+    const std::uint32_t degree = l.degree(q);
+    const std::uint32_t base = base_of(l, q);
+    const std::uint32_t begin = d.incidence.offsets[l.first + l.body(q)];
+    for (std::uint32_t k = 0; k < degree; ++k) {
+      const std::uint32_t side = __float_as_uint(d.incidence.b[begin + k].w);
+      if (side & 1u) continue;
+      const float4 c = l.c(base + kGroup * k);
+      d.multipliers[side >> 1] = c.z;
+      d.gaps[side >> 1] = c.w;
+      d.iterate[side >> 1] = make_float2(c.z, c.w);
+    }
+  }
+  if (comm.rank == 0 && threadIdx.x == 0) {
+    state->step = step;
+    state->residual = residual;
+    state->bound = bound;
+    state->iterations = iterations;
+    state->status = status;
+    state->mode = 1;
+  }
+}
+
+template <int kForm, int P>
+__global__ void __launch_bounds__(kThreads, 1)
+    resident_kernel(const __grid_constant__ SolveDesc problem, const __grid_constant__ ResidentArrays arrays,
+                    SolveDesc* state, std::uint32_t bytes) {
+  __shared__ Shared s;
+  Comm<kForm> comm{blockIdx.x, gridDim.x, &arrays};
+  resident_solve<kForm, P>(problem, arrays, comm, s, bytes, state);
+  if constexpr (kForm == kCluster) cg::this_cluster().sync();  // no CTA leaves while another may read its sums
+}
+
+constexpr std::uint32_t kSharedLimit = 227 * 1024;  // of one CTA on an SM
+constexpr std::uint32_t kDynamicBytes = (kSharedLimit - std::uint32_t(sizeof(Shared)) - 1024) & ~15u;
+
+template <int kForm, int P>
+cudaError_t configure(cudaLaunchConfig_t& config, cudaLaunchAttribute& attribute, int ctas, cudaStream_t stream) {
+  const auto kernel = resident_kernel<kForm, P>;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDynamicBytes));
+  if (e != cudaSuccess) return e;
+  config = cudaLaunchConfig_t{};
+  config.gridDim = dim3(unsigned(ctas));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kDynamicBytes;
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = kForm == kSingle ? 0 : 1;
+  if (kForm == kCluster) {
+    // Clusters of 16 CTAs are beyond the portable size of 8.
+    if (ctas > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    attribute.id = cudaLaunchAttributeClusterDimension;
+    attribute.val.clusterDim.x = unsigned(ctas);
+    attribute.val.clusterDim.y = 1;
+    attribute.val.clusterDim.z = 1;
+  } else if (kForm == kGrid) {
+    attribute.id = cudaLaunchAttributeCooperative;
+    attribute.val.cooperative = 1;
+  }
+  return e;
+}
+
+template <int kForm, int P>
+int launch_form(const SolveDesc& problem, SolveDesc* desc, const ResidentArrays& arrays, int ctas,
+                cudaStream_t stream) {
+  cudaLaunchConfig_t config;
+  cudaLaunchAttribute attribute;
+  const cudaError_t e = configure<kForm, P>(config, attribute, ctas, stream);
+  if (e != cudaSuccess) return int(e);
+  count_launch();
+  return int(cudaLaunchKernelEx(&config, resident_kernel<kForm, P>, problem, arrays, desc, kDynamicBytes));
+}
+
+template <int kForm>
+int launch_lanes(const SolveDesc& problem, SolveDesc* desc, const ResidentArrays& arrays, ResidentPlan plan,
+                 cudaStream_t stream) {
+  return plan.lanes == 4 ? launch_form<kForm, 4>(problem, desc, arrays, plan.ctas, stream)
+                         : launch_form<kForm, 1>(problem, desc, arrays, plan.ctas, stream);
+}
+
+}  // namespace
+
+std::uint32_t resident_stride() { return kSharedLimit / kEntryBytes; }
+
+ResidentLimits resident_limits() {
+  ResidentLimits limits;
+  int device = 0, sms = 0, cooperative = 0, per_sm = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return limits;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  cudaDeviceGetAttribute(&cooperative, cudaDevAttrCooperativeLaunch, device);
+  cudaLaunchConfig_t config;
+  cudaLaunchAttribute attribute;
+  for (const int ctas : {8, 16}) {
+    int clusters = 0;
+    if (configure<kCluster, 1>(config, attribute, ctas, nullptr) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, resident_kernel<kCluster, 1>, &config) == cudaSuccess && clusters > 0) {
+      limits.cluster = ctas;
+    }
+  }
+  if (cooperative != 0 && configure<kGrid, 1>(config, attribute, 1, nullptr) == cudaSuccess &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resident_kernel<kGrid, 1>, kThreads, kDynamicBytes) ==
+          cudaSuccess) {
+    limits.grid = std::min(sms * per_sm, int(kResidentMaxCtas));
+  }
+  cudaGetLastError();
+  return limits;
+}
+
+ResidentPlan resident_plan(const ResidentLimits& limits, std::uint64_t rows, std::uint64_t bodies) {
+  const std::uint64_t bytes = 2 * rows * kEntryBytes + bodies * kBodyBytes;
+  // 3 % for the slots that pad the groups of bodies.
+  const std::uint64_t share = std::uint64_t(kDynamicBytes) * 97 / 100;
+  ResidentPlan plan;
+  if (bytes <= share * 3 / 4 || (limits.cluster == 0 && bytes <= share)) {
+    plan = {1, false, 1};
+  } else if (bytes <= std::uint64_t(limits.cluster) * share) {
+    plan = {limits.cluster, false, 1};
+  } else if (bytes <= std::uint64_t(limits.grid) * share) {
+    plan = {limits.grid, true, 1};
+  }
+  // Four lanes a body while its CTA's bodies are few; one thread a body keeps
+  // more of them in flight.
+  if (plan.ctas > 1 && bodies <= 256ull * plan.ctas) plan.lanes = 4;
+  return plan;
+}
+
+int launch_resident(const SolveDesc& problem, SolveDesc* desc, const ResidentArrays& arrays, ResidentPlan plan,
+                    cudaStream_t stream) {
+  if (plan.grid) return launch_lanes<kGrid>(problem, desc, arrays, plan, stream);
+  if (plan.ctas > 1) return launch_lanes<kCluster>(problem, desc, arrays, plan, stream);
+  return launch_lanes<kSingle>(problem, desc, arrays, plan, stream);
+}
+
+}  // namespace msb

@@ -642,12 +642,13 @@ __global__ void incidence_order_kernel(const std::uint32_t* __restrict__ offsets
 __global__ void incidence_gather_kernel(RowArrays r, const std::uint32_t* __restrict__ values,
                                         const std::uint32_t* __restrict__ total, std::uint32_t rows,
                                         float4* __restrict__ out_a, float4* __restrict__ out_b,
-                                        std::uint32_t* status) {
+                                        std::uint32_t* __restrict__ places, std::uint32_t* status) {
   const std::uint32_t entries = *total;
   for (std::uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < entries; k += gridDim.x * blockDim.x) {
     const std::uint32_t v = values[k];
     const std::uint32_t row = v >> 1;
     if (!index_ok(row, rows, status)) continue;
+    if (places != nullptr) places[v] = k;
     if (v & 1u) {
       const float4 c = r.c[row];
       const float4 d = r.d[row];
@@ -702,7 +703,7 @@ void incidence_pass(RowArrays rows, std::uint32_t row_count, std::uint32_t body_
   incidence_order_kernel<<<grid_for(body_count, 256), 256, 0, stream>>>(incidence.offsets, body_count, values);
   count_launch();
   incidence_gather_kernel<<<grid_for(2ull * row_count, 256), 256, 0, stream>>>(
-      rows, values, incidence.offsets + body_count, row_count, incidence.a, incidence.b, status);
+      rows, values, incidence.offsets + body_count, row_count, incidence.a, incidence.b, incidence.places, status);
   count_launch();
 }
 

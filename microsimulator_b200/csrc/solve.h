@@ -47,13 +47,16 @@ struct ResponseArrays {
 //   sides     = each side's term of the gap rate, jacobian . velocity -
 //               lever * elongation rate, indexed by the entries' side bits
 //               and written by the body pass.  A constraint row's second
-//               side holds -0.0f, which adds nothing: x + -0.0f == x.
+//               side holds -0.0f, which adds nothing: x + -0.0f == x;
+//   places    = by side bits, where in the incidence the side's entry is (a
+//               constraint row's second side: undefined).
 struct IncidenceArrays {
   std::uint32_t* offsets;
   float4* a;
   float4* b;
   float2* constants;
   float2* sides;
+  std::uint32_t* places;
 };
 
 // Everything one solve reads and writes, in device memory at a fixed address
@@ -97,6 +100,7 @@ struct SolveDesc {
   std::uint32_t barrier_generation;
   std::uint32_t barrier_abort;  // a barrier wait ran out of time: every block stops
   std::uint32_t check_status;   // checked build: the first index check that failed (0: none)
+  std::uint32_t misfit;         // a resident solve whose shares did not fit: nothing was done
 };
 
 // Builds the incidence of `rows` over `bodies` bodies.  Scratch: `keys` and

@@ -1,0 +1,88 @@
+"""The resident solve (the system in shared memory: one CTA, one cluster, the
+whole grid) against the solve graph on the same systems.
+
+Gaps and the residual of given multipliers take no sum over rows, and the
+first step's length is 1 / bound, so after 0 and 1 iterations the two agree
+bit for bit.  From the second step on the step length is a ratio of FP64 sums
+taken in another order, which rounds to FP32: at most one unit in the last
+place (6e-8) a step, each step moving a multiplier by at most a step length
+times its gap."""
+
+import numpy as np
+import pytest
+
+from microsimulator_b200 import abi
+from microsimulator_b200.backend import B200Backend
+from microsimulator_b200.types import ContactSolveParameters, ContactSystem
+from tests.systems import LAWS, mixed_system, multipliers_for
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def forms(backend):
+    yield backend
+    backend.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+
+
+def solve_both(backend, system, initial, iterations):
+    out = []
+    for form in (B200Backend.RELAXATION_AUTOMATIC, B200Backend.RELAXATION_GRAPH):
+        backend.set_relaxation(form)
+        out.append(backend.solve_contact_forces(system, initial, ContactSolveParameters(1e-9, iterations)))
+    return out
+
+
+# (bodies, rows): one CTA (two rows, fewer bodies than a group, a full
+# group and one more, the largest), one cluster, the grid.
+SIZES = [(3, 2), (7, 5), (8, 30), (9, 30), (300, 1100), (350, 1300), (2000, 4000), (9000, 21000), (20000, 40000),
+         (90000, 200000)]
+
+
+@pytest.mark.parametrize("bodies,rows", SIZES)
+@pytest.mark.parametrize("law", range(3))
+def test_agrees_with_the_graph(forms, bodies, rows, law):
+    system = mixed_system(bodies + law, bodies, rows, LAWS[law])
+    initial = multipliers_for(system, rows)
+    for iterations in (0, 1):
+        resident, graph = solve_both(forms, system, initial, iterations)
+        assert resident.report == graph.report
+        assert np.array_equal(resident.multipliers, graph.multipliers)
+    resident, graph = solve_both(forms, system, initial, 6)
+    assert resident.report.status == graph.report.status
+    assert resident.report.iterations == graph.report.iterations
+    scale = np.max(np.abs(graph.multipliers))
+    assert np.max(np.abs(resident.multipliers - graph.multipliers)) <= 1e-5 * scale
+
+
+def hub_system(degree: int, bodies: int = 400) -> ContactSystem:
+    """A chain whose middle body also touches every tenth of `degree` others."""
+    system = mixed_system(degree, bodies, bodies - 1, LAWS[0], walls=0.0)
+    system.rows["first_slot"] = np.arange(bodies - 1)
+    system.rows["second_slot"] = np.arange(1, bodies)
+    hub = np.resize(system.rows, degree - 2)
+    hub["first_slot"], hub["second_slot"] = bodies // 2, np.arange(degree - 2)
+    system.rows = np.concatenate([system.rows, hub]).astype(abi.CONTACT_ROW_DTYPE)
+    return system
+
+
+@pytest.mark.parametrize("degree", [61, 62, 63, 64, 150])
+def test_bodies_of_many_rows(forms, degree):
+    # Up to 62 entries a body the system is resident; beyond it takes the graph.
+    system = hub_system(degree)
+    initial = multipliers_for(system, 3)
+    resident, graph = solve_both(forms, system, initial, 1)
+    assert resident.report == graph.report
+    assert np.array_equal(resident.multipliers, graph.multipliers)
+
+
+def test_empty_bodies_and_profile_hook(forms):
+    # Bodies without rows are evaluated too; the timing hook goes on from the
+    # resident solve's iterate.
+    system = mixed_system(5, 5000, 300, LAWS[2])
+    initial = multipliers_for(system, 1)
+    resident, graph = solve_both(forms, system, initial, 1)
+    assert np.array_equal(resident.multipliers, graph.multipliers)
+    forms.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+    forms.solve_contact_forces(system, initial, ContactSolveParameters(1e-9, 1))
+    assert forms.profile_iterations(2)["rows"] == 300
