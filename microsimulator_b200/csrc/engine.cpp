@@ -555,6 +555,10 @@ struct msb_context {
   std::optional<msb::ResidentLimits> resident_limits;
   msb::DBuf<std::uint32_t> resident_slots;
   msb::DBuf<unsigned long long> resident_inbox;
+  // The cells along a curve through the substep's base geometry, for the
+  // grid form; valid within a substep of one system.
+  msb::DBuf<std::uint32_t> spatial_keys, spatial_order, spatial_offsets;
+  bool spatial_valid = false;
   msb::DBuf<ulonglong2> resident_records;
   msb::DBuf<float> slack;
 
@@ -1284,9 +1288,18 @@ bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_r
     c.resident_inbox.ensure(std::size_t(resident_stride()) * kResidentMaxCtas);
     c.resident_records.ensure(2ull * kResidentRecords * kResidentWords);
   }
+  const bool ordered = plan.grid && c.spatial_valid;
+  if (ordered) {
+    c.counts.ensure(c.n + 1ull);
+    c.spatial_offsets.ensure(c.n + 1ull);
+    c.temp.ensure(scan_temp_words(c.n + 1ull) + 64);
+    launch_order_offsets(c.n, c.spatial_order.p, c.inc_offsets.p, c.counts.p, c.spatial_offsets.p, c.temp.p, c.stream);
+  }
   fill_desc(c, c.rows.count, dt, growth, tolerance, max_iterations, true);
-  const ResidentArrays arrays{c.inc_places.p, c.resident_slots.p, c.resident_inbox.p, c.resident_records.p,
-                              resident_stride()};
+  const ResidentArrays arrays{c.inc_places.p,       c.resident_slots.p,
+                              c.resident_inbox.p,   c.resident_records.p,
+                              resident_stride(),    ordered ? c.spatial_order.p : nullptr,
+                              ordered ? c.spatial_offsets.p : nullptr};
   check(cudaError_t(launch_resident(*c.host_desc, c.desc, arrays, plan, c.stream)), "solve launch");
   check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
   sync(c);
@@ -1678,6 +1691,19 @@ Attempt advance_substep(Ctx& c, float dt, const msb_contact_dynamics_parameters&
   const std::uint32_t found = find_touches(c, c.state, cp, wp, p.candidate_margin, c.touches,
                                            p.candidate_margin + (c.colonies > 0 ? kBatchRecheckReach : kRecheckReach), true);
   mark(c, kPhaseRows);
+  // Systems that take the resident solve's grid form get their cells'
+  // spatial order, from the grid of the search just made.
+  c.spatial_valid = false;
+  if (c.colonies == 0 && c.relaxation == 0 && found > 0 && n > 1) {
+    if (!c.resident_limits) c.resident_limits = resident_limits();
+    if (resident_plan(*c.resident_limits, found, n).grid) {
+      c.spatial_keys.ensure(n);
+      c.spatial_order.ensure(n);
+      c.temp.ensure(sort_temp_words(n) + 64);
+      launch_spatial_order(n, c.state.pos_len.p, c.grid.p, c.spatial_keys.p, c.spatial_order.p, c.temp.p, c.stream);
+      c.spatial_valid = true;
+    }
+  }
   c.rows.count = 0;
   c.rows.ensure(std::max<std::uint32_t>(found, 1));
   reset_scalars(c);
@@ -1915,6 +1941,7 @@ void write_outputs(Ctx& c, msb_contact_dynamics_outputs* outputs, bool device_po
 void load_system(Ctx& c, const msb_contact_system& s, const float* multipliers) {
   validate_system(s);
   c.n = std::uint32_t(s.body_count);
+  c.spatial_valid = false;  // the records carry no geometry
   c.has_drift = false;
   for (std::uint64_t b = 0; b < s.body_count && !c.has_drift; ++b) {
     for (float v : s.bodies[b].drift) c.has_drift = c.has_drift || v != 0.0f || std::signbit(v);

@@ -182,6 +182,11 @@ __device__ std::uint32_t find_split(const std::uint32_t* offsets, std::uint32_t 
   return lo;
 }
 
+// The body at a place of the order in which CTAs take them.
+__device__ __forceinline__ std::uint32_t body_at(const ResidentArrays& r, std::uint32_t place) {
+  return r.order != nullptr ? r.order[place] : place;
+}
+
 template <int kForm>
 struct Comm {
   std::uint32_t rank, size;
@@ -419,7 +424,7 @@ __device__ __forceinline__ void send_sides(const SolveDesc& d, const Layout& l, 
 #pragma unroll
         for (int i = 0; i < 7; ++i) w[i] = __shfl_sync(0xFFFFFFFFu, mine[i % kShare], i / kShare, P);
       }
-      const std::uint32_t b = l.first + l.body(q);
+      const std::uint32_t b = body_at(*comm.arrays, l.first + l.body(q));
       const float wrench[6] = {w[0], w[1], w[2], w[3], w[4], w[5]};
       respond(d, b, ba, bb, wrench, w[6], v, rate);
       if (round == kFinal) {
@@ -482,7 +487,7 @@ __device__ __forceinline__ Sums receive_sides(const SolveDesc& d, const Layout& 
 template <int kForm>
 __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm, Shared& s, Layout& l,
                            std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1, SolveDesc* state) {
-  const std::uint32_t* offsets = d.incidence.offsets;
+  const std::uint32_t* offsets = r.order != nullptr ? r.order_offsets : d.incidence.offsets;
   const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   std::uint32_t first = b0, last = b1;
   if constexpr (kForm != kSingle) {
@@ -608,12 +613,12 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
     __syncthreads();
     if (s.misfit == 0) {
       for (std::uint32_t q = threadIdx.x; q < bodies; q += kThreads) {
-        const std::uint32_t b = first + l.body(q);
+        const std::uint32_t b = body_at(r, first + l.body(q));
         l.body_a(q) = d.bodies.a[b];
         l.body_b(q) = d.bodies.b[b];
         const std::uint32_t degree = l.degree(q), depth = depth_of(l, q);
         const std::uint32_t base = base_of(l, q);
-        const std::uint32_t begin = offsets[b];
+        const std::uint32_t begin = d.incidence.offsets[b];
         for (std::uint32_t k = 0; k < degree; ++k) {
           const std::uint32_t j = base + kGroup * k;
           const float4 eb = d.incidence.b[begin + k];
@@ -792,7 +797,7 @@ __device__ __forceinline__ void resident_solve(const SolveDesc& d, const Residen
   for (std::uint32_t q = threadIdx.x; q < l.bodies; q += kThreads) {
     const std::uint32_t degree = l.degree(q);
     const std::uint32_t base = base_of(l, q);
-    const std::uint32_t begin = d.incidence.offsets[l.first + l.body(q)];
+    const std::uint32_t begin = d.incidence.offsets[body_at(r, l.first + l.body(q))];
     for (std::uint32_t k = 0; k < degree; ++k) {
       const std::uint32_t side = __float_as_uint(d.incidence.b[begin + k].w);
       if (side & 1u) continue;
@@ -820,6 +825,34 @@ __global__ void __launch_bounds__(kThreads, 1)
   Comm<kForm> comm{blockIdx.x, gridDim.x, &arrays};
   resident_solve<kForm, P>(problem, arrays, comm, s, bytes, state);
   if constexpr (kForm == kCluster) cg::this_cluster().sync();  // no CTA leaves while another may read its sums
+}
+
+// Eight bits of each of x and y, interleaved; both axes at the scale of the
+// longer one.
+__global__ void spatial_keys_kernel(std::uint32_t n, const float4* __restrict__ pos_len, const GridParams* grid_ptr,
+                                    std::uint32_t* __restrict__ keys, std::uint32_t* __restrict__ order) {
+  const double wx = grid_ptr->inv_width[0], wy = grid_ptr->inv_width[1];
+  const double x0 = grid_ptr->low[0], y0 = grid_ptr->low[1];
+  const double scale = 256.0 / fmax(double(grid_ptr->dims[0]) / wx, double(grid_ptr->dims[1]) / wy);
+  for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const float4 p = pos_len[i];
+    const auto cell = [&](double at) { return std::uint32_t(fmin(fmax(at * scale, 0.0), 255.0)); };
+    const auto spread = [](std::uint32_t v) {
+      v = (v | (v << 4)) & 0x0F0Fu;
+      v = (v | (v << 2)) & 0x3333u;
+      return (v | (v << 1)) & 0x5555u;
+    };
+    keys[i] = spread(cell(double(p.x) - x0)) | spread(cell(double(p.y) - y0)) << 1;
+    order[i] = i;
+  }
+}
+
+__global__ void order_counts_kernel(std::uint32_t n, const std::uint32_t* __restrict__ order,
+                                    const std::uint32_t* __restrict__ offsets, std::uint32_t* __restrict__ counts) {
+  for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
+    const std::uint32_t b = i < n ? order[i] : 0u;
+    counts[i] = i < n ? offsets[b + 1] - offsets[b] : 0u;
+  }
 }
 
 constexpr std::uint32_t kSharedLimit = 227 * 1024;  // of one CTA on an SM
@@ -870,6 +903,21 @@ int launch_lanes(const SolveDesc& problem, SolveDesc* desc, const ResidentArrays
 }
 
 }  // namespace
+
+void launch_spatial_order(std::uint32_t n, const float4* pos_len, const GridParams* grid, std::uint32_t* keys,
+                          std::uint32_t* order, std::uint32_t* temp, cudaStream_t stream) {
+  spatial_keys_kernel<<<grid_for(n, 256), 256, 0, stream>>>(n, pos_len, grid, keys, order);
+  count_launch();
+  radix_sort_pairs(keys, order, n, 16, temp, stream);
+}
+
+void launch_order_offsets(std::uint32_t n, const std::uint32_t* order, const std::uint32_t* offsets,
+                          std::uint32_t* counts, std::uint32_t* order_offsets, std::uint32_t* temp,
+                          cudaStream_t stream) {
+  order_counts_kernel<<<grid_for(n + 1ull, 256), 256, 0, stream>>>(n, order, offsets, counts);
+  count_launch();
+  exclusive_scan(counts, order_offsets, n + 1ull, temp, stream);
+}
 
 std::uint32_t resident_stride() { return kSharedLimit / kEntryBytes; }
 

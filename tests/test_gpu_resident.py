@@ -11,9 +11,9 @@ times its gap."""
 import numpy as np
 import pytest
 
-from microsimulator_b200 import abi
+from microsimulator_b200 import abi, workloads
 from microsimulator_b200.backend import B200Backend
-from microsimulator_b200.types import ContactSolveParameters, ContactSystem
+from microsimulator_b200.types import ContactDynamicsParameters, ContactSolveParameters, ContactSystem
 from tests.systems import LAWS, mixed_system, multipliers_for
 
 pytestmark = pytest.mark.gpu
@@ -86,3 +86,25 @@ def test_empty_bodies_and_profile_hook(forms):
     forms.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
     forms.solve_contact_forces(system, initial, ContactSolveParameters(1e-9, 1))
     assert forms.profile_iterations(2)["rows"] == 300
+
+
+@pytest.mark.parametrize("cells", [9000, 30000])
+@pytest.mark.parametrize("flat", [True, False])
+def test_steps_in_spatial_order(forms, cells, flat):
+    """Steps whose solves spread over the grid in spatial order (a colony in
+    the plane, one whose cells share one x, where every key is of y alone):
+    within four solve tolerances, as two solves of one system may differ."""
+    world = workloads.jammed(cells, seed=cells)
+    if not flat:
+        world.position_z, world.position_x = world.position_x.copy(), np.zeros(cells, np.float32)
+        world.direction_z, world.direction_x = world.direction_x.copy(), np.zeros(cells, np.float32)
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4)
+    results = []
+    for form in (B200Backend.RELAXATION_AUTOMATIC, B200Backend.RELAXATION_GRAPH):
+        forms.set_relaxation(form)
+        stepped = world.copy()
+        report = forms.advance_contact_dynamics(stepped, None, 0.02, p).report
+        results.append((stepped, report))
+    (a, ra), (b, rb) = results
+    assert ra.substeps == rb.substeps and ra.halvings == rb.halvings
+    assert np.max(np.abs(a.geometry() - b.geometry())) <= 4 * p.overlap_tolerance
