@@ -20,11 +20,6 @@ __device__ __forceinline__ std::uint32_t pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const std::uint32_t*>(&v);
 }
 
-// The derivative of GELU in its exact error-function form.
-__device__ __forceinline__ float gelu_grad(float z) {
-  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
-}
-
 // Floats as unsigned words that order like the floats.
 __device__ __forceinline__ std::uint32_t ordered(float f) {
   const std::uint32_t b = __float_as_uint(f);
@@ -188,36 +183,26 @@ __global__ void __launch_bounds__(kThreads) features_kernel(std::uint32_t n, con
   }
 }
 
-__global__ void output_grad_kernel(std::uint32_t n, const float* __restrict__ dy, std::uint16_t* __restrict__ out) {
-  for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n * kOutputPad;
-       i += gridDim.x * blockDim.x) {
-    const std::uint32_t r = i / kOutputPad, c = i % kOutputPad;
-    const float v = c < kOutputs ? dy[std::size_t(r) * kOutputs + c] : 0.0f;
-    const __nv_bfloat16 b = __float2bfloat16_rn(v);
-    out[i] = *reinterpret_cast<const std::uint16_t*>(&b);
+// dY as bf16 padded to kOutputPad columns, and each warp's column sums of the
+// fp32 gradients (kOutputPad columns a warp).
+__global__ void output_grad_kernel(std::uint32_t n, const float* __restrict__ dy, std::uint16_t* __restrict__ out,
+                                   float* __restrict__ column_partials) {
+  const std::uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+  float v[kOutputs] = {};
+  if (r < n) {
+#pragma unroll
+    for (int c = 0; c < kOutputs; ++c) v[c] = dy[std::size_t(r) * kOutputs + c];
+    *reinterpret_cast<uint4*>(out + std::size_t(r) * kOutputPad) =
+        make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], 0.0f), 0u, 0u);
   }
-}
-
-// dZ = dH * gelu'(Z), in fp32 (for the bias sums) and bf16 (for the GEMMs).
-__global__ void gelu_backward_kernel(std::uint64_t count, const float* __restrict__ dh, const float* __restrict__ z,
-                                     float* __restrict__ dz, std::uint16_t* __restrict__ dz_bf16) {
-  for (std::uint64_t i = blockIdx.x * std::uint64_t(blockDim.x) + threadIdx.x; i < count;
-       i += std::uint64_t(gridDim.x) * blockDim.x) {
-    const float v = dh[i] * gelu_grad(z[i]);
-    dz[i] = v;
-    const __nv_bfloat16 b = __float2bfloat16_rn(v);
-    dz_bf16[i] = *reinterpret_cast<const std::uint16_t*>(&b);
+#pragma unroll
+  for (int c = 0; c < kOutputs; ++c) {
+    for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_xor_sync(0xFFFFFFFFu, v[c], o);
   }
-}
-
-// Column sums of an n x cols fp32 matrix (row stride `stride`), in row order.
-__global__ void column_sums_kernel(std::uint32_t n, std::uint32_t cols, std::uint32_t stride,
-                                   const float* __restrict__ x, float* __restrict__ out) {
-  const std::uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.0f;
-  for (std::uint32_t r = 0; r < n; ++r) s += x[std::size_t(r) * stride + c];
-  out[c] = s;
+  const std::uint32_t lane = threadIdx.x & 31u;
+  if (lane < kOutputPad) {
+    column_partials[std::size_t(r / 32) * kOutputPad + lane] = lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : 0.0f;
+  }
 }
 
 __global__ void adam_kernel(float* __restrict__ params, const float* __restrict__ grads, float* __restrict__ m,
@@ -315,47 +300,48 @@ int launch_backward(const std::uint16_t* weights, const std::uint16_t* features,
     return int(cudaMemsetAsync(grads, 0, kParameters * sizeof(float), stream));
   }
   const Activations act = activations_at(const_cast<void*>(activations), n);
-  auto* p = static_cast<unsigned char*>(scratch);
-  float* dh = reinterpret_cast<float*>(p);
-  p += std::size_t(n) * kHidden * 4;
-  float* dz = reinterpret_cast<float*>(p);
-  p += std::size_t(n) * kHidden * 4;
-  auto* dzb = reinterpret_cast<std::uint16_t*>(p);
-  p += std::size_t(n) * kHidden * 2;
+  // 16-byte aligned, as the GEMMs write and read it.
+  auto* p = reinterpret_cast<unsigned char*>((reinterpret_cast<std::uintptr_t>(scratch) + 15) & ~std::uintptr_t(15));
+  std::uint16_t* dz[2];
+  for (auto*& d : dz) {
+    d = reinterpret_cast<std::uint16_t*>(p);
+    p += std::size_t(n) * kHidden * 2;
+  }
   auto* dyb = reinterpret_cast<std::uint16_t*>(p);
   p += std::size_t(n) * 16 * 2;
+  auto* columns = reinterpret_cast<float*>(p);
+  p += column_partial_rows(n) * kHidden * 4;
   // The GEMMs' split-K partials, 256-byte aligned.
   auto* partials = reinterpret_cast<float*>((reinterpret_cast<std::uintptr_t>(p) + 255) & ~std::uintptr_t(255));
 
-  output_grad_kernel<<<grid_for(std::uint64_t(n) * kOutputPad, kThreads), kThreads, 0, stream>>>(n, output_grad, dyb);
+  const std::uint32_t rows = std::uint32_t(column_partial_rows(n));  // of 32 gradients each
+  output_grad_kernel<<<rows / 4, 128, 0, stream>>>(n, output_grad, dyb, columns);
   count_launch();
   float* gw = grads;
   float* gb = grads + kWeights;
-  cudaMemsetAsync(gb + kB3, 0, kOutputPad * sizeof(float), stream);
-  column_sums_kernel<<<1, 32, 0, stream>>>(n, kOutputs, kOutputs, output_grad, gb + kB3);
-  count_launch();
   const auto* h3 = reinterpret_cast<const std::uint16_t*>(act.h[2]);
   int status = 0;
-  const auto gemm = [&](const Gemm& g) {
-    if (status == 0) status = tc_gemm(g, partials, error, stream);
+  const auto gemm = [&](const Gemm& g, const ColumnSums& sums = {}) {
+    if (status == 0) status = tc_gemm(g, partials, error, stream, sums);
   };
-  // dW3 (8 x 128) = dY^T H3;  dH3 (n x 128) = dY W3.
-  gemm({kOutputPad, kHidden, n, dyb, 1, kOutputPad, h3, kHidden, 1, gw + kW3, kHidden, 1});
-  gemm({n, kHidden, kOutputPad, dyb, kOutputPad, 1, weights + kW3, kHidden, 1, dh, kHidden, 1});
+  // dW3 (8 x 128) = dY^T H3 and db3;  dZ2 (n x 128) = dY W3 * gelu'(Z2).
+  gemm({kOutputPad, kHidden, n, dyb, 1, kOutputPad, h3, kHidden, 1, gw + kW3, kHidden, 1},
+       {columns, rows, kOutputPad, gb + kB3});
+  gemm({n, kHidden, kOutputPad, dyb, kOutputPad, 1, weights + kW3, kHidden, 1, nullptr, 0, 0, act.z[2], dz[0], columns});
   const std::uint32_t bias_at[3] = {kB0, kB1, kB2};
   const std::uint32_t weight_at[3] = {kW0, kW1, kW2};
   for (int l = 2; l >= 0; --l) {
-    const std::uint64_t count = std::uint64_t(n) * kHidden;
-    gelu_backward_kernel<<<grid_for(count, kThreads), kThreads, 0, stream>>>(count, dh, act.z[l], dz, dzb);
-    count_launch();
-    column_sums_kernel<<<1, kHidden, 0, stream>>>(n, kHidden, kHidden, dz, gb + bias_at[l]);
-    count_launch();
+    std::uint16_t* dzl = dz[l & 1];  // 2: 0, 1: 1, 0: 0
     const std::uint16_t* input = l == 0 ? features : reinterpret_cast<const std::uint16_t*>(act.h[l - 1]);
     const std::uint32_t width = l == 0 ? kInput : kHidden;
-    // dW_l (128 x width) = dZ^T H_{l-1}.
-    gemm({kHidden, width, n, dzb, 1, kHidden, input, width, 1, gw + weight_at[l], width, 1});
-    // dH_{l-1} (n x 128) = dZ W_l.
-    if (l > 0) gemm({n, kHidden, kHidden, dzb, kHidden, 1, weights + weight_at[l], kHidden, 1, dh, kHidden, 1});
+    // dW_l (128 x width) = dZ_l^T H_{l-1} and db_l.
+    gemm({kHidden, width, n, dzl, 1, kHidden, input, width, 1, gw + weight_at[l], width, 1},
+         {columns, rows, kHidden, gb + bias_at[l]});
+    // dZ_{l-1} (n x 128) = dZ_l W_l * gelu'(Z_{l-1}).
+    if (l > 0) {
+      gemm({n, kHidden, kHidden, dzl, kHidden, 1, weights + weight_at[l], kHidden, 1, nullptr, 0, 0, act.z[l - 1],
+            dz[(l - 1) & 1], columns});
+    }
   }
   return status;
 }

@@ -38,14 +38,20 @@ constexpr float kLengthScale = 3.0f;
 constexpr float kBinSide = 6.0f;
 
 // Bytes of the split-K partial sums tc_gemm may use.
-constexpr std::uint64_t kGemmPartialBytes = std::uint64_t(32) * 128 * 128 * 4;
+constexpr std::uint32_t kGemmMaxSplits = 128;
+constexpr std::uint64_t kGemmPartialBytes = std::uint64_t(kGemmMaxSplits) * 128 * 128 * 4;
+
+// Rows of partial column sums that n rows leave: one per warp of a 128-row
+// tile.
+constexpr std::uint64_t column_partial_rows(std::uint64_t n) { return 4 * ((n + 127) / 128); }
 
 // Bytes of the activations the forward pass keeps for the backward pass:
 // H1..H3 (bf16) and Z1..Z3 (fp32), n x 128 each.
 inline std::uint64_t activation_bytes(std::uint64_t n) { return n * kHidden * (3 * 2 + 3 * 4); }
-// Bytes of the backward pass's scratch (its GEMMs' split-K partials last).
+// Bytes of the backward pass's scratch: two layers' dZ (bf16), dY (bf16),
+// the partial column sums, and its GEMMs' split-K partials last.
 inline std::uint64_t backward_scratch_bytes(std::uint64_t n) {
-  return n * kHidden * (4 + 4 + 2) + n * 16 * 2 + 256 + kGemmPartialBytes + 256;
+  return n * kHidden * (2 + 2) + n * 16 * 2 + column_partial_rows(n) * kHidden * 4 + 256 + kGemmPartialBytes + 256;
 }
 
 // The activations a training forward pass keeps, in activation_bytes(n):
@@ -67,13 +73,27 @@ struct Gemm {
   std::int64_t sbk, sbn;
   float* c;
   std::int64_t scm, scn;
+  // With z (m x n, n == 128): C is not stored; dz (bf16, m x n) = C *
+  // gelu'(z), and each warp's column sums of the fp32 product go to
+  // column_partials (column_partial_rows(m) x 128).
+  const float* z = nullptr;
+  std::uint16_t* dz = nullptr;
+  float* column_partials = nullptr;
+};
+// Column sums to finish beside a GEMM: out[c] = sum over `rows` of
+// partials[row * cols + c], in a fixed order.
+struct ColumnSums {
+  const float* partials = nullptr;
+  std::uint32_t rows = 0;
+  std::uint32_t cols = 0;
+  float* out = nullptr;
 };
 // The GEMM on tcgen05 (mlp_tc.cu): 128-row tiles of C accumulated in TMEM,
-// a long k split over up to 32 CTAs whose partial sums (in `partials`,
-// kGemmPartialBytes) are added in a fixed order.  *error (if not null)
-// becomes kStatusIterations when a wait for the tensor cores gave up.
-// Returns a CUDA error code.
-int tc_gemm(const Gemm& p, float* partials, std::uint32_t* error, cudaStream_t stream);
+// a long k split over up to kGemmMaxSplits CTAs whose partial sums (in
+// `partials`, kGemmPartialBytes) are added in a fixed order, by the launch
+// that also finishes `sums`.  *error (if not null) becomes kStatusIterations
+// when a wait for the tensor cores gave up.  Returns a CUDA error code.
+int tc_gemm(const Gemm& p, float* partials, std::uint32_t* error, cudaStream_t stream, const ColumnSums& sums = {});
 
 struct Grid {
   float x0, y0, inverse_side;

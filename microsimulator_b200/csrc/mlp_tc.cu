@@ -125,6 +125,11 @@ __device__ __forceinline__ void load32(std::uint32_t address, float (&v)[32]) {
 
 __device__ __forceinline__ float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
 
+// The derivative of GELU in its exact error-function form.
+__device__ __forceinline__ float gelu_grad(float z) {
+  return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
+}
+
 __device__ __forceinline__ std::uint32_t pack(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const std::uint32_t*>(&v);
@@ -277,12 +282,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) forward_tc_kernel(const std::ui
 // (128 x 64) and the B chunk (n rounded up to 16, x 64) in the canonical
 // K-major layout, thread 0 issues four tcgen05.mma (K = 16 each) into the
 // TMEM accumulator and commits them to an mbarrier, and the chunk after
-// waits for them.  The four warps then read their 32 lanes of the
-// accumulator with tcgen05.ld and store C (or the split's partial sums).
+// waits for them; the next chunk's loads are in flight meanwhile.  The four
+// warps then read their 32 lanes of the accumulator with tcgen05.ld and
+// store C (or the split's partial sums), or the layer's dZ.
+//
+// Each thread stages one 8 x 8 tile of each operand with eight 16-byte loads
+// along whichever dimension is contiguous, transposed in registers where that
+// is not k.  With one 2-byte load per element (strided by a row for the
+// weight gradients) a GEMM of a training step of 8,192 rows took 70 us, and
+// a bias sum, one block adding 8,192 rows in order, 317 us; the step went
+// from 1,166 to 223 us with the vector loads, the GELU derivative and the
+// column sums in the epilogue.  At 8,192 rows it is bound by its fourteen
+// dependent launches of 5-12 us.
 
 constexpr int kGemmThreads = 128;
 constexpr std::uint32_t kGemmChunk = 64;
-constexpr std::uint32_t kGemmMaxSplits = 32;
 constexpr std::uint32_t kGemmBytesA = 128 * kGemmChunk * 2;  // 16 KB
 constexpr std::uint32_t kGemmBytesB = 128 * kGemmChunk * 2;  // 16 KB (n <= 128)
 constexpr std::uint32_t kGemmOffB = kGemmBytesA;
@@ -293,7 +307,115 @@ constexpr std::uint32_t kGemmOffTmem = kGemmOffBarrier + 8;
 constexpr std::size_t kGemmSmem = 56 * 1024;
 static_assert(kGemmOffTmem + 8 <= kGemmSmem, "gemm shared memory");
 
-__global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, std::uint32_t chunk_split, float* partials,
+// How an operand (rows x k) is read: 16 bytes along k, 16 bytes along its
+// rows, or element by element.
+enum Staging : int { kAlongK = 0, kAlongRows = 1, kByElement = 2 };
+
+// The vector forms read whole groups of eight from 16-byte aligned rows.
+Staging staging_of(const std::uint16_t* p, std::uint32_t rows, std::uint32_t k, std::int64_t row_stride,
+                   std::int64_t k_stride) {
+  if (reinterpret_cast<std::uintptr_t>(p) % 16 == 0) {
+    if (k_stride == 1 && k % 8 == 0 && row_stride % 8 == 0) return kAlongK;
+    if (row_stride == 1 && rows % 8 == 0 && k_stride % 8 == 0) return kAlongRows;
+  }
+  return kByElement;
+}
+
+// One operand's chunk: rows [row0, row0 + tile_rows), k [k0, k0 + 64), zero
+// outside [0, rows) x [0, k_end); thread t holds the 8 x 8 tile (row group,
+// k group) that place() names.
+struct Operand {
+  const std::uint16_t* p;
+  std::uint32_t rows, row0, tile_rows;
+  std::int64_t row_stride, k_stride;
+  int staging;
+
+  __device__ __forceinline__ bool place(std::uint32_t& row_group, std::uint32_t& k_group) const {
+    const std::uint32_t groups = tile_rows / 8;
+    if (staging == kAlongK) {
+      k_group = threadIdx.x % 8;
+      row_group = threadIdx.x / 8;
+    } else {
+      row_group = threadIdx.x % groups;
+      k_group = threadIdx.x / groups;
+    }
+    return row_group < groups && k_group < 8;
+  }
+  __device__ __forceinline__ void load(std::uint32_t k0, std::uint32_t k_end, uint4 (&v)[8]) const {
+    std::uint32_t rg, kg;
+    const bool mine = place(rg, kg);
+    const std::uint32_t r = row0 + rg * 8, k = k0 + kg * 8;
+    if (staging == kAlongK) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (mine && r + i < rows && k < k_end) {
+          v[i] = *reinterpret_cast<const uint4*>(p + std::int64_t(r + i) * row_stride + k);
+        }
+      }
+    } else if (staging == kAlongRows) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        v[i] = make_uint4(0u, 0u, 0u, 0u);
+        if (mine && r < rows && k + i < k_end) {
+          v[i] = *reinterpret_cast<const uint4*>(p + std::int64_t(k + i) * k_stride + r);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        std::uint32_t w[4] = {};
+        for (int j = 0; j < 8; ++j) {
+          if (mine && r + i < rows && k + j < k_end) {
+            w[j / 2] |= std::uint32_t(p[std::int64_t(r + i) * row_stride + std::int64_t(k + j) * k_stride]) << (16 * (j % 2));
+          }
+        }
+        v[i] = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+  }
+  __device__ __forceinline__ void store(unsigned char* smem, const uint4 (&v)[8]) const {
+    std::uint32_t rg, kg;
+    if (!place(rg, kg)) return;
+    unsigned char* to = smem + core_offset(tile_rows, rg * 8, kg * 8);
+    if (staging != kAlongRows) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(to + 16 * i) = v[i];
+    } else {
+      // v[i] holds rows 0..7 at k = i; row r's eight k values are wanted.
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const std::uint32_t pick = (r & 1) ? 0x7632u : 0x5410u;
+        const auto word = [&](int i) {
+          const std::uint32_t lo = reinterpret_cast<const std::uint32_t*>(&v[i])[r / 2];
+          const std::uint32_t hi = reinterpret_cast<const std::uint32_t*>(&v[i + 1])[r / 2];
+          return __byte_perm(lo, hi, pick);
+        };
+        *reinterpret_cast<uint4*>(to + 16 * r) = make_uint4(word(0), word(2), word(4), word(6));
+      }
+    }
+  }
+};
+
+// a[j] summed over the warp's lanes for each j, column `lane`'s sum in each
+// lane: halves of the columns are exchanged for halves of the lanes.
+__device__ __forceinline__ float column_sums(float (&a)[32]) {
+  const std::uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const bool upper = (lane & std::uint32_t(o)) != 0u;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float keep = upper ? a[i + o] : a[i];
+      const float send = upper ? a[i] : a[i + o];
+      a[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+    }
+  }
+  return a[0];
+}
+
+__global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, int staging_a, int staging_b,
+                                                              std::uint32_t chunk_split, float* partials,
                                                               std::uint32_t* error) {
   extern __shared__ __align__(128) unsigned char smem[];
   const std::uint32_t base = static_cast<std::uint32_t>(__cvta_generic_to_shared(smem));
@@ -304,6 +426,11 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, std::uint
   const std::uint32_t m0 = blockIdx.y * 128;
   const std::uint32_t k_begin = blockIdx.z * chunk_split * kGemmChunk;
   const std::uint32_t k_end = smin<std::uint32_t>(p.k, k_begin + chunk_split * kGemmChunk);
+  const Operand a{p.a, p.m, m0, 128u, p.sam, p.sak, staging_a};
+  const Operand b{p.b, p.n, 0u, nt, p.sbn, p.sbk, staging_b};
+  uint4 va[8], vb[8];
+  a.load(k_begin, k_end, va);
+  b.load(k_begin, k_end, vb);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(barrier), "r"(1u) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -319,22 +446,11 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, std::uint
   __syncthreads();
   fence_after();
   const std::uint32_t tmem = *tmem_slot;
-  unsigned char* sa = smem;
-  unsigned char* sb = smem + kGemmOffB;
   std::uint32_t phase = 0;
   std::uint32_t issued = 0;
   for (std::uint32_t k0 = k_begin; k0 < k_end; k0 += kGemmChunk) {
-    // Stage the chunk: A (128 x 64) and B (nt x 64), zero outside the matrices.
-    for (std::uint32_t e = threadIdx.x; e < 128 * kGemmChunk; e += kGemmThreads) {
-      const std::uint32_t r = e / kGemmChunk, kk = e % kGemmChunk;
-      const std::uint32_t mm = m0 + r, k = k0 + kk;
-      const std::uint16_t va = (mm < p.m && k < k_end) ? p.a[std::int64_t(mm) * p.sam + std::int64_t(k) * p.sak] : 0;
-      *reinterpret_cast<std::uint16_t*>(sa + core_offset(128, r, kk)) = va;
-      if (r < nt) {
-        const std::uint16_t vb = (r < p.n && k < k_end) ? p.b[std::int64_t(k) * p.sbk + std::int64_t(r) * p.sbn] : 0;
-        *reinterpret_cast<std::uint16_t*>(sb + core_offset(nt, r, kk)) = vb;
-      }
-    }
+    a.store(smem, va);
+    b.store(smem + kGemmOffB, vb);
     fence_async_smem();
     fence_before();
     __syncthreads();
@@ -347,6 +463,12 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, std::uint
         mma(tmem, ad, bd, idesc, (issued > 0 || s > 0) ? 1u : 0u);
       }
       commit(barrier);
+    }
+    if (k0 + kGemmChunk < k_end) {
+      a.load(k0 + kGemmChunk, k_end, va);
+      b.load(k0 + kGemmChunk, k_end, vb);
+    }
+    if (threadIdx.x == 0) {
       std::uint32_t polls = 0;
       while (!try_wait(barrier, phase)) {
         if (++polls > kWaitPolls) {
@@ -374,9 +496,31 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, std::uint
 #pragma unroll
         for (int j = 0; j < 32; ++j) v[j] = 0.0f;  // an empty share of k
       }
-      if (row < p.m) {
-        for (std::uint32_t j = 0; j < 32 && c0 + j < p.n; ++j) {
+      if (p.z != nullptr) {
+        const std::size_t at = std::size_t(row) * p.n + c0;
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+          float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          if (row < p.m) z = *reinterpret_cast<const float4*>(p.z + at + j);
+          v[j] = row < p.m ? v[j] * gelu_grad(z.x) : 0.0f;
+          v[j + 1] = row < p.m ? v[j + 1] * gelu_grad(z.y) : 0.0f;
+          v[j + 2] = row < p.m ? v[j + 2] * gelu_grad(z.z) : 0.0f;
+          v[j + 3] = row < p.m ? v[j + 3] * gelu_grad(z.w) : 0.0f;
+        }
+        if (row < p.m) {
+#pragma unroll
+          for (int j = 0; j < 32; j += 8) {
+            *reinterpret_cast<uint4*>(p.dz + at + j) = make_uint4(pack(v[j], v[j + 1]), pack(v[j + 2], v[j + 3]),
+                                                                  pack(v[j + 4], v[j + 5]), pack(v[j + 6], v[j + 7]));
+          }
+        }
+        const float sum = column_sums(v);
+        p.column_partials[(std::size_t(blockIdx.y) * 4 + warp) * p.n + c0 + (threadIdx.x & 31)] = sum;
+      } else if (row < p.m) {
+#pragma unroll
+        for (std::uint32_t j = 0; j < 32; ++j) {
           const std::uint32_t col = c0 + j;
+          if (col >= p.n) continue;
           if (partials != nullptr) {
             partials[(std::size_t(blockIdx.z) * p.m + row) * p.n + col] = v[j];
           } else {
@@ -394,39 +538,75 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, std::uint
   }
 }
 
-// C = the sum of the splits' partial sums, in split order.
-__global__ void gemm_reduce_kernel(Gemm p, std::uint32_t splits, const float* __restrict__ partials) {
-  const std::uint64_t total = std::uint64_t(p.m) * p.n;
-  for (std::uint64_t i = blockIdx.x * std::uint64_t(blockDim.x) + threadIdx.x; i < total;
-       i += std::uint64_t(gridDim.x) * blockDim.x) {
+// The first `blocks` blocks: C = the sum of the splits' partial sums, 64
+// elements a block, four threads each taking every fourth split and the
+// four added in order.  The others: 32 of the column sums each, eight threads
+// taking every eighth row.
+constexpr int kReduceThreads = 256;
+__global__ void __launch_bounds__(kReduceThreads) gemm_reduce_kernel(Gemm p, std::uint32_t splits,
+                                                                    const float* __restrict__ partials,
+                                                                    std::uint32_t blocks, ColumnSums sums) {
+  __shared__ float parts[8][64];
+  if (blockIdx.x < blocks) {
+    const std::uint64_t total = std::uint64_t(p.m) * p.n;
+    const std::uint32_t e = threadIdx.x % 64, part = threadIdx.x / 64;
+    const std::uint64_t i = blockIdx.x * std::uint64_t(64) + e;
     float sum = 0.0f;
-    for (std::uint32_t z = 0; z < splits; ++z) sum += partials[z * total + i];
-    const std::uint32_t row = std::uint32_t(i / p.n), col = std::uint32_t(i % p.n);
-    p.c[std::int64_t(row) * p.scm + std::int64_t(col) * p.scn] = sum;
+    if (i < total) {
+#pragma unroll 8
+      for (std::uint32_t z = part; z < splits; z += 4) sum += partials[z * total + i];
+    }
+    parts[part][e] = sum;
+    __syncthreads();
+    if (part == 0 && i < total) {
+      const std::uint32_t row = std::uint32_t(i / p.n), col = std::uint32_t(i % p.n);
+      p.c[std::int64_t(row) * p.scm + std::int64_t(col) * p.scn] =
+          ((parts[0][e] + parts[1][e]) + parts[2][e]) + parts[3][e];
+    }
+  } else {
+    const std::uint32_t c = (blockIdx.x - blocks) * 32 + threadIdx.x % 32, part = threadIdx.x / 32;
+    float sum = 0.0f;
+    if (c < sums.cols) {
+#pragma unroll 8
+      for (std::uint32_t r = part; r < sums.rows; r += 8) sum += sums.partials[std::size_t(r) * sums.cols + c];
+    }
+    parts[part][threadIdx.x % 32] = sum;
+    __syncthreads();
+    if (part == 0 && c < sums.cols) {
+      for (int k = 1; k < 8; ++k) sum += parts[k][threadIdx.x];
+      sums.out[c] = sum;
+    }
   }
 }
 
 }  // namespace
 
-int tc_gemm(const Gemm& p, float* partials, std::uint32_t* error, cudaStream_t stream) {
+int tc_gemm(const Gemm& p, float* partials, std::uint32_t* error, cudaStream_t stream, const ColumnSums& sums) {
   if (p.m == 0 || p.n == 0) return 0;
-  if (p.n > 128) return int(cudaErrorInvalidValue);
+  if (p.n > 128 || (p.z != nullptr && p.n != 128)) return int(cudaErrorInvalidValue);
   cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kGemmSmem));
   if (e != cudaSuccess) return int(e);
   const std::uint32_t tiles = (p.m + 127) / 128;
   const std::uint32_t chunks = std::max<std::uint32_t>(1, (p.k + kGemmChunk - 1) / kGemmChunk);
-  // A long k over several CTAs when the tiles alone leave SMs idle.
+  // A long k over several CTAs when the tiles alone leave SMs idle, two
+  // chunks or more each: with one, a CTA's TMEM allocation and epilogue
+  // outweigh its chunk.
   std::uint32_t splits = 1;
-  if (tiles < 64 && partials != nullptr && std::uint64_t(p.m) * p.n * kGemmMaxSplits * 4 <= kGemmPartialBytes) {
-    splits = std::min(std::min(kGemmMaxSplits, chunks), std::max<std::uint32_t>(1, 128 / tiles));
+  if (tiles < 64 && p.z == nullptr && partials != nullptr &&
+      std::uint64_t(p.m) * p.n * kGemmMaxSplits * 4 <= kGemmPartialBytes) {
+    splits = std::min(std::min(kGemmMaxSplits, std::max(1u, chunks / 2)), std::max<std::uint32_t>(1, 128 / tiles));
   }
   const std::uint32_t per_split = (chunks + splits - 1) / splits;
   splits = (chunks + per_split - 1) / per_split;
   const dim3 grid(1, tiles, splits);
-  gemm_tc_kernel<<<grid, kGemmThreads, kGemmSmem, stream>>>(p, per_split, splits > 1 ? partials : nullptr, error);
+  gemm_tc_kernel<<<grid, kGemmThreads, kGemmSmem, stream>>>(p, staging_of(p.a, p.m, p.k, p.sam, p.sak),
+                                                            staging_of(p.b, p.n, p.k, p.sbn, p.sbk), per_split,
+                                                            splits > 1 ? partials : nullptr, error);
   count_launch();
-  if (splits > 1) {
-    gemm_reduce_kernel<<<grid_for(std::uint64_t(p.m) * p.n, 256), 256, 0, stream>>>(p, splits, partials);
+  const std::uint32_t blocks = splits > 1 ? std::uint32_t((std::uint64_t(p.m) * p.n + 63) / 64) : 0u;
+  const std::uint32_t column_blocks = sums.out != nullptr ? (sums.cols + 31) / 32 : 0u;
+  if (blocks + column_blocks > 0) {
+    gemm_reduce_kernel<<<blocks + column_blocks, kReduceThreads, 0, stream>>>(p, splits, partials, blocks, sums);
     count_launch();
   }
   return int(cudaGetLastError());
