@@ -559,6 +559,10 @@ struct msb_context {
   // grid form; valid within a substep of one system.
   msb::DBuf<std::uint32_t> spatial_keys, spatial_order, spatial_offsets;
   bool spatial_valid = false;
+  // A batch's schedule: jobs, gangs, each CTA's list.
+  msb::DBuf<msb::ResidentJob> batch_jobs;
+  msb::DBuf<msb::ResidentGang> batch_gangs;
+  msb::DBuf<std::uint32_t> batch_lists, batch_flags, colony_rest;
   msb::DBuf<ulonglong2> resident_records;
   msb::DBuf<float> slack;
 
@@ -1203,9 +1207,9 @@ IncidenceArrays incidence_arrays(Ctx& c) {
   return {c.inc_offsets.p, c.inc_a.p, c.inc_b.p, c.inc_constants.p, c.inc_sides.p, c.inc_places.p};
 }
 
-void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_response& growth, float tolerance,
-               std::uint32_t max_iterations, bool with_state = false) {
-  SolveDesc& d = *c.host_desc;
+// The problem part of a solve's descriptor.
+void fill_problem(Ctx& c, SolveDesc& d, std::uint32_t row_count, float dt, const msb_growth_load_response& growth,
+                  float tolerance, std::uint32_t max_iterations) {
   d.rows = c.rows.arrays();
   d.bodies = {c.body_a.p, c.body_b.p, c.drift_a.p, c.drift_b.p};
   d.incidence = incidence_arrays(c);
@@ -1224,6 +1228,12 @@ void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_
   d.tolerance = tolerance;
   d.max_iterations = max_iterations;
   d.has_drift = c.has_drift ? 1u : 0u;
+}
+
+void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_response& growth, float tolerance,
+               std::uint32_t max_iterations, bool with_state = false) {
+  SolveDesc& d = *c.host_desc;
+  fill_problem(c, d, row_count, dt, growth, tolerance, max_iterations);
   if (with_state) {
     // The fused solve resets nothing itself: copy the state part too.
     d.step = 0.0f;
@@ -1241,7 +1251,7 @@ void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_
     d.barrier_generation = 0;
     d.barrier_abort = 0;
     d.check_status = 0;
-    d.misfit = 0;
+    d.gang = {};
     check(cudaMemcpyAsync(c.desc, &d, sizeof(SolveDesc), cudaMemcpyHostToDevice, c.stream), "desc");
     return;
   }
@@ -1279,34 +1289,40 @@ void build_row_keys(Ctx& c, RowStore& store) {
 // incidence of c.rows and the bodies.
 SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growth, std::uint32_t max_iterations);
 
-// The solve with the system in shared memory, in one launch; c.host_desc
-// holds its report.  False, with nothing done, when a share does not fit.
-bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_response& growth, float tolerance,
-                    std::uint32_t max_iterations) {
-  c.resident_slots.ensure(2ull * c.rows.count);
-  if (plan.grid) {
+// A resident solve's arrays; over several CTAs with words in global memory
+// (`grid`), and in spatial order where the substep has one.
+ResidentArrays resident_arrays(Ctx& c, bool grid) {
+  c.resident_slots.ensure(2ull * std::max<std::uint32_t>(c.rows.count, 1));
+  if (grid) {
     c.resident_inbox.ensure(std::size_t(resident_stride()) * kResidentMaxCtas);
-    c.resident_records.ensure(2ull * kResidentRecords * kResidentWords);
+    c.resident_records.ensure(2ull * kResidentMaxCtas * kResidentWords);
   }
-  const bool ordered = plan.grid && c.spatial_valid;
+  const bool ordered = grid && c.spatial_valid;
   if (ordered) {
     c.counts.ensure(c.n + 1ull);
     c.spatial_offsets.ensure(c.n + 1ull);
     c.temp.ensure(scan_temp_words(c.n + 1ull) + 64);
     launch_order_offsets(c.n, c.spatial_order.p, c.inc_offsets.p, c.counts.p, c.spatial_offsets.p, c.temp.p, c.stream);
   }
+  return {c.inc_places.p,    c.resident_slots.p,
+          c.resident_inbox.p, c.resident_records.p,
+          resident_stride(), ordered ? c.spatial_order.p : nullptr,
+          ordered ? c.spatial_offsets.p : nullptr};
+}
+
+// The solve with the system in shared memory, in one launch; c.host_desc
+// holds its report.  False, with nothing done, when a share does not fit.
+bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_response& growth, float tolerance,
+                    std::uint32_t max_iterations) {
+  const ResidentArrays arrays = resident_arrays(c, plan.grid);
   fill_desc(c, c.rows.count, dt, growth, tolerance, max_iterations, true);
-  const ResidentArrays arrays{c.inc_places.p,       c.resident_slots.p,
-                              c.resident_inbox.p,   c.resident_records.p,
-                              resident_stride(),    ordered ? c.spatial_order.p : nullptr,
-                              ordered ? c.spatial_offsets.p : nullptr};
   check(cudaError_t(launch_resident(*c.host_desc, c.desc, arrays, plan, c.stream)), "solve launch");
   check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
   sync(c);
-  if (c.host_desc->barrier_abort != 0) throw DeviceCheckError("a wait of the resident solve ran out of time");
+  if (c.host_desc->gang.late != 0) throw DeviceCheckError("a wait of the resident solve ran out of time");
   if (c.host_desc->check_status != 0) throw DeviceCheckError("an index check of the resident solve failed");
   c.last_blocks = grid_for(std::max(c.rows.count, c.n), kSolveThreads, 4);
-  return c.host_desc->misfit == 0;
+  return c.host_desc->gang.misfit == 0;
 }
 
 SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, float tolerance,
@@ -1438,6 +1454,105 @@ void tune_batch(Ctx& c, const msb::BatchDesc& d) {
   c.batch_tuned = true;
 }
 
+// Colonies of a batch that takes the resident solve at most: the host lays
+// out their schedule (and a colony's spatial key has 16 bits).
+constexpr std::uint32_t kResidentColonies = 8192;
+
+// The active colonies' jobs, largest first, each on the stretch of CTAs that
+// is free first; colonies that no stretch holds go to `rest`.  Jobs are
+// weighed alike, one CTA's at half of that: its iteration needs no word of
+// another CTA (4 against 8 us with the shared memory full).
+struct BatchSchedule {
+  std::vector<ResidentJob> jobs;
+  std::vector<std::uint32_t> list_offsets, lists;
+  std::vector<std::uint32_t> rest;
+};
+BatchSchedule schedule_batch(const std::vector<std::uint32_t>& active, const std::vector<std::uint32_t>& rows,
+                             const std::vector<std::uint32_t>& cell_offsets, std::uint32_t ctas) {
+  BatchSchedule out;
+  std::vector<std::pair<std::uint32_t, std::uint32_t>> order;  // (CTAs, colony)
+  for (std::uint32_t i = 0; i < active.size(); ++i) {
+    if (active[i] == 0u) continue;
+    const std::uint32_t wanted = std::max(1u, resident_ctas(rows[i], cell_offsets[i + 1] - cell_offsets[i]));
+    if (wanted > ctas) {
+      out.rest.push_back(i);
+    } else {
+      order.emplace_back(wanted, i);
+    }
+  }
+  std::stable_sort(order.begin(), order.end(), [](const auto& x, const auto& y) { return x.first > y.first; });
+  std::vector<float> busy(ctas, 0.0f);
+  std::vector<std::vector<std::uint32_t>> lists(ctas);
+  for (const auto& [size, colony] : order) {
+    std::uint32_t best = 0;
+    float start = -1.0f;
+    for (std::uint32_t first = 0; first + size <= ctas; ++first) {
+      const float at = *std::max_element(busy.begin() + first, busy.begin() + first + size);
+      if (start < 0.0f || at < start) {
+        start = at;
+        best = first;
+      }
+    }
+    for (std::uint32_t k = best; k < best + size; ++k) {
+      busy[k] = start + (size == 1 ? 0.5f : 1.0f);
+      lists[k].push_back(std::uint32_t(out.jobs.size()));
+    }
+    out.jobs.push_back({colony, best, size});
+  }
+  out.list_offsets.push_back(0);
+  for (const auto& list : lists) {
+    out.lists.insert(out.lists.end(), list.begin(), list.end());
+    out.list_offsets.push_back(std::uint32_t(out.lists.size()));
+  }
+  return out;
+}
+
+// The active colonies by gangs of CTAs that hold them in shared memory;
+// returns those left over (too large, or whose shares did not fit).
+std::vector<std::uint32_t> solve_batch_resident(Ctx& c, const std::vector<std::uint32_t>& active,
+                                                const std::vector<std::uint32_t>& row_counts, float dt,
+                                                const msb_growth_load_response& growth,
+                                                std::uint32_t max_iterations) {
+  const std::uint32_t ctas = std::uint32_t(c.resident_limits->grid);
+  BatchSchedule plan = schedule_batch(active, row_counts, c.host_colony_offsets, ctas);
+  if (plan.jobs.empty()) return plan.rest;
+  SolveDesc problem{};
+  fill_problem(c, problem, c.rows.count, dt, growth, 0.0f, max_iterations);
+  const ResidentArrays arrays = resident_arrays(c, true);
+  c.batch_jobs.ensure(plan.jobs.size());
+  c.batch_gangs.ensure(plan.jobs.size());
+  c.batch_lists.ensure(plan.list_offsets.size() + plan.lists.size());
+  c.batch_flags.ensure(2);
+  check(cudaMemcpyAsync(c.batch_jobs.p, plan.jobs.data(), plan.jobs.size() * sizeof(ResidentJob),
+                        cudaMemcpyHostToDevice, c.stream),
+        "copy jobs");
+  check(cudaMemcpyAsync(c.batch_lists.p, plan.list_offsets.data(), plan.list_offsets.size() * 4,
+                        cudaMemcpyHostToDevice, c.stream),
+        "copy jobs");
+  check(cudaMemcpyAsync(c.batch_lists.p + plan.list_offsets.size(), plan.lists.data(), plan.lists.size() * 4,
+                        cudaMemcpyHostToDevice, c.stream),
+        "copy jobs");
+  check(cudaMemsetAsync(c.batch_gangs.p, 0, plan.jobs.size() * sizeof(ResidentGang), c.stream), "memset");
+  check(cudaMemsetAsync(c.batch_flags.p, 0, 8, c.stream), "memset");
+  const ResidentBatch batch{c.batch_jobs.p,     c.batch_gangs.p,       c.batch_lists.p,
+                            c.batch_lists.p + plan.list_offsets.size(), c.colony_offsets.p,
+                            c.colony_row_counts.p, c.colony_solve_tolerance.p, c.colony_state.p,
+                            c.batch_flags.p,    c.batch_flags.p + 1};
+  check(cudaError_t(launch_resident_batch(problem, arrays, batch, int(ctas), c.stream)), "batched solve launch");
+  std::uint32_t flags[2] = {0, 0};
+  check(cudaMemcpyAsync(flags, c.batch_flags.p, 8, cudaMemcpyDeviceToHost, c.stream), "read flags");
+  check(cudaMemcpyAsync(c.host_colony_state.data(), c.colony_state.p, c.colonies * sizeof(msb::ColonyState),
+                        cudaMemcpyDeviceToHost, c.stream),
+        "read colony states");
+  sync(c);
+  if (flags[1] != 0) throw DeviceCheckError("a wait of the batched resident solve ran out of time");
+  if (flags[0] != 0) throw DeviceCheckError("an index check of the batched resident solve failed");
+  for (const ResidentJob& job : plan.jobs) {
+    if (c.host_colony_state[job.colony].status == kResidentMisfit) plan.rest.push_back(job.colony);
+  }
+  return plan.rest;
+}
+
 SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growth, std::uint32_t max_iterations) {
   const std::uint32_t rows = c.rows.count;
   const std::uint32_t k = c.colonies;
@@ -1451,35 +1566,69 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
   check(cudaMemsetAsync(c.colony_row_counts.p, 0, (k + 1ull) * 4, c.stream), "memset");
   launch_colony_row_keys(c.rows.slots.p, rows, c.colony_of_slot.p, c.sort_keys.p, c.colony_rows.p,
                          c.colony_row_counts.p, c.stream);
-  exclusive_scan(c.colony_row_counts.p, c.colony_row_offsets.p, k + 1ull, c.temp.p, c.stream);
-  if (rows > 1) radix_sort_pairs(c.sort_keys.p, c.colony_rows.p, rows, std::max(1, int(std::bit_width(k))), c.temp.p,
-                                 c.stream);
-  const msb::BatchDesc d = batch_desc(c, dt, growth, max_iterations);
-  if (!c.batch_tuned) tune_batch(c, d);
-  // A solve of few colonies (a step's later refinement rounds, where most
-  // colonies have settled) runs them on clusters of 16 CTAs: the largest
-  // colonies then set the time, and twice the CTAs halve their iteration
-  // (256-colony sweep, 3.0M capsules: 100k-row colonies 131 -> 63 us an
-  // iteration; solves of 3 colonies 1.8-2.0 -> 1.1 ms, of 83 5.0 -> 4.8 ms).
-  // With many colonies the tuned shape's more clusters serve them better.
   c.host_colony_active.resize(k);
+  std::vector<std::uint32_t> row_counts(k);
   check(cudaMemcpyAsync(c.host_colony_active.data(), c.colony_active.p, k * 4ull, cudaMemcpyDeviceToHost, c.stream),
         "read active colonies");
+  check(cudaMemcpyAsync(row_counts.data(), c.colony_row_counts.p, k * 4ull, cudaMemcpyDeviceToHost, c.stream),
+        "read row counts");
   sync(c);
+  c.host_colony_state.resize(k);
   std::uint32_t active = 0;
   for (const std::uint32_t a : c.host_colony_active) active += a != 0u ? 1u : 0u;
-  const msb::BatchShape wide{16, 512, true};
-  const int wide_clusters = active > 0 && active <= kFewColonies ? batch_resident_clusters(wide) : 0;
-  if (wide_clusters > 0) {
-    run_batch(c, d, wide, std::min<int>(wide_clusters, int(active)));
+  // The colonies that gangs of CTAs hold in shared memory, then the others.
+  if (!c.resident_limits) c.resident_limits = resident_limits();
+  bool all = false;
+  std::vector<std::uint32_t> left = c.host_colony_active;  // the colonies still to solve
+  if (c.relaxation == 0 && c.resident_limits->grid > 0 && k <= kResidentColonies && c.batch_tuned) {
+    const auto rest = solve_batch_resident(c, c.host_colony_active, row_counts, dt, growth, max_iterations);
+    all = rest.empty();
+    std::fill(left.begin(), left.end(), 0u);
+    for (const std::uint32_t i : rest) left[i] = 1u;
+    active = std::uint32_t(rest.size());
+    c.colony_rest.ensure(k);
+    if (!all) {
+      check(cudaMemcpyAsync(c.colony_rest.p, left.data(), k * 4ull, cudaMemcpyHostToDevice, c.stream), "copy colonies");
+      sync(c);
+    }
   } else {
-    run_batch(c, d, c.batch_shape, c.batch_clusters);
+    c.colony_rest.ensure(k);
+    check(cudaMemcpyAsync(c.colony_rest.p, c.colony_active.p, k * 4ull, cudaMemcpyDeviceToDevice, c.stream),
+          "copy colonies");
   }
-  c.host_colony_state.resize(k);
-  check(cudaMemcpyAsync(c.host_colony_state.data(), c.colony_state.p, k * sizeof(msb::ColonyState),
-                        cudaMemcpyDeviceToHost, c.stream),
-        "read colony states");
-  sync(c);
+  if (!all) {
+    exclusive_scan(c.colony_row_counts.p, c.colony_row_offsets.p, k + 1ull, c.temp.p, c.stream);
+    if (rows > 1) radix_sort_pairs(c.sort_keys.p, c.colony_rows.p, rows, std::max(1, int(std::bit_width(k))), c.temp.p,
+                                   c.stream);
+    msb::BatchDesc d = batch_desc(c, dt, growth, max_iterations);
+    if (!c.batch_tuned) tune_batch(c, d);
+    d.active = c.colony_rest.p;
+    // A solve of few colonies (a step's later refinement rounds, where most
+    // colonies have settled) runs them on clusters of 16 CTAs: the largest
+    // colonies then set the time, and twice the CTAs halve their iteration
+    // (256-colony sweep, 3.0M capsules: 100k-row colonies 131 -> 63 us an
+    // iteration; solves of 3 colonies 1.8-2.0 -> 1.1 ms, of 83 5.0 -> 4.8 ms).
+    // With many colonies the tuned shape's more clusters serve them better.
+    const msb::BatchShape wide{16, 512, true};
+    const int wide_clusters = active > 0 && active <= kFewColonies ? batch_resident_clusters(wide) : 0;
+    if (wide_clusters > 0) {
+      run_batch(c, d, wide, std::min<int>(wide_clusters, int(active)));
+    } else {
+      run_batch(c, d, c.batch_shape, c.batch_clusters);
+    }
+    std::vector<msb::ColonyState> states(k);
+    check(cudaMemcpyAsync(states.data(), c.colony_state.p, k * sizeof(msb::ColonyState), cudaMemcpyDeviceToHost,
+                          c.stream),
+          "read colony states");
+    sync(c);
+    // The kernel zeroes the iterations of the colonies it leaves out.
+    for (std::uint32_t i = 0; i < k; ++i) {
+      if (left[i] != 0u || c.host_colony_active[i] == 0u) c.host_colony_state[i] = states[i];
+    }
+  }
+  for (std::uint32_t i = 0; i < k; ++i) {
+    if (c.host_colony_active[i] == 0u) c.host_colony_state[i].iterations = 0;
+  }
   SolveOutcome out{};
   out.status = MSB_SOLVE_CONVERGED;
   std::uint32_t worst = 0;
@@ -1694,13 +1843,15 @@ Attempt advance_substep(Ctx& c, float dt, const msb_contact_dynamics_parameters&
   // Systems that take the resident solve's grid form get their cells'
   // spatial order, from the grid of the search just made.
   c.spatial_valid = false;
-  if (c.colonies == 0 && c.relaxation == 0 && found > 0 && n > 1) {
+  if (c.relaxation == 0 && found > 0 && n > 1) {
     if (!c.resident_limits) c.resident_limits = resident_limits();
-    if (resident_plan(*c.resident_limits, found, n).grid) {
+    if (c.colonies > 0 ? c.resident_limits->grid > 0 && c.colonies <= kResidentColonies
+                       : resident_plan(*c.resident_limits, found, n).grid) {
       c.spatial_keys.ensure(n);
       c.spatial_order.ensure(n);
       c.temp.ensure(sort_temp_words(n) + 64);
-      launch_spatial_order(n, c.state.pos_len.p, c.grid.p, c.spatial_keys.p, c.spatial_order.p, c.temp.p, c.stream);
+      launch_spatial_order(n, c.state.pos_len.p, c.grid.p, c.colonies > 0 ? c.colony_of_slot.p : nullptr,
+                           std::max(c.colonies, 1u), c.spatial_keys.p, c.spatial_order.p, c.temp.p, c.stream);
       c.spatial_valid = true;
     }
   }

@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <bit>
 #include <type_traits>
 #include <cstdint>
 
@@ -64,8 +65,7 @@ struct Shared {
   std::uint32_t class_base[kClasses];
   Sums warp[16];   // each warp's sums
   Sums parts[16];  // the cluster's, written by its CTAs
-  float alpha;
-  int round;
+  std::uint32_t round;
   std::uint32_t misfit;
   std::uint32_t remote_count;
   std::uint32_t slots;
@@ -154,6 +154,16 @@ __device__ __forceinline__ bool wait_word(const unsigned long long* p, std::uint
   return true;
 }
 
+// Waits until *p has reached `count`, a gang's CTAs having arrived: they may
+// first finish other systems.
+__device__ __forceinline__ bool wait_count(const std::uint32_t* p, std::uint32_t count) {
+  for (std::uint32_t polls = 0; *static_cast<const volatile std::uint32_t*>(p) < count; ++polls) {
+    if (polls == (1u << 28)) return false;
+    if (polls > 1024u) __nanosleep(500);
+  }
+  return true;
+}
+
 __device__ __forceinline__ std::uint32_t cluster_address(std::uint32_t local, std::uint32_t rank) {
   std::uint32_t out;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(local), "r"(rank));
@@ -191,7 +201,9 @@ template <int kForm>
 struct Comm {
   std::uint32_t rank, size;
   const ResidentArrays* arrays;
-  std::uint32_t round = 0;
+  std::uint32_t first = 0;  // grid form: the first of the gang's CTAs
+  std::uint32_t round = 0;  // grid form: tags words, never falls within a launch
+  ResidentGang* gang = nullptr;
 
   __device__ void sync_all() const {
     if constexpr (kForm == kCluster) {
@@ -221,7 +233,7 @@ struct Comm {
       sync_all();
       return true;
     } else {
-      const unsigned long long* words = arrays->inbox + std::size_t(rank) * arrays->stride;
+      const unsigned long long* words = arrays->inbox + std::size_t(first + rank) * arrays->stride;
       bool late = false;
       constexpr int kFlight = 4;
       for (std::uint32_t x0 = threadIdx.x; x0 < s.remote_count; x0 += kFlight * kThreads) {
@@ -263,6 +275,11 @@ __device__ __forceinline__ double fold_warp(const Sums& x, std::uint32_t& bits) 
   bits = __reduce_max_sync(0xFFFFFFFFu, x.bits);
   return p;
 }
+__device__ __forceinline__ void store_sums(Sums& to, double p, std::uint32_t bits) {
+  const std::uint32_t lane = threadIdx.x & 31u;
+  if (lane == 24u) to.bits = bits;
+  if ((lane & 7u) == 0u && lane < 24u) to.v[lane / 8] = p;
+}
 // The same of 16 records in shared memory, and its totals in every lane.
 __device__ __forceinline__ Sums fold_records(const Sums* records) {
   const std::uint32_t lane = threadIdx.x & 31u, k = lane >> 3, i = lane & 7u;
@@ -272,21 +289,14 @@ __device__ __forceinline__ Sums fold_records(const Sums* records) {
   return {{__shfl_sync(0xFFFFFFFFu, p, 0), __shfl_sync(0xFFFFFFFFu, p, 8), __shfl_sync(0xFFFFFFFFu, p, 16)}, bits};
 }
 
-constexpr std::uint32_t kFan = 12;  // CTAs a group of the grid form's reduction
-static_assert((kResidentMaxCtas + kFan - 1) / kFan <= 32 && kFan <= 32, "a warp reads a group's records, and the groups'");
 static_assert(kWarps <= 16, "fold_records reads 16 records");
-// Records of two alternating sets: a CTA writes a set again only after every
-// CTA has read the other, and so has read this one.
-__device__ __forceinline__ ulonglong2* record_at(const Comm<kGrid>& comm, std::uint32_t index) {
-  return comm.arrays->records + (std::size_t(comm.round & 1u) * kResidentRecords + index) * kResidentWords;
+// CTA `rank`'s record, in one of two alternating sets: a CTA writes a set
+// again only after every CTA has read the other, and so has read this one.
+__device__ __forceinline__ ulonglong2* record_of(const Comm<kGrid>& comm, std::uint32_t rank) {
+  return comm.arrays->records + (std::size_t(comm.round & 1u) * kResidentMaxCtas + comm.first + rank) * kResidentWords;
 }
-// fold_warp's sums as the record `index` (the whole warp).
-__device__ __forceinline__ void put_record(const Comm<kGrid>& comm, std::uint32_t index, double p, std::uint32_t bits) {
-  const std::uint32_t lane = threadIdx.x & 31u;
-  if ((lane & 7u) == 0u && lane < 24u) put_wide(record_at(comm, index) + lane / 8, comm.round, bits, p);
-}
-__device__ __forceinline__ bool get_record(const Comm<kGrid>& comm, std::uint32_t index, Sums& x) {
-  const ulonglong2* from = record_at(comm, index);
+__device__ __forceinline__ bool get_record(const Comm<kGrid>& comm, std::uint32_t rank, Sums& x) {
+  const ulonglong2* from = record_of(comm, rank);
   ulonglong2 w[3];
   const auto there = [&] {
     bool all = true;
@@ -306,21 +316,14 @@ __device__ __forceinline__ bool get_record(const Comm<kGrid>& comm, std::uint32_
   return true;
 }
 
-// The sums of every CTA, in a fixed order: in every thread, in the grid form
-// in warp 0.  False (grid form, in some lanes) once a wait has run out.
+// The sums of every CTA, in a fixed order, in every thread.  False (grid
+// form) once a wait has run out.
 template <int kForm>
 __device__ __forceinline__ bool reduce(const Comm<kForm>& comm, Shared& s, Sums& x) {
   const std::uint32_t lane = threadIdx.x & 31u;
   std::uint32_t bits;
   double p = fold_warp(x, bits);
-  if ((lane & 7u) == 0u) {
-    Sums& to = s.warp[threadIdx.x >> 5];
-    if (lane < 24u) {
-      to.v[lane / 8] = p;
-    } else {
-      to.bits = bits;
-    }
-  }
+  store_sums(s.warp[threadIdx.x >> 5], p, bits);
   __syncthreads();
   if constexpr (kForm == kSingle) {
     x = fold_records(s.warp);
@@ -331,27 +334,23 @@ __device__ __forceinline__ bool reduce(const Comm<kForm>& comm, Shared& s, Sums&
     }
     comm.sync_all();
     x = fold_records(s.parts);
-  } else if (threadIdx.x < 32) {
-    // Two hops: every kFan-th CTA adds its group's records, and every CTA
-    // adds the groups' sums.
-    bool late = false;
-    const std::uint32_t groups = (comm.size + kFan - 1) / kFan;
-    const std::uint32_t leader = comm.rank - comm.rank % kFan;
-    const std::uint32_t members = smin<std::uint32_t>(comm.size - leader, kFan);
-    x = fold_records(s.warp);
-    if (comm.rank != leader) {
-      put_record(comm, comm.rank, lane < 8u ? x.v[0] : lane < 16u ? x.v[1] : x.v[2], x.bits);
-    } else {
-      if (lane > 0) x = Sums{{0.0, 0.0, 0.0}, 0u};
-      if (lane > 0 && lane < members) late = !get_record(comm, leader + lane, x);
-      p = fold_warp(x, bits);
-      put_record(comm, kResidentMaxCtas + leader / kFan, p, bits);
+  } else {
+    // Every CTA reads every CTA's record, 32 a warp (a second hop, through
+    // sums of 12 CTAs each, took an iteration of 60,000 cells from 9.9 to
+    // 12.6 us).
+    if (threadIdx.x < 32) {
+      x = fold_records(s.warp);
+      if (lane < 3u) put_wide(record_of(comm, comm.rank) + lane, comm.round, x.bits, lane == 0u ? x.v[0] : lane == 1u ? x.v[1] : x.v[2]);
     }
+    bool late = false;
     x = Sums{{0.0, 0.0, 0.0}, 0u};
-    if (lane < groups) late = !get_record(comm, kResidentMaxCtas + lane, x) || late;
-    p = fold_warp(x, bits);
-    x = Sums{{__shfl_sync(0xFFFFFFFFu, p, 0), __shfl_sync(0xFFFFFFFFu, p, 8), __shfl_sync(0xFFFFFFFFu, p, 16)}, bits};
-    return !late;
+    if ((threadIdx.x & ~31u) < comm.size) {
+      if (threadIdx.x < comm.size) late = !get_record(comm, threadIdx.x, x);
+      p = fold_warp(x, bits);
+      store_sums(s.parts[threadIdx.x >> 5], p, bits);
+    }
+    if (__syncthreads_or(late) != 0) return false;
+    x = fold_records(s.parts);
   }
   return true;
 }
@@ -486,7 +485,7 @@ __device__ __forceinline__ Sums receive_sides(const SolveDesc& d, const Layout& 
 // CTA's share does not fit `bytes` of shared memory.
 template <int kForm>
 __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm, Shared& s, Layout& l,
-                           std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1, SolveDesc* state) {
+                           std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1, std::uint32_t* check) {
   const std::uint32_t* offsets = r.order != nullptr ? r.order_offsets : d.incidence.offsets;
   const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   std::uint32_t first = b0, last = b1;
@@ -642,39 +641,28 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
           pad_slot(l, l.group(groups - 1) + kGroup * (i / missing) + there + i % missing);
         }
       }
-      if constexpr (kForm == kGrid) {
-        unsigned long long* words = r.inbox + std::size_t(comm.rank) * r.stride;
-        for (std::uint32_t j = threadIdx.x; j < slots; j += kThreads) words[j] = 0ull;
-        for (std::uint32_t i = threadIdx.x; i < 2 * kResidentWords; i += kThreads) {
-          const std::size_t set = std::size_t(i / kResidentWords) * kResidentRecords;
-          r.records[(set + comm.rank) * kResidentWords + i % kResidentWords] = make_ulonglong2(0ull, 0ull);
-          if (comm.rank % kFan == 0) {
-            r.records[(set + kResidentMaxCtas + comm.rank / kFan) * kResidentWords + i % kResidentWords] =
-                make_ulonglong2(0ull, 0ull);
-          }
-        }
-      }
     }
   }
   // Every CTA's slots are known (or one does not fit) from here on.
   if constexpr (kForm == kGrid) {
-    if (threadIdx.x == 0 && s.misfit != 0) atomicExch(&state->misfit, 1u);
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-      atomicAdd(&state->barrier_count, 1u);
-      std::uint32_t polls = 0;
-      while (*static_cast<volatile std::uint32_t*>(&state->barrier_count) < comm.size) {
-        if (++polls == kWaitPolls) {
-          atomicExch(&state->barrier_abort, 1u);
-          s.misfit = 1u;
-          break;
-        }
+      ResidentGang& gang = *comm.gang;
+      if (s.misfit != 0) atomicExch(&gang.misfit, 1u);
+      atomicMax(&gang.base, comm.round);
+      __threadfence();
+      atomicAdd(&gang.arrived, 1u);
+      if (!wait_count(&gang.arrived, comm.size)) {
+        atomicExch(&gang.late, 1u);
+        s.misfit = 1u;
       }
       __threadfence();
-      if (*static_cast<volatile std::uint32_t*>(&state->misfit) != 0u) s.misfit = 1u;
+      if (*static_cast<volatile std::uint32_t*>(&gang.misfit) != 0u) s.misfit = 1u;
+      s.round = *static_cast<volatile std::uint32_t*>(&gang.base);
     }
     __syncthreads();
+    comm.round = s.round;
   } else if constexpr (kForm == kCluster) {
     __threadfence();
     comm.sync_all();
@@ -696,12 +684,12 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
       const std::uint32_t j = base + kGroup * k;
       const std::uint32_t side = __float_as_uint(l.b(j).w);
       std::uint32_t meta = kNobody;
-      if (!index_ok(side >> 1, d.row_count, &state->check_status)) {
+      if (!index_ok(side >> 1, d.row_count, check)) {
         l.inbox(j) = -0.0f;
       } else if ((side & 1u) != 0u || d.rows.slots[side >> 1].y != kInvalidSlot) {
         const std::uint32_t place = r.places[side ^ 1u];
         const std::uint32_t to =
-            index_ok(place, 2ull * d.row_count, &state->check_status) ? __ldcg(&r.slot_of[place]) : comm.rank << 16 | j;
+            index_ok(place, 2ull * d.row_count, check) ? __ldcg(&r.slot_of[place]) : comm.rank << 16 | j;
         const std::uint32_t cta = to >> 16, slot = to & 0xFFFFu;
         if constexpr (kForm == kSingle) {
           meta = slot;
@@ -710,7 +698,7 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
         } else if (cta == comm.rank) {
           meta = slot;
         } else {
-          meta = kRemote | (cta * r.stride + slot);
+          meta = kRemote | ((comm.first + cta) * r.stride + slot);
           l.remote(atomicAdd(&s.remote_count, 1u)) = std::uint16_t(j);
         }
       } else {
@@ -724,20 +712,22 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
   return true;
 }
 
+struct Report {
+  float step, residual, bound;
+  std::uint32_t iterations, status;
+};
+enum Outcome { kSolved, kMisfit, kLate };
+
 // The whole solve of bodies [b0, b1) by the CTAs of `comm`.
 template <int kForm, int P>
-__device__ __forceinline__ void resident_solve(const SolveDesc& d, const ResidentArrays& r, Comm<kForm> comm, Shared& s,
-                               std::uint32_t bytes, SolveDesc* state) {
+__device__ __forceinline__ Outcome resident_solve(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm,
+                                                  Shared& s, std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1,
+                                                  float tolerance, std::uint32_t* check, Report& report) {
   Layout l{};
-  if (!load_share(d, r, comm, s, l, bytes, 0u, d.body_count, state)) {
-    if (kForm != kGrid && comm.rank == 0 && threadIdx.x == 0) state->misfit = 1u;
-    return;
-  }
-  // Every thread takes the same decisions from the same sums (in the grid
-  // form warp 0 does, and the block reads them).  The rounds share one copy
-  // of the code: what a round executes is fetched once per iteration, by few
-  // warps, so its size counts.
-  constexpr bool kBlockDecides = kForm != kGrid;
+  if (!load_share(d, r, comm, s, l, bytes, b0, b1, check)) return kMisfit;
+  // Every thread takes the same decisions from the same sums.  The rounds
+  // share one copy of the code: what a round executes is fetched once per
+  // iteration, by few warps, so its size counts.
   float bound = 0.0f, step = 0.0f, residual = 0.0f;
   std::uint32_t iterations = 0, status = MSB_SOLVE_ITERATION_LIMIT;
   int round = kBound;
@@ -746,51 +736,29 @@ __device__ __forceinline__ void resident_solve(const SolveDesc& d, const Residen
     ++comm.round;
     send_sides<P>(d, l, comm, round, step);
     if (round == kFinal) break;
-    bool arrived = comm.exchange(l, s);
-    if (arrived) {
-      Sums x = receive_sides(d, l, round, step);
-      arrived = reduce(comm, s, x);
-      if (kBlockDecides || threadIdx.x < 32) {
-        const float value = __uint_as_float(x.bits);
-        if (round == kBound) {
-          bound = value;
-          round = kInitial;
-        } else {
-          residual = value;
-          if (round == kInitial && (!isfinite(bound) || !(bound > 0.0f))) {
-            status = 3;  // no positive diagonal: an invalid system
-            round = kFinal;
-          } else if (!isfinite(residual)) {
-            status = MSB_SOLVE_BREAKDOWN;
-            iterations += round == kIterate ? 1u : 0u;
-            round = kFinal;
-          } else if (!(residual > d.tolerance)) {
-            status = MSB_SOLVE_CONVERGED;
-            iterations += round == kIterate ? 1u : 0u;
-            round = kFinal;
-          } else if (round == kInitial) {
-            step = 1.0f / bound;
-            round = d.max_iterations > 0 ? kIterate : kFinal;
-          } else {
-            iterations += 1;
-            step = next_step(step, x.v[0], x.v[1], x.v[2], iterations);
-            round = iterations < d.max_iterations ? kIterate : kFinal;
-          }
-        }
-      }
+    if (!comm.exchange(l, s)) return kLate;
+    Sums x = receive_sides(d, l, round, step);
+    if (!reduce(comm, s, x)) return kLate;
+    const float value = __uint_as_float(x.bits);
+    if (round == kBound) {
+      bound = value;
+      round = kInitial;
+      continue;
     }
-    if constexpr (!kBlockDecides) {
-      if (threadIdx.x == 0) {
-        s.alpha = step;
-        s.round = round;
-      }
-      arrived = __syncthreads_or(!arrived) == 0;
-      step = s.alpha;
-      round = s.round;
-    }
-    if (!arrived) {
-      if (threadIdx.x == 0) atomicExch(&state->barrier_abort, 1u);
-      return;
+    residual = value;
+    iterations += round == kIterate ? 1u : 0u;
+    if (round == kInitial && (!isfinite(bound) || !(bound > 0.0f))) {
+      status = 3;  // no positive diagonal: an invalid system
+      round = kFinal;
+    } else if (!isfinite(residual)) {
+      status = MSB_SOLVE_BREAKDOWN;
+      round = kFinal;
+    } else if (!(residual > tolerance)) {
+      status = MSB_SOLVE_CONVERGED;
+      round = kFinal;
+    } else {
+      step = round == kInitial ? 1.0f / bound : next_step(step, x.v[0], x.v[1], x.v[2], iterations);
+      round = iterations < d.max_iterations ? kIterate : kFinal;
     }
   }
   // The solution (the last round wrote its response).
@@ -807,14 +775,20 @@ __device__ __forceinline__ void resident_solve(const SolveDesc& d, const Residen
       d.iterate[side >> 1] = make_float2(c.z, c.w);
     }
   }
-  if (comm.rank == 0 && threadIdx.x == 0) {
-    state->step = step;
-    state->residual = residual;
-    state->bound = bound;
-    state->iterations = iterations;
-    state->status = status;
-    state->mode = 1;
+  report = {step, residual, bound, iterations, status};
+  return kSolved;
+}
+
+// This CTA's inbox and records before its first gang's first word arrives.
+__device__ void clear_words(const Comm<kGrid>& comm) {
+  const ResidentArrays& r = *comm.arrays;
+  unsigned long long* words = r.inbox + std::size_t(comm.first + comm.rank) * r.stride;
+  for (std::uint32_t j = threadIdx.x; j < r.stride; j += kThreads) words[j] = 0ull;
+  if (threadIdx.x < 2 * kResidentWords) {
+    const std::size_t set = std::size_t(threadIdx.x / kResidentWords) * kResidentMaxCtas;
+    r.records[(set + comm.first + comm.rank) * kResidentWords + threadIdx.x % kResidentWords] = make_ulonglong2(0ull, 0ull);
   }
+  __threadfence();
 }
 
 template <int kForm, int P>
@@ -823,14 +797,91 @@ __global__ void __launch_bounds__(kThreads, 1)
                     SolveDesc* state, std::uint32_t bytes) {
   __shared__ Shared s;
   Comm<kForm> comm{blockIdx.x, gridDim.x, &arrays};
-  resident_solve<kForm, P>(problem, arrays, comm, s, bytes, state);
-  if constexpr (kForm == kCluster) cg::this_cluster().sync();  // no CTA leaves while another may read its sums
+  if constexpr (kForm == kGrid) {
+    comm.gang = &state->gang;
+    clear_words(comm);
+  }
+  Report report;
+  const Outcome outcome = resident_solve<kForm, P>(problem, arrays, comm, s, bytes, 0u, problem.body_count,
+                                                   problem.tolerance, &state->check_status, report);
+  if constexpr (kForm == kCluster) cg::this_cluster().sync();  // no CTA leaves while another may write its sums
+  if (threadIdx.x != 0) return;
+  if (outcome == kLate) atomicExch(&state->gang.late, 1u);
+  if (comm.rank != 0) return;
+  if (outcome == kMisfit) {
+    state->gang.misfit = 1u;
+  } else if (outcome == kSolved) {
+    state->step = report.step;
+    state->residual = report.residual;
+    state->bound = report.bound;
+    state->iterations = report.iterations;
+    state->status = report.status;
+    state->mode = 1;
+  }
+}
+
+// A batch: each CTA takes its jobs in order, with the other CTAs of each
+// job's gang.  Every list is a part of one sequence of all jobs, so the first
+// unfinished job of the sequence always has all of its CTAs.
+__global__ void __launch_bounds__(kThreads, 1)
+    resident_batch_kernel(const __grid_constant__ SolveDesc problem, const __grid_constant__ ResidentArrays arrays,
+                          const __grid_constant__ ResidentBatch batch, std::uint32_t bytes) {
+  __shared__ Shared s;
+  std::uint32_t round = 0;
+  {
+    Comm<kGrid> all{blockIdx.x, gridDim.x, &arrays};
+    clear_words(all);
+  }
+  for (std::uint32_t k = batch.list_offsets[blockIdx.x]; k < batch.list_offsets[blockIdx.x + 1]; ++k) {
+    const ResidentJob job = batch.jobs[batch.lists[k]];
+    const std::uint32_t b0 = batch.cell_offsets[job.colony], b1 = batch.cell_offsets[job.colony + 1];
+    const float tolerance = batch.tolerance[job.colony];
+    Report report{};
+    Outcome outcome;
+    std::uint32_t rank = 0;
+    if (job.size == 1) {
+      Comm<kSingle> comm{0, 1, &arrays};
+      outcome = resident_solve<kSingle, 1>(problem, arrays, comm, s, bytes, b0, b1, tolerance, batch.check, report);
+    } else {
+      Comm<kGrid> comm{blockIdx.x - job.first, job.size, &arrays, job.first, round, &batch.gangs[batch.lists[k]]};
+      outcome = resident_solve<kGrid, 1>(problem, arrays, comm, s, bytes, b0, b1, tolerance, batch.check, report);
+      rank = comm.rank;
+      round = comm.round;
+    }
+    __syncthreads();
+    bool late = outcome == kLate;
+    if (threadIdx.x == 0) {
+      if (rank == 0) {
+        // A colony without rows has no diagonal either, and is converged.
+        const bool empty = batch.row_counts[job.colony] == 0u;
+        ColonyState& to = batch.state[job.colony];
+        if (outcome == kSolved) {
+          to = {report.step, empty ? 0.0f : report.residual, report.bound, report.iterations,
+                empty ? std::uint32_t(MSB_SOLVE_CONVERGED) : report.status};
+        } else {
+          to.status = kResidentMisfit;
+        }
+      }
+      if (job.size > 1 && outcome == kSolved && k + 1 < batch.list_offsets[blockIdx.x + 1]) {
+        // The others may still read this CTA's last record.
+        ResidentGang& gang = batch.gangs[batch.lists[k]];
+        __threadfence();
+        atomicAdd(&gang.left, 1u);
+        late = !wait_count(&gang.left, job.size);
+      } else if (job.size > 1) {
+        atomicAdd(&batch.gangs[batch.lists[k]].left, 1u);
+      }
+      if (late) atomicExch(batch.late, 1u);
+    }
+    if (__syncthreads_or(late) != 0) return;
+  }
 }
 
 // Eight bits of each of x and y, interleaved; both axes at the scale of the
 // longer one.
 __global__ void spatial_keys_kernel(std::uint32_t n, const float4* __restrict__ pos_len, const GridParams* grid_ptr,
-                                    std::uint32_t* __restrict__ keys, std::uint32_t* __restrict__ order) {
+                                    const std::uint32_t* __restrict__ colony, std::uint32_t* __restrict__ keys,
+                                    std::uint32_t* __restrict__ order) {
   const double wx = grid_ptr->inv_width[0], wy = grid_ptr->inv_width[1];
   const double x0 = grid_ptr->low[0], y0 = grid_ptr->low[1];
   const double scale = 256.0 / fmax(double(grid_ptr->dims[0]) / wx, double(grid_ptr->dims[1]) / wy);
@@ -842,7 +893,8 @@ __global__ void spatial_keys_kernel(std::uint32_t n, const float4* __restrict__ 
       v = (v | (v << 2)) & 0x3333u;
       return (v | (v << 1)) & 0x5555u;
     };
-    keys[i] = spread(cell(double(p.x) - x0)) | spread(cell(double(p.y) - y0)) << 1;
+    keys[i] = spread(cell(double(p.x) - x0)) | spread(cell(double(p.y) - y0)) << 1 |
+              (colony != nullptr ? colony[i] << 16 : 0u);
     order[i] = i;
   }
 }
@@ -904,11 +956,12 @@ int launch_lanes(const SolveDesc& problem, SolveDesc* desc, const ResidentArrays
 
 }  // namespace
 
-void launch_spatial_order(std::uint32_t n, const float4* pos_len, const GridParams* grid, std::uint32_t* keys,
-                          std::uint32_t* order, std::uint32_t* temp, cudaStream_t stream) {
-  spatial_keys_kernel<<<grid_for(n, 256), 256, 0, stream>>>(n, pos_len, grid, keys, order);
+void launch_spatial_order(std::uint32_t n, const float4* pos_len, const GridParams* grid, const std::uint32_t* colony,
+                          std::uint32_t colonies, std::uint32_t* keys, std::uint32_t* order, std::uint32_t* temp,
+                          cudaStream_t stream) {
+  spatial_keys_kernel<<<grid_for(n, 256), 256, 0, stream>>>(n, pos_len, grid, colony, keys, order);
   count_launch();
-  radix_sort_pairs(keys, order, n, 16, temp, stream);
+  radix_sort_pairs(keys, order, n, 16 + (colony != nullptr ? int(std::bit_width(colonies - 1)) : 0), temp, stream);
 }
 
 void launch_order_offsets(std::uint32_t n, const std::uint32_t* order, const std::uint32_t* offsets,
@@ -945,10 +998,38 @@ ResidentLimits resident_limits() {
   return limits;
 }
 
+// What a CTA can hold, less 3 % for the slots that pad the groups of bodies.
+constexpr std::uint64_t kShareBytes = std::uint64_t(kDynamicBytes) * 97 / 100;
+constexpr std::uint64_t system_bytes(std::uint64_t rows, std::uint64_t bodies) {
+  return 2 * rows * kEntryBytes + bodies * kBodyBytes;
+}
+
+std::uint32_t resident_ctas(std::uint64_t rows, std::uint64_t bodies) {
+  return std::uint32_t(std::min<std::uint64_t>((system_bytes(rows, bodies) + kShareBytes - 1) / kShareBytes, 1u << 30));
+}
+
+int launch_resident_batch(const SolveDesc& problem, const ResidentArrays& arrays, const ResidentBatch& batch, int ctas,
+                          cudaStream_t stream) {
+  cudaError_t e = cudaFuncSetAttribute(resident_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       int(kDynamicBytes));
+  if (e != cudaSuccess) return int(e);
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(unsigned(ctas));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kDynamicBytes;
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeCooperative;
+  attribute.val.cooperative = 1;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  count_launch();
+  return int(cudaLaunchKernelEx(&config, resident_batch_kernel, problem, arrays, batch, kDynamicBytes));
+}
+
 ResidentPlan resident_plan(const ResidentLimits& limits, std::uint64_t rows, std::uint64_t bodies) {
-  const std::uint64_t bytes = 2 * rows * kEntryBytes + bodies * kBodyBytes;
-  // 3 % for the slots that pad the groups of bodies.
-  const std::uint64_t share = std::uint64_t(kDynamicBytes) * 97 / 100;
+  const std::uint64_t bytes = system_bytes(rows, bodies);
+  const std::uint64_t share = kShareBytes;
   ResidentPlan plan;
   if (bytes <= share * 3 / 4 || (limits.cluster == 0 && bytes <= share)) {
     plan = {1, false, 1};

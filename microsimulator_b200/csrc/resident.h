@@ -4,6 +4,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "batch.h"
 #include "solve.h"
 
 namespace msb {
@@ -13,7 +14,7 @@ struct ResidentArrays {
   const std::uint32_t* places;  // per side (row << 1 | side): its entry's place in the incidence
   std::uint32_t* slot_of;       // per entry: CTA << 16 | slot in that CTA's shared memory
   unsigned long long* inbox;    // grid form: (round, side term) words, `stride` per CTA
-  ulonglong2* records;          // grid form: two sets of kResidentRecords records of sums
+  ulonglong2* records;          // grid form: two sets of a record of sums per CTA
   std::uint32_t stride;
   // Bodies in the order in which CTAs take them, and the entries before each
   // in that order (bodies + 1); null: by slot.
@@ -22,7 +23,6 @@ struct ResidentArrays {
 };
 
 constexpr std::uint32_t kResidentMaxCtas = 160;  // grid form at most
-constexpr std::uint32_t kResidentRecords = kResidentMaxCtas + 16;  // one per CTA and one per group of CTAs
 constexpr std::uint32_t kResidentWords = 4;                        // 16-byte words a record
 
 // What the device takes: the largest cluster, and the CTAs of a cooperative
@@ -45,18 +45,19 @@ struct ResidentPlan {
 //   1,148 rows, 300 bodies      one CTA 3.6, a cluster of 16 3.8; graph 15.6
 //   7,000 rows, 1,000 bodies    clusters of 4, 8 and 16 6.6, 5.4 and 4.6, 32
 //                               CTAs of a grid 9.3; graph 23.2
-//   82,000 rows, 20,011 bodies  148 CTAs 8.4 with 4 lanes a body, 11.5 with 1
-//                               (7.3 in spatial order); graph 18.8
-//   247,000 rows, 60,000 bodies 148 CTAs 15.7 with 1 lane a body, 17.2 with 4
-//                               (12.6 in spatial order); graph 23.1
-//   221,000 rows, 100,000 bodies in a trap  148 CTAs 15.5, 9.0 in spatial
-//                               order; graph 21.7
+//   82,000 rows, 20,011 bodies  148 CTAs 7.6 with 4 lanes a body; graph 18.8
+//   247,000 rows, 60,000 bodies 148 CTAs 9.9 with 1 lane a body; graph 23.1
+//   221,000 rows, 100,000 bodies in a trap  148 CTAs 8.8; graph 21.7
+// (bodies by slot, not in spatial order: 8.4, 15.7 and 15.5; 4 lanes a body
+// where 1 is taken: 17.2 and 10.5 in spatial order.)
 ResidentPlan resident_plan(const ResidentLimits& limits, std::uint64_t rows, std::uint64_t bodies);
-// The bodies along a Morton curve over their centres (16 bits of key), so
-// that a CTA of the grid form holds neighbours and few side terms leave it.
-// `temp` holds sort_temp_words(n) words.
-void launch_spatial_order(std::uint32_t n, const float4* pos_len, const GridParams* grid, std::uint32_t* keys,
-                          std::uint32_t* order, std::uint32_t* temp, cudaStream_t stream);
+// The bodies along a Morton curve over their centres (16 bits of key; with
+// `colony`, colony by colony, at most 65,536), so that a CTA of the grid form
+// holds neighbours and few side terms leave it.  `temp` holds
+// sort_temp_words(n) words.
+void launch_spatial_order(std::uint32_t n, const float4* pos_len, const GridParams* grid, const std::uint32_t* colony,
+                          std::uint32_t colonies, std::uint32_t* keys, std::uint32_t* order, std::uint32_t* temp,
+                          cudaStream_t stream);
 // The entries before each body in `order`; counts: n + 1 words, temp:
 // scan_temp_words(n + 1).
 void launch_order_offsets(std::uint32_t n, const std::uint32_t* order, const std::uint32_t* offsets,
@@ -73,5 +74,34 @@ std::uint32_t resident_stride();
 int launch_resident(const SolveDesc& problem, SolveDesc* desc, const ResidentArrays& arrays, ResidentPlan plan,
                     cudaStream_t stream);
 constexpr std::uint32_t kResidentDegree = 62;
+
+// A batch of independent colonies in one launch: each colony is the job of a
+// gang of neighbouring CTAs that holds it, and each CTA takes its jobs in the
+// order of `jobs`.  On one cluster of 16 CTAs the largest colony sets a
+// solve's time while the other clusters idle (20,000 cells: about 55 us an
+// iteration); a gang of 46 CTAs takes 8 us.  64 colonies of 500-20,000 cells:
+// solve phase 52 -> 26 ms a step.
+struct ResidentJob {
+  std::uint32_t colony;
+  std::uint32_t first;  // the gang's CTAs: first, first + 1, ...
+  std::uint32_t size;
+};
+struct ResidentBatch {
+  const ResidentJob* jobs;
+  ResidentGang* gangs;                // one per job, zero at launch
+  const std::uint32_t* list_offsets;  // CTAs + 1: each CTA's jobs in `lists`
+  const std::uint32_t* lists;
+  const std::uint32_t* cell_offsets;
+  const std::uint32_t* row_counts;
+  const float* tolerance;
+  ColonyState* state;  // status kResidentMisfit: the colony's share did not fit, nothing was done
+  std::uint32_t* check;
+  std::uint32_t* late;  // set once a wait has run out
+};
+constexpr std::uint32_t kResidentMisfit = 0xFFFFFFFFu;
+// CTAs that hold a system.
+std::uint32_t resident_ctas(std::uint64_t rows, std::uint64_t bodies);
+int launch_resident_batch(const SolveDesc& problem, const ResidentArrays& arrays, const ResidentBatch& batch, int ctas,
+                          cudaStream_t stream);
 
 }  // namespace msb

@@ -59,6 +59,17 @@ struct IncidenceArrays {
   std::uint32_t* places;
 };
 
+// Where the CTAs of a resident solve meet: how many hold their shares and how
+// many are done, the round they count from (the largest of their own), and
+// whether a share did not fit (nothing was done) or a wait ran out.
+struct ResidentGang {
+  std::uint32_t arrived;
+  std::uint32_t left;
+  std::uint32_t base;
+  std::uint32_t misfit;
+  std::uint32_t late;
+};
+
 // Everything one solve reads and writes, in device memory at a fixed address
 // so that the captured solve graph can be replayed for any system.
 struct SolveDesc {
@@ -100,7 +111,7 @@ struct SolveDesc {
   std::uint32_t barrier_generation;
   std::uint32_t barrier_abort;  // a barrier wait ran out of time: every block stops
   std::uint32_t check_status;   // checked build: the first index check that failed (0: none)
-  std::uint32_t misfit;         // a resident solve whose shares did not fit: nothing was done
+  ResidentGang gang;            // the resident solve's
 };
 
 // Builds the incidence of `rows` over `bodies` bodies.  Scratch: `keys` and

@@ -13,6 +13,7 @@ import pytest
 
 from microsimulator_b200 import abi, workloads
 from microsimulator_b200.backend import B200Backend
+from microsimulator_b200.sweep import ColonyBatch
 from microsimulator_b200.types import ContactDynamicsParameters, ContactSolveParameters, ContactSystem
 from tests.systems import LAWS, mixed_system, multipliers_for
 
@@ -108,3 +109,29 @@ def test_steps_in_spatial_order(forms, cells, flat):
     (a, ra), (b, rb) = results
     assert ra.substeps == rb.substeps and ra.halvings == rb.halvings
     assert np.max(np.abs(a.geometry() - b.geometry())) <= 4 * p.overlap_tolerance
+
+
+def test_batch_by_gangs_steps_as_by_clusters(backend):
+    """Colonies held by one CTA, by gangs of several and (one body touching
+    more than 62 rows) by none, against the clusters' solve: the same rows,
+    geometry within four solve tolerances."""
+    sizes = [1, 2, 40, 300, 900, 3000, 12000]
+    worlds = [workloads.sweep_colony(n, seed=n) for n in sizes]
+    star = workloads.sweep_colony(120, seed=9)
+    star.position_x[:], star.position_y[:] = star.position_x * 0.02, star.position_y * 0.02
+    batch = ColonyBatch([*worlds, star], np.full(8, 1.0), np.full(8, 1.0e4))
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4)
+    counts = batch.counts()
+    results = []
+    with B200Backend(0) as b:
+        b.advance_contact_dynamics_batch(batch.concatenated(), counts, batch.drag, batch.stiffness, 0.002, p)  # tunes
+        for form in (B200Backend.RELAXATION_AUTOMATIC, B200Backend.RELAXATION_GRAPH):
+            b.set_relaxation(form)
+            cells = batch.concatenated()
+            report, colonies = b.advance_contact_dynamics_batch(cells, counts, batch.drag, batch.stiffness, 0.002, p)
+            results.append((cells.geometry(), report, colonies))
+    (a, ra, ca), (g, rg, cg) = results
+    assert ra.substeps == rg.substeps
+    assert np.array_equal(ca["rows"], cg["rows"])
+    assert np.array_equal(ca["status"], cg["status"])
+    assert np.max(np.abs(a - g)) <= 4 * p.overlap_tolerance
