@@ -71,10 +71,14 @@ __device__ std::uint32_t external_contact_reason(const msb_external_contact& c, 
 }
 
 // Checks each contact and counts the entries of each slot (valid contacts
-// only, so that every counted slot is in range).
+// only, so that every counted slot is in range).  The counts as they were
+// before each contact's entries are their ranks within their slots, kept as
+// two bytes for the scatter (which takes no list with a segment longer than
+// kSegmentLimit), so that one atomic per entry serves both passes.
 template <bool External>
 __global__ void validate_kernel(const void* __restrict__ records, std::uint64_t count, std::uint64_t cell_count,
-                                unsigned long long* words, std::uint32_t* __restrict__ counts) {
+                                unsigned long long* words, std::uint32_t* __restrict__ counts,
+                                std::uint16_t* __restrict__ ranks) {
   unsigned long long largest = 0;
   for (std::uint64_t i = blockIdx.x * std::uint64_t(blockDim.x) + threadIdx.x; i < count;
        i += std::uint64_t(gridDim.x) * blockDim.x) {
@@ -82,14 +86,15 @@ __global__ void validate_kernel(const void* __restrict__ records, std::uint64_t 
     if constexpr (External) {
       const msb_external_contact& c = static_cast<const msb_external_contact*>(records)[i];
       reason = external_contact_reason(c, cell_count);
-      if (reason == 0) atomicAdd(&counts[c.cell_slot], 1u);
+      if (reason == 0) ranks[i] = std::uint16_t(atomicAdd(&counts[c.cell_slot], 1u) & 0xFFu);
     } else {
       const msb_cell_contact& c = static_cast<const msb_cell_contact*>(records)[i];
       reason = cell_contact_reason(c, cell_count);
       largest = smax<unsigned long long>(largest, c.second_id);
       if (reason == 0) {
-        atomicAdd(&counts[c.first_slot], 1u);
-        atomicAdd(&counts[c.second_slot], 1u);
+        const std::uint32_t a = atomicAdd(&counts[c.first_slot], 1u) & 0xFFu;
+        const std::uint32_t b = atomicAdd(&counts[c.second_slot], 1u) & 0xFFu;
+        ranks[i] = std::uint16_t(a | b << 8);
       }
     }
     if (reason != 0) atomicMin(&words[0], (static_cast<unsigned long long>(i) << 8) | reason);
@@ -222,22 +227,22 @@ __global__ void largest_count_kernel(const std::uint32_t* __restrict__ counts, s
   if ((threadIdx.x & 31) == 0 && m != 0) atomicMax(largest, static_cast<unsigned long long>(m));
 }
 
-// Each entry to a free place in its slot's range (counts run back to zero):
-// its contact index and, for a neighbour index, the partner's id beside it
+// Each entry to its place in its slot's range: its contact index and, for a neighbour index, the partner's id beside it
 // (read here from the same 32-byte sector as the slots).
 template <bool External, bool Neighbors>
 __global__ void scatter_entries_kernel(const void* __restrict__ records, std::uint64_t count,
-                                       const std::uint32_t* __restrict__ starts, std::uint32_t* __restrict__ counts,
-                                       std::uint32_t* __restrict__ entries, std::uint64_t* __restrict__ partners) {
+                                       const std::uint32_t* __restrict__ starts,
+                                       const std::uint16_t* __restrict__ ranks, std::uint32_t* __restrict__ entries, std::uint64_t* __restrict__ partners) {
   for (std::uint64_t i = blockIdx.x * std::uint64_t(blockDim.x) + threadIdx.x; i < count;
        i += std::uint64_t(gridDim.x) * blockDim.x) {
     if constexpr (External) {
       const std::uint32_t slot = static_cast<const msb_external_contact*>(records)[i].cell_slot;
-      entries[starts[slot] + atomicSub(&counts[slot], 1u) - 1u] = std::uint32_t(i);
+      entries[starts[slot] + ranks[i]] = std::uint32_t(i);
     } else {
       const msb_cell_contact& c = static_cast<const msb_cell_contact*>(records)[i];
-      const std::uint32_t a = starts[c.first_slot] + atomicSub(&counts[c.first_slot], 1u) - 1u;
-      const std::uint32_t b = starts[c.second_slot] + atomicSub(&counts[c.second_slot], 1u) - 1u;
+      const std::uint32_t rank = ranks[i];
+      const std::uint32_t a = starts[c.first_slot] + (rank & 0xFFu);
+      const std::uint32_t b = starts[c.second_slot] + (rank >> 8);
       entries[a] = std::uint32_t(i);
       entries[b] = std::uint32_t(i);
       if constexpr (Neighbors) {
@@ -288,31 +293,31 @@ constexpr int kRegisterSegment = 16;
 // One slot's segment [begin, begin + k): its contact indices sorted into
 // `incidence`; with neighbours, its partner ids sorted, made distinct and
 // written at the front of the same range of `distinct`.  Returns the
-// distinct count.
-template <bool Neighbors>
+// distinct count.  N: the network's width, at least k.
+template <bool Neighbors, int N>
 __device__ __forceinline__ std::uint32_t register_segment(const std::uint32_t* __restrict__ entries,
                                                           const std::uint64_t* __restrict__ partners,
                                                           std::uint32_t begin, std::uint32_t k,
                                                           std::uint64_t* __restrict__ incidence,
                                                           std::uint64_t* __restrict__ distinct) {
-  std::uint32_t e[kRegisterSegment];
+  std::uint32_t e[N];
 #pragma unroll
-  for (int j = 0; j < kRegisterSegment; ++j) e[j] = std::uint32_t(j) < k ? entries[begin + j] : 0xFFFFFFFFu;
+  for (int j = 0; j < N; ++j) e[j] = std::uint32_t(j) < k ? entries[begin + j] : 0xFFFFFFFFu;
   bitonic_sort(e);
 #pragma unroll
-  for (int j = 0; j < kRegisterSegment; ++j) {
+  for (int j = 0; j < N; ++j) {
     if (std::uint32_t(j) < k) incidence[begin + j] = e[j];
   }
   if constexpr (!Neighbors) {
     return 0;
   } else {
-    std::uint64_t p[kRegisterSegment];
+    std::uint64_t p[N];
 #pragma unroll
-    for (int j = 0; j < kRegisterSegment; ++j) p[j] = std::uint32_t(j) < k ? partners[begin + j] : ~0ull;
+    for (int j = 0; j < N; ++j) p[j] = std::uint32_t(j) < k ? partners[begin + j] : ~0ull;
     bitonic_sort(p);
     std::uint32_t u = 0;
 #pragma unroll
-    for (int j = 0; j < kRegisterSegment; ++j) {
+    for (int j = 0; j < N; ++j) {
       if (std::uint32_t(j) < k && (j == 0 || p[j] != p[j - 1])) distinct[begin + u++] = p[j];
     }
     return u;
@@ -344,26 +349,38 @@ __device__ __noinline__ std::uint32_t local_segment(const std::uint32_t* __restr
 }
 
 // One thread per slot: its contacts in contact order (the incidence) and,
-// with neighbours, its distinct partner ids with their count.
+// with neighbours, its distinct partner ids with their count.  A warp takes
+// the narrowest network that holds its longest segment: 16 wide the two
+// sorts of a thread are 160 exchanges, 4 wide 12.
 template <bool Neighbors>
 __global__ void __launch_bounds__(kThreads) segment_kernel(
     const std::uint32_t* __restrict__ starts, const std::uint32_t* __restrict__ entries,
     const std::uint64_t* __restrict__ partners, std::uint64_t cell_count,
     std::uint64_t* __restrict__ incidence_offsets, std::uint64_t* __restrict__ incidence,
     std::uint64_t* __restrict__ distinct, std::uint32_t* __restrict__ distinct_counts) {
-  for (std::uint64_t s = blockIdx.x * std::uint64_t(blockDim.x) + threadIdx.x; s <= cell_count;
-       s += std::uint64_t(gridDim.x) * blockDim.x) {
-    const std::uint32_t begin = starts[s];
-    incidence_offsets[s] = begin;
-    if (s == cell_count) {
-      if constexpr (Neighbors) distinct_counts[s] = 0;
-      continue;
+  const std::uint64_t stride = std::uint64_t(gridDim.x) * blockDim.x;
+  for (std::uint64_t s0 = blockIdx.x * std::uint64_t(blockDim.x) + (threadIdx.x & ~31u); s0 <= cell_count; s0 += stride) {
+    const std::uint64_t s = s0 + (threadIdx.x & 31u);
+    std::uint32_t begin = 0, k = 0;
+    if (s <= cell_count) {
+      begin = starts[s];
+      incidence_offsets[s] = begin;
+      if (s < cell_count) k = starts[s + 1] - begin;
     }
-    const std::uint32_t k = starts[s + 1] - begin;
-    const std::uint32_t u = k <= std::uint32_t(kRegisterSegment)
-                                ? register_segment<Neighbors>(entries, partners, begin, k, incidence, distinct)
-                                : local_segment<Neighbors>(entries, partners, begin, k, incidence, distinct);
-    if constexpr (Neighbors) distinct_counts[s] = u;
+    const std::uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, k);
+    std::uint32_t u = 0;
+    if (longest <= 4u) {
+      u = register_segment<Neighbors, 4>(entries, partners, begin, k, incidence, distinct);
+    } else if (longest <= 8u) {
+      u = register_segment<Neighbors, 8>(entries, partners, begin, k, incidence, distinct);
+    } else if (k <= std::uint32_t(kRegisterSegment)) {
+      u = register_segment<Neighbors, kRegisterSegment>(entries, partners, begin, k, incidence, distinct);
+    } else {
+      u = local_segment<Neighbors>(entries, partners, begin, k, incidence, distinct);
+    }
+    if constexpr (Neighbors) {
+      if (s <= cell_count) distinct_counts[s] = u;
+    }
   }
 }
 
@@ -470,10 +487,15 @@ void build_neighbors(const void* contacts, std::uint64_t count, std::uint64_t ce
 
 }  // namespace
 
-std::uint64_t graph_scratch_words(std::uint64_t entries, std::uint64_t cell_count) {
+// The contacts' ranks (two bytes each) follow everything else.
+static std::uint64_t ranks_at(std::uint64_t entries, std::uint64_t cell_count) {
   const Layout l{cell_count + 1, entries};
   const std::uint64_t rest = l.short_words() > l.radix_words() ? l.short_words() : l.radix_words();
   return ((l.slots + 1) & ~1ull) + rest + 64;
+}
+
+std::uint64_t graph_scratch_words(std::uint64_t entries, std::uint64_t cell_count) {
+  return ranks_at(entries, cell_count) + entries / 2 + 1;
 }
 
 void launch_validate_contacts(const void* contacts, std::uint64_t count, std::uint64_t cell_count, bool external,
@@ -482,12 +504,13 @@ void launch_validate_contacts(const void* contacts, std::uint64_t count, std::ui
   cudaMemsetAsync(words + 1, 0, 3 * sizeof(unsigned long long), stream);
   cudaMemsetAsync(scratch, 0, (cell_count + 1) * sizeof(std::uint32_t), stream);
   if (count == 0) return;
+  auto* ranks = reinterpret_cast<std::uint16_t*>(scratch + ranks_at(external ? count : 2 * count, cell_count));
   if (external) {
     validate_kernel<true><<<grid_for(count, kThreads), kThreads, 0, stream>>>(contacts, count, cell_count, words,
-                                                                             scratch);
+                                                                             scratch, ranks);
   } else {
     validate_kernel<false><<<grid_for(count, kThreads), kThreads, 0, stream>>>(contacts, count, cell_count, words,
-                                                                              scratch);
+                                                                              scratch, ranks);
   }
   count_launch();
   largest_count_kernel<<<grid_for(cell_count, kThreads), kThreads, 0, stream>>>(scratch, cell_count, words + 3);
@@ -518,17 +541,18 @@ void build_graph_index(const void* contacts, std::uint64_t count, std::uint64_t 
   std::uint32_t* places = distinct_counts + l.slots;
   std::uint32_t* entries = places + l.slots;
   std::uint32_t* temp = entries + l.entries;
+  const auto* ranks = reinterpret_cast<const std::uint16_t*>(scratch + ranks_at(l.entries, cell_count));
   exclusive_scan(counts, starts, l.slots, temp, stream);
   const int grid = grid_for(count, kThreads);
   if (count > 0) {
     if (external) {
-      scatter_entries_kernel<true, false><<<grid, kThreads, 0, stream>>>(contacts, count, starts, counts, entries,
+      scatter_entries_kernel<true, false><<<grid, kThreads, 0, stream>>>(contacts, count, starts, ranks, entries,
                                                                         nullptr);
     } else if (neighbors) {
-      scatter_entries_kernel<false, true><<<grid, kThreads, 0, stream>>>(contacts, count, starts, counts, entries,
+      scatter_entries_kernel<false, true><<<grid, kThreads, 0, stream>>>(contacts, count, starts, ranks, entries,
                                                                         partners);
     } else {
-      scatter_entries_kernel<false, false><<<grid, kThreads, 0, stream>>>(contacts, count, starts, counts, entries,
+      scatter_entries_kernel<false, false><<<grid, kThreads, 0, stream>>>(contacts, count, starts, ranks, entries,
                                                                          nullptr);
     }
     count_launch();
