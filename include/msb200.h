@@ -451,13 +451,15 @@ int msb_set_search_reuse(msb_context* context, uint32_t mode);
 /* The form of the BB relaxation on the device (no counterpart in the
  * reference, whose CUDA backend synchronises with the host every iteration,
  * cpp/cuda/cuda_backend.cu:1397-1400):
- *   0  automatic (the default): 1, which measures faster at every size;
+ *   0  automatic (the default): systems that fit in the device's shared memory
+ *      run their whole relaxation in one launch there; larger ones of a step
+ *      run 1's graph over tiles of neighbouring bodies; others run 1;
  *   1  a CUDA graph: bound, initial gaps, then a WHILE node repeating a body
  *      pass and a row pass kernel, whose last block sets the condition;
  *   2  fused: one persistent cooperative kernel runs the whole solve, with
  *      two grid barriers per iteration (bounded waits; a wait that runs out
  *      fails the call with MSB_ERR_DEVICE_CHECK).
- * Both run the same arithmetic per pass and converge to the same tolerance;
+ * All run the same arithmetic per row and body and converge to the same tolerance;
  * the block count they reduce the BB products over can differ, so step
  * lengths can differ in the last bits. */
 int msb_set_relaxation(msb_context* context, uint32_t form);

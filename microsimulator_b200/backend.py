@@ -129,7 +129,8 @@ class B200Backend:
     RELAXATION_FUSED = 2
 
     def set_relaxation(self, form: int) -> None:
-        """The BB relaxation's form on the device: 0 automatic, 1 a CUDA
+        """The BB relaxation's form on the device: 0 automatic (resident in
+        shared memory, or a graph over tiles of neighbouring bodies), 1 a CUDA
         graph with a WHILE node (two kernels per iteration), 2 one persistent
         cooperative kernel with grid barriers."""
         self._check(self._lib.msb_set_relaxation(self._handle, form))

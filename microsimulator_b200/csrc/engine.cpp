@@ -37,6 +37,7 @@
 #include "resident.h"
 #include "solve.h"
 #include "step.h"
+#include "tiles.h"
 #include "mlp.h"
 
 namespace msb {
@@ -190,11 +191,11 @@ constexpr std::uint32_t kWarmCarry = 1;       // the previous step's final force
 constexpr std::uint32_t kWarmGuess = 2;    // forces that a motion guess asks of each body
 constexpr std::uint32_t kWarmLearned = 4;  // the warm-start network makes the motion guess
 constexpr std::uint32_t kWarmFlags = kWarmCarry | kWarmGuess | kWarmLearned;
-// Systems up to this many rows (or bodies) take the fused relaxation when the
-// form is automatic; larger ones the graph.  Measured on B200 the graph is
-// faster at every size (per iteration: 116 against 149 us at 1M capsules,
-// 24 against 28 us at 100k, 19 against 22 us at 20k), so automatic is the
-// graph.
+// Systems up to this many rows (or bodies) that are neither resident nor
+// tiled take the fused relaxation when the form is automatic; larger ones the
+// graph.  Measured on B200 the graph is faster at every size (per iteration:
+// 116 against 149 us at 1M capsules, 24 against 28 us at 100k, 19 against
+// 22 us at 20k), so none do.
 constexpr std::uint32_t kFusedRelaxationItems = 0;
 // The substep's first search pads its candidate boxes by this much more
 // than the candidate margin, so that its candidates serve the overlap
@@ -559,6 +560,14 @@ struct msb_context {
   // grid form; valid within a substep of one system.
   msb::DBuf<std::uint32_t> spatial_keys, spatial_order, spatial_offsets;
   bool spatial_valid = false;
+  // The tiled solve's renumbered system (tiles.h) and its graph.
+  msb::DBuf<std::uint32_t> tile_order, tile_place_of, tile_slots, tile_slot_base, tile_group, tile_row_counts,
+      tile_row_start, tile_row_base, tile_guest_counts, tile_guest_start, tile_guest_base, tile_guests, tile_row_of, tile_new_of, tile_flags, tile_positions, tile_boundary, tile_report;
+  msb::DBuf<std::uint8_t> tile_degree;
+  msb::DBuf<float4> tile_a, tile_b, tile_body_a, tile_body_b;
+  msb::DBuf<float2> tile_constants, tile_iterate;
+  msb::DBuf<float> tile_first, tile_second;
+  std::array<std::unique_ptr<msb::SolveGraph>, 5> tile_graphs;  // by blocks an SM
   // A batch's schedule: jobs, gangs, each CTA's list.
   msb::DBuf<msb::ResidentJob> batch_jobs;
   msb::DBuf<msb::ResidentGang> batch_gangs;
@@ -590,6 +599,7 @@ struct msb_context {
 
   // solve
   int last_blocks = 0;
+  int last_tiled = 0;  // the last solved system was taken by tiles, this many blocks an SM
   msb::SolveDesc* desc = nullptr;
   msb::DBuf<double> partials;
   std::vector<std::unique_ptr<msb::SolveGraph>> graphs;
@@ -1322,9 +1332,74 @@ bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_r
   if (c.host_desc->gang.late != 0) throw DeviceCheckError("a wait of the resident solve ran out of time");
   if (c.host_desc->check_status != 0) throw DeviceCheckError("an index check of the resident solve failed");
   c.last_blocks = grid_for(std::max(c.rows.count, c.n), kSolveThreads, 4);
+  c.last_tiled = 0;
   return c.host_desc->gang.misfit == 0;
 }
 
+// Renumbers c.rows by tiles of c.spatial_order into `out`; returns how many
+// blocks of the tile pass share an SM, 0 when a body or a tile has too many
+// rows.
+int build_tiles(Ctx& c, TileArrays& out) {
+  const std::uint32_t n = c.n, rows = c.rows.count;
+  const std::uint32_t tiles = (n + kTileBodies - 1) / kTileBodies;
+  const std::uint64_t slots = tile_slot_capacity(2ull * rows, tiles);
+  if (slots > 0xFFFFFFFFull) return 0;
+  c.tile_order.ensure(n);
+  c.tile_place_of.ensure(n);
+  c.tile_degree.ensure(n);
+  c.tile_slots.ensure(tiles + 1ull);
+  c.tile_slot_base.ensure(tiles + 1ull);
+  c.tile_group.ensure(n / 8 + 64ull);
+  c.tile_a.ensure(slots);
+  c.tile_b.ensure(slots);
+  c.tile_body_a.ensure(n);
+  c.tile_body_b.ensure(n);
+  c.tile_row_counts.ensure(n + 1ull);
+  c.tile_row_start.ensure(n + 1ull);
+  c.tile_row_base.ensure(tiles + 1ull);
+  c.tile_row_of.ensure(rows);
+  c.tile_new_of.ensure(rows);
+  c.tile_constants.ensure(rows + 2ull);  // the copies of a tile's rows start and end on 16 bytes
+  c.tile_iterate.ensure(rows + 2ull);
+  c.tile_flags.ensure(rows + 1ull);
+  c.tile_positions.ensure(rows + 1ull);
+  c.tile_boundary.ensure(rows);
+  c.tile_first.ensure(rows);
+  c.tile_second.ensure(rows);
+  c.tile_report.ensure(4);
+  c.tile_guest_counts.ensure(n + 1ull);
+  c.tile_guest_start.ensure(n + 1ull);
+  c.tile_guest_base.ensure(tiles + 1ull);
+  c.tile_guests.ensure(rows + 1ull);
+  c.temp.ensure(scan_temp_words(std::max<std::uint64_t>(n, rows) + 1) + 64);
+  const TileBuild build{c.tile_order.p,      c.tile_place_of.p,  c.tile_degree.p,    c.tile_slots.p,
+                        c.tile_slot_base.p,  c.tile_group.p,     c.tile_a.p,         c.tile_b.p,
+                        c.tile_body_a.p,     c.tile_body_b.p,    c.tile_row_counts.p, c.tile_row_start.p,
+                        c.tile_row_base.p,   c.tile_guest_counts.p, c.tile_guest_start.p, c.tile_guest_base.p,
+                        c.tile_guests.p,     c.tile_row_of.p,    c.tile_new_of.p,    c.tile_constants.p,
+                        c.tile_iterate.p,    c.tile_flags.p,     c.tile_positions.p, c.tile_boundary.p,
+                        c.tile_report.p};
+  launch_tile_build(n, rows, c.spatial_order.p, c.rows.slots.p, incidence_arrays(c),
+                    {c.body_a.p, c.body_b.p, c.drift_a.p, c.drift_b.p}, c.rows.keyed_offsets.p, c.rows.keyed_rows.p,
+                    c.rows.multipliers.p, build, c.temp.p, c.stream);
+  check(cudaMemcpyAsync(&c.host_scalars[kScalarCount + 6], c.tile_report.p, 16, cudaMemcpyDeviceToHost, c.stream),
+        "read");
+  const std::uint32_t boundary = read_u32(c, c.tile_positions.p + rows);
+  if (c.host_scalars[kScalarCount + 6] != 0u) return 0;
+  const std::uint32_t max_slots = c.host_scalars[kScalarCount + 7], max_rows = c.host_scalars[kScalarCount + 8],
+                      max_locals = c.host_scalars[kScalarCount + 9];
+  out = {c.tile_order.p,    c.tile_degree.p,   c.tile_slot_base.p, c.tile_group.p,     c.tile_a.p,
+         c.tile_b.p,        c.tile_body_a.p,   c.tile_body_b.p,    c.tile_row_base.p,  c.tile_guest_base.p,
+         c.tile_guests.p,   c.tile_row_of.p,   c.tile_constants.p, c.tile_iterate.p,   c.tile_first.p,
+         c.tile_second.p,   c.tile_boundary.p, tiles,              boundary,           max_slots,
+         max_rows,          max_locals};
+  return tile_blocks_per_sm(max_slots, max_rows, max_locals);
+}
+
+// Systems too large to be resident take the tiled passes where the substep
+// has a spatial order (per iteration against the two passes by slot: 1M
+// capsules in tracks, 4.15M rows, 113 against 187 us; 1M at random, 2.65M
+// rows, 94 against 103; 300k at random, 782,000 rows, 31 against 37).
 SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, float tolerance,
                    std::uint32_t max_iterations) {
   if (c.colonies > 0) return solve_batch(c, dt, growth, max_iterations);
@@ -1348,6 +1423,7 @@ SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, flo
     }
   }
   const bool fused = use_fused_relaxation(c, std::max(rows, c.n));
+  int tiled = 0;
   if (fused) {
     // One cooperative launch runs the whole solve (relax_kernel).
     const std::uint32_t wanted = (std::max(rows, c.n) + kSolveThreads - 1) / kSolveThreads;
@@ -1358,18 +1434,30 @@ SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, flo
   } else {
     auto& graph = graph_for(c, std::max(rows, c.n));
     c.last_blocks = graph.blocks();
+    if (c.relaxation == 0 && c.spatial_valid) tiled = build_tiles(c, c.host_desc->tiles);
     fill_desc(c, rows, dt, growth, tolerance, max_iterations);
-    check(cudaError_t(graph.launch(c.stream)), "solve launch");
+    auto& made = c.tile_graphs[tiled];
+    if (tiled > 0 && !made) {
+      auto fresh = std::make_unique<SolveGraph>();
+      check(cudaError_t(fresh->create(c.desc, kMaxPassBlocks, c.stream, tiled)), "solve graph");
+      made = std::move(fresh);
+    }
+    check(cudaError_t((tiled > 0 ? *made : graph).launch(c.stream)), "solve launch");
   }
   // The final multipliers and gaps, and their response (the passes of a
   // solve write only the rows' side terms).
-  launch_unpack_iterate(c.desc, c.last_blocks, c.stream);
+  c.last_tiled = tiled;
+  if (tiled > 0) {
+    launch_unpack_tiles(c.desc, c.last_blocks, c.stream);
+  } else {
+    launch_unpack_iterate(c.desc, c.last_blocks, c.stream);
+  }
   launch_evaluate(c.desc, c.last_blocks, false, c.stream);
   check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
   sync(c);
   const SolveDesc& d = *c.host_desc;
   if (d.barrier_abort != 0) throw DeviceCheckError("a grid barrier of the relaxation ran out of time");
-  if (d.check_status != 0) throw DeviceCheckError("an index check of the relaxation failed");
+  if (d.check_status != 0) throw DeviceCheckError("an index check or a bounded wait of the relaxation failed");
   if (!fused) count_launch(SolveGraph::loop_launches(d.iterations));
   c.solve_log.push_back({rows, d.iterations, d.status, d.residual});
   if (d.status == 3) throw std::invalid_argument("contact system has no positive diagonal");
@@ -1840,13 +1928,15 @@ Attempt advance_substep(Ctx& c, float dt, const msb_contact_dynamics_parameters&
   const std::uint32_t found = find_touches(c, c.state, cp, wp, p.candidate_margin, c.touches,
                                            p.candidate_margin + (c.colonies > 0 ? kBatchRecheckReach : kRecheckReach), true);
   mark(c, kPhaseRows);
-  // Systems that take the resident solve's grid form get their cells'
-  // spatial order, from the grid of the search just made.
+  // Systems that take the resident solve's grid form, and those too large
+  // for it, get their cells' spatial order from the grid of the search just
+  // made.
   c.spatial_valid = false;
   if (c.relaxation == 0 && found > 0 && n > 1) {
     if (!c.resident_limits) c.resident_limits = resident_limits();
     if (c.colonies > 0 ? c.resident_limits->grid > 0 && c.colonies <= kResidentColonies
-                       : resident_plan(*c.resident_limits, found, n).grid) {
+                       : resident_plan(*c.resident_limits, found, n).grid ||
+                             resident_plan(*c.resident_limits, found, n).ctas == 0) {
       c.spatial_keys.ensure(n);
       c.spatial_order.ensure(n);
       c.temp.ensure(sort_temp_words(n) + 64);
@@ -2303,6 +2393,7 @@ void msb_context_destroy(msb_context* context) {
   for (auto e : context->phase_events) cudaEventDestroy(e);
   for (auto e : context->download_events) cudaEventDestroy(e);
   context->graphs.clear();
+  for (auto& graph : context->tile_graphs) graph.reset();
   if (context->desc != nullptr) cudaFree(context->desc);
   if (context->host_scalars != nullptr) cudaFreeHost(context->host_scalars);
   if (context->host_desc != nullptr) cudaFreeHost(context->host_desc);
@@ -2828,11 +2919,18 @@ int msb_profile_iterations(msb_context* context, uint32_t iterations, float* bod
     check(cudaEventCreate(&between), "event");
     check(cudaEventCreate(&stop), "event");
     // Warm the caches as the solve loop does.
-    launch_iteration(c.desc, c.last_blocks, nullptr, c.stream);
+    const auto iterate = [&](cudaEvent_t middle) {
+      if (c.last_tiled > 0) {
+        launch_tile_iteration(c.desc, c.last_tiled, middle, c.stream);
+      } else {
+        launch_iteration(c.desc, c.last_blocks, middle, c.stream);
+      }
+    };
+    iterate(nullptr);
     double body = 0.0, row = 0.0;
     for (std::uint32_t k = 0; k < iterations; ++k) {
       check(cudaEventRecord(start, c.stream), "event");
-      launch_iteration(c.desc, c.last_blocks, between, c.stream);
+      iterate(between);
       check(cudaEventRecord(stop, c.stream), "event");
       check(cudaEventSynchronize(stop), "event");
       float a = 0.0f, b = 0.0f;

@@ -625,7 +625,8 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
           const float2 constants = d.incidence.constants[row];
           l.a(j) = d.incidence.a[begin + k];
           l.b(j) = eb;
-          l.c(j) = make_float4(constants.x, (side & 1u) ? constants.y : -constants.y, d.multipliers[row], 0.0f);
+          const float compliance = fabsf(constants.y);  // -0 included
+          l.c(j) = make_float4(constants.x, (side & 1u) ? compliance : -compliance, d.multipliers[row], 0.0f);
           l.own(j) = 0.0f;
           l.inbox(j) = 0.0f;
           r.slot_of[begin + k] = comm.rank << 16 | j;

@@ -27,6 +27,7 @@
 #include "device.cuh"
 #include "kernels.h"
 #include "solve.h"
+#include "solve_decide.cuh"
 #include "solve_math.cuh"
 #include "../../include/msb200.h"
 
@@ -245,9 +246,7 @@ __device__ __forceinline__ void row_pass(const SolveDesc& d, std::uint32_t mode,
   float2* __restrict__ iterate = d.iterate;
   const float2* __restrict__ sides = d.incidence.sides;
   const float2* __restrict__ constants = d.incidence.constants;
-  double ss = 0.0, sy = 0.0, yy = 0.0;
-  float residual = 0.0f;
-  bool finite = true;
+  PassSums sums;
   (void)check;
   // row_gap (cpp/cpu/cpu_contact_dynamics.cpp:149-159): offset + dt * (first
   // side's term + second side's term) + compliance * multiplier.  The body
@@ -264,15 +263,7 @@ __device__ __forceinline__ void row_pass(const SolveDesc& d, std::uint32_t mode,
     const float m = project ? smax(0.0f, gi - alpha * gpi) : gi;
     const float rate = side.x + side.y;
     const float gn = k.x + dt * rate + k.y * m;
-    residual = smax(residual, row_residual(m, gn));
-    finite = finite && isfinite(gn);
-    if (project) {
-      const double moved = double(m) - double(gi);
-      const double change = double(gn) - double(gpi);
-      ss += moved * moved;
-      sy += moved * change;
-      yy += change * change;
-    }
+    sums.add(project, make_float2(gi, gpi), m, gn);
     if (mode == 2) {
       gap[i] = gn;
     } else {
@@ -281,104 +272,7 @@ __device__ __forceinline__ void row_pass(const SolveDesc& d, std::uint32_t mode,
   }
   if (mode == 2) return;
 
-  // Block reduction in a fixed tree.
-  __shared__ double red[5][kSolveThreads / 32];
-  double v[5] = {ss, sy, yy, double(residual), finite ? 1.0 : 0.0};
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    for (int o = 16; o > 0; o >>= 1) {
-      const double other = __shfl_down_sync(0xFFFFFFFFu, v[k], o);
-      v[k] = k < 3 ? v[k] + other : (k == 3 ? fmax(v[k], other) : fmin(v[k], other));
-    }
-    if (lane == 0) red[k][warp] = v[k];
-  }
-  __syncthreads();
-  if (threadIdx.x < 5) {
-    const int k = threadIdx.x;
-    double r = red[k][0];
-    for (int w = 1; w < kSolveThreads / 32; ++w) {
-      r = k < 3 ? r + red[k][w] : (k == 3 ? fmax(r, red[k][w]) : fmin(r, red[k][w]));
-    }
-    d.partials[5 * block + k] = r;
-  }
-  __syncthreads();
-}
-
-// One block combines the partials of `blocks` blocks in block order (so the
-// result does not depend on scheduling), sets the next step length, the
-// status and whether to go on (d.proceed), as one iteration of
-// iterate_contact_steps does (cpp/core/contact_solver.hpp:66-82); mode 0
-// judges the initial multipliers.  Returns d.proceed (thread 0).
-__device__ __forceinline__ std::uint32_t decide(SolveDesc& d, std::uint32_t mode, std::uint32_t blocks) {
-  __shared__ double red[5][kSolveThreads / 32];
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  double t[5] = {0.0, 0.0, 0.0, 0.0, 1.0};
-  for (std::uint32_t p = threadIdx.x; p < blocks; p += blockDim.x) {
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const double x = __ldcg(&d.partials[5 * p + k]);
-      t[k] = k < 3 ? t[k] + x : (k == 3 ? fmax(t[k], x) : fmin(t[k], x));
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    for (int o = 16; o > 0; o >>= 1) {
-      const double other = __shfl_down_sync(0xFFFFFFFFu, t[k], o);
-      t[k] = k < 3 ? t[k] + other : (k == 3 ? fmax(t[k], other) : fmin(t[k], other));
-    }
-  }
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < 5; ++k) red[k][warp] = t[k];
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return 0;
-  double total[5];
-  for (int k = 0; k < 5; ++k) {
-    total[k] = red[k][0];
-    for (int w = 1; w < kSolveThreads / 32; ++w) {
-      total[k] = k < 3 ? total[k] + red[k][w] : (k == 3 ? fmax(total[k], red[k][w]) : fmin(total[k], red[k][w]));
-    }
-  }
-  d.ticket = 0;
-  const float reported = total[4] > 0.5 ? float(total[3]) : __int_as_float(0x7FC00000);
-  d.residual = reported;
-  std::uint32_t proceed = 0;
-  if (mode == 0) {
-    const float bound = __uint_as_float(__ldcg(&d.bound_bits));
-    d.bound = bound;
-    d.iterations = 0;
-    if (!isfinite(bound) || !(bound > 0.0f)) {
-      d.status = 3;  // no positive diagonal: an invalid system
-    } else if (!isfinite(reported)) {
-      d.status = MSB_SOLVE_BREAKDOWN;
-    } else if (reported <= d.tolerance) {
-      d.status = MSB_SOLVE_CONVERGED;
-    } else {
-      d.status = MSB_SOLVE_ITERATION_LIMIT;
-      d.step = 1.0f / bound;
-      proceed = d.max_iterations > 0 ? 1u : 0u;
-    }
-    d.mode = 1;
-  } else {
-    const std::uint32_t iteration = d.iterations + 1;
-    d.iterations = iteration;
-    if (!isfinite(reported)) {
-      d.status = MSB_SOLVE_BREAKDOWN;
-    } else if (!(reported > d.tolerance)) {
-      d.status = MSB_SOLVE_CONVERGED;
-    } else {
-      d.step = next_step(d.step, total[0], total[1], total[2], iteration);
-      d.status = MSB_SOLVE_ITERATION_LIMIT;
-      proceed = iteration < d.max_iterations ? 1u : 0u;
-    }
-  }
-  d.proceed = proceed;
-  return proceed;
+  sums.reduce_to(d.partials + 5 * block);
 }
 
 // mode 0: gaps of the initial multipliers and the first residual (sets the
@@ -749,7 +643,7 @@ SolveGraph::~SolveGraph() {
   if (graph_ != nullptr) cudaGraphDestroy(graph_);
 }
 
-int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream) {
+int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream, int tiles_per_sm) {
   // At most one resident wave: a grid-stride pass whose blocks do not all
   // fit at once leaves a partly empty second wave.
   int device = 0, sms = kSmCount, body_active = 1, row_active = 1;
@@ -763,6 +657,13 @@ int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream) {
   const int row_blocks = row_pass_blocks();
   blocks = std::max(1, std::min(blocks, wave));
   blocks_ = blocks;
+  // The tiled solve's passes take the body and row passes' places.
+  const bool tiled = tiles_per_sm > 0;
+  void* const first_pass = tiled ? tile_pass_function(tiles_per_sm) : reinterpret_cast<void*>(body_pass_kernel<0>);
+  void* const second_pass = tiled ? boundary_pass_function() : reinterpret_cast<void*>(row_pass_kernel<0>);
+  const std::uint32_t first_bytes = tiled ? tile_pass_bytes(tiles_per_sm) : 0u;
+  int first_blocks = tiled ? tile_pass_blocks(tiles_per_sm) : blocks;
+  const int second_blocks = tiled ? boundary_pass_blocks() : row_blocks;
   desc_ = desc;
   cudaError_t err = cudaGraphCreate(&graph_, 0);
   if (err != cudaSuccess) return err;
@@ -772,12 +673,12 @@ int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream) {
   handle_ = handle;
 
   auto kernel_node = [&](cudaGraph_t graph, cudaGraphNode_t* node, const cudaGraphNode_t* deps, size_t ndeps,
-                         void* func, void** args, int grid, int threads = kSolveThreads) {
+                         void* func, void** args, int grid, int threads = kSolveThreads, std::uint32_t bytes = 0) {
     cudaKernelNodeParams p{};
     p.func = func;
     p.gridDim = dim3(grid);
     p.blockDim = dim3(threads);
-    p.sharedMemBytes = 0;
+    p.sharedMemBytes = bytes;
     p.kernelParams = args;
     p.extra = nullptr;
     return cudaGraphAddKernelNode(node, graph, deps, ndeps, &p);
@@ -789,12 +690,12 @@ int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream) {
   void* reset_args[] = {&d};
   void* bound_args[] = {&d};
   void* body_args[] = {&d, &mode_auto};
-  void* row_args[] = {&d, &mode_auto, &with_condition};
+  void* row_args[] = {&d, &mode_auto, &with_condition, &first_blocks};  // the last: tiled only
   cudaGraphNode_t reset, bound, body0, row0, loop;
   if ((err = kernel_node(graph_, &reset, nullptr, 0, (void*)solve_reset_kernel, reset_args, 1, 32)) != cudaSuccess) return err;
   if ((err = kernel_node(graph_, &bound, &reset, 1, (void*)bound_kernel, bound_args, blocks)) != cudaSuccess) return err;
-  if ((err = kernel_node(graph_, &body0, &bound, 1, (void*)body_pass_kernel<0>, body_args, blocks)) != cudaSuccess) return err;
-  if ((err = kernel_node(graph_, &row0, &body0, 1, (void*)row_pass_kernel<0>, row_args, row_blocks)) != cudaSuccess) return err;
+  if ((err = kernel_node(graph_, &body0, &bound, 1, first_pass, body_args, first_blocks, kSolveThreads, first_bytes)) != cudaSuccess) return err;
+  if ((err = kernel_node(graph_, &row0, &body0, 1, second_pass, row_args, second_blocks)) != cudaSuccess) return err;
 
   cudaGraphNodeParams cp{};
   cp.type = cudaGraphNodeTypeConditional;
@@ -807,10 +708,10 @@ int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream) {
   for (int pair = 0; pair < MSB_WHILE_UNROLL; ++pair) {
     cudaGraphNode_t body1, row1;
     if ((err = kernel_node(body, &body1, previous != nullptr ? &previous : nullptr, previous != nullptr ? 1 : 0,
-                           (void*)body_pass_kernel<0>, body_args, blocks)) != cudaSuccess) {
+                           first_pass, body_args, first_blocks, kSolveThreads, first_bytes)) != cudaSuccess) {
       return err;
     }
-    if ((err = kernel_node(body, &row1, &body1, 1, (void*)row_pass_kernel<0>, row_args, row_blocks)) != cudaSuccess) return err;
+    if ((err = kernel_node(body, &row1, &body1, 1, second_pass, row_args, second_blocks)) != cudaSuccess) return err;
     previous = row1;
   }
   err = cudaGraphInstantiate(&exec_, graph_, 0);

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "kernels.h"
+#include "tiles.h"
 
 namespace msb {
 
@@ -94,6 +95,7 @@ struct SolveDesc {
   float tolerance;
   std::uint32_t max_iterations;
   std::uint32_t has_drift;  // 0: every drift is zero and the drift arrays are not read
+  TileArrays tiles;         // of a tiled solve
   // solver state
   float step;
   float residual;
@@ -134,8 +136,9 @@ class SolveGraph {
   SolveGraph(const SolveGraph&) = delete;
   SolveGraph& operator=(const SolveGraph&) = delete;
   ~SolveGraph();
-  // Returns a CUDA error code.
-  int create(SolveDesc* desc, int blocks, cudaStream_t stream);
+  // `tiles_per_sm` > 0: the passes of tiles.cu, which read desc->tiles, with
+  // that many blocks an SM.  Returns a CUDA error code.
+  int create(SolveDesc* desc, int blocks, cudaStream_t stream, int tiles_per_sm = 0);
   int launch(cudaStream_t stream);
   int blocks() const { return blocks_; }
   // Kernel launches of the WHILE node for a solve of `iterations`

@@ -1,0 +1,64 @@
+"""The tiled solve of systems too large to be resident, against the solve
+graph on the same steps: the same substeps, geometry within four solve
+tolerances (two solves of one system may differ by that)."""
+
+import numpy as np
+import pytest
+
+from microsimulator_b200 import workloads
+from microsimulator_b200.backend import B200Backend
+from microsimulator_b200.types import ContactDynamicsParameters, GrowthLoadResponse
+from microsimulator_b200.world import WorldState
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def forms(backend):
+    yield backend
+    backend.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+
+
+def step_both(backend, world, constraints=None, dt=0.002, **parameters):
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4, **parameters)
+    results = []
+    for form in (B200Backend.RELAXATION_AUTOMATIC, B200Backend.RELAXATION_GRAPH):
+        backend.set_relaxation(form)
+        stepped = world.copy()
+        result = backend.advance_contact_dynamics(stepped, constraints, dt, p)
+        results.append((stepped, result.report))
+    (a, ra), (b, rb) = results
+    assert ra.substeps == rb.substeps and ra.halvings == rb.halvings
+    assert np.max(np.abs(a.geometry() - b.geometry())) <= 4 * p.overlap_tolerance
+    return ra
+
+
+# A last tile of one body, of all its bodies, of all but one.
+@pytest.mark.parametrize("cells", [768 * 256 + 1, 640 * 256, 641 * 256 - 1])
+@pytest.mark.parametrize("law", [0, 2])
+def test_steps_by_tiles(forms, cells, law):
+    world = workloads.jammed(cells, seed=cells)
+    step_both(forms, world, growth=GrowthLoadResponse(law, 0.0, 0.2, 3.0))
+    assert forms.profile_iterations(2)["bodies"] == cells
+
+
+def test_walls_by_tiles(forms):
+    world, walls = workloads.trap_colony(180_000, seed=3)
+    world.position_y *= np.float32(1.15)  # into the side walls
+    step_both(forms, world, walls)
+
+
+@pytest.mark.parametrize("cells", [20_000, 180_000])
+def test_a_body_of_many_rows(forms, cells):
+    """A long capsule over a colony touches more than 62 cells: neither the
+    resident nor the tiled solve holds it, and the graph does."""
+    world = workloads.jammed(cells, seed=4)
+    middle = float(world.position_x.mean())
+    fields = {name: getattr(world, name) for name in WorldState.FIELDS}
+    long = WorldState.from_arrays(
+        np.stack([np.append(fields["position_x"], middle), np.append(fields["position_y"], middle),
+                  np.append(fields["position_z"], 0.995)], axis=1),
+        np.stack([np.append(fields["direction_x"], 1.0), np.append(fields["direction_y"], 0.0),
+                  np.append(fields["direction_z"], 0.0)], axis=1),
+        np.append(fields["lengths"], 120.0), 0.5, growth_rates=0.5)
+    step_both(forms, long)
