@@ -1398,8 +1398,8 @@ int build_tiles(Ctx& c, TileArrays& out) {
 
 // Systems too large to be resident take the tiled passes where the substep
 // has a spatial order (per iteration against the two passes by slot: 1M
-// capsules in tracks, 4.15M rows, 113 against 187 us; 1M at random, 2.65M
-// rows, 94 against 103; 300k at random, 782,000 rows, 31 against 37).
+// capsules in tracks, 4.15M rows, 97 against 187 us; 1M at random, 2.65M
+// rows, 80 against 104; 300k at random, 782,000 rows, 31 against 37).
 SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, float tolerance,
                    std::uint32_t max_iterations) {
   if (c.colonies > 0) return solve_batch(c, dt, growth, max_iterations);

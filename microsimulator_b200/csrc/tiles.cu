@@ -19,11 +19,12 @@
 // (Entries loaded into registers by each thread, 8 or 4 at a time, were
 // bound by latency: 250 and 197 us a pass at 4.15 M rows.)
 //
-// At 4.15 M rows over 1 M bodies the tile pass takes 100 us and the boundary
-// pass 16 (145 and 40 in the two passes by slot), 153 of 155 MB at 1.66 M
-// rows being what it cannot do without; two blocks an SM, its chain of copy,
-// sums, side terms and rows keeps DRAM at 41 %.  Two lanes a body (512
-// threads) measured 118 us: more instructions, no more overlap.
+// At 4.15 M rows over 1 M bodies the tile pass takes 85 us and the boundary
+// pass 16 (145 and 40 in the two passes by slot); 153 of the 155 MB it moves
+// at 1.66 M rows are what it cannot do without.  Two blocks an SM, the chain
+// of each tile's copy, sums, side terms and rows bounds it, not DRAM.  Two
+// lanes a body (512 threads) measured 118 us where one measured 111: more
+// instructions, no more overlap; tiles of 128 to 248 bodies 0 to 15 % slower.
 //
 // The arithmetic is the two passes', term by term; a body's entries are in
 // row order.  Only the FP64 sums are taken in another fixed order.
@@ -129,19 +130,25 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
   float* const multiplier = reinterpret_cast<float*>(side + t.max_locals);
   const auto shared_at = [](const void* p) { return static_cast<std::uint32_t>(__cvta_generic_to_shared(p)); };
   const std::uint32_t barrier = shared_at(tile_memory);
-  Tile now{}, next{};
-  std::uint32_t guest_row[kGuests];
-  float2 guest[kGuests];
-  const auto guest_rows = [&](const Tile& tile) {
+  // Each load is issued a phase or a tile before its value is needed: what
+  // the tile after the next consists of, the next tile's guests, then their
+  // iterates.  (With the next tile's alone looked up, its guests' chain of
+  // three loads was 4,500 of a tile's 9,600 cycles.)
+  Tile now{}, next{}, after{};
+  std::uint32_t guest_row[kGuests] = {}, next_row[kGuests] = {};
+  float2 guest[kGuests] = {};
+  const auto guest_rows = [&](const Tile& tile, std::uint32_t (&row)[kGuests]) {
 #pragma unroll
     for (int i = 0; i < kGuests; ++i) {
       const std::uint32_t g = threadIdx.x + i * kThreads;
-      guest_row[i] = t.guests[tile.g0 + (g < tile.guests ? g : 0u)];
+      if (g < tile.guests) row[i] = t.guests[tile.g0 + g];
     }
   };
-  const auto guest_values = [&] {
+  const auto guest_values = [&](const Tile& tile, const std::uint32_t (&row)[kGuests]) {
 #pragma unroll
-    for (int i = 0; i < kGuests; ++i) guest[i] = t.iterate[guest_row[i]];
+    for (int i = 0; i < kGuests; ++i) {
+      if (threadIdx.x + i * kThreads < tile.guests) guest[i] = t.iterate[row[i]];
+    }
   };
   std::uint32_t tile = blockIdx.x;
   if (threadIdx.x == 0) {
@@ -155,17 +162,16 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
       fetch_entries(now, t.a, t.b, shared_at(a), shared_at(b), barrier);
       fetch_rows(now, t.iterate, t.constants, shared_at(iterate), shared_at(constants), barrier);
     }
-    if (now.guests > 0u) {
-      guest_rows(now);
-      guest_values();
-    }
+    guest_rows(now, guest_row);
+    guest_values(now, guest_row);
+    if (tile + gridDim.x < t.tiles) next.load(t, tile + gridDim.x, bodies);
   }
   std::uint32_t phase = 0;
   PassSums sums;
   for (; tile < t.tiles; tile += gridDim.x) {
-    const std::uint32_t following = tile + gridDim.x;
-    const bool more = following < t.tiles;
-    if (more) next.load(t, following, bodies);
+    const bool more = tile + gridDim.x < t.tiles;
+    if (more) guest_rows(next, next_row);
+    if (tile + 2 * gridDim.x < t.tiles) after.load(t, tile + 2 * gridDim.x, bodies);
     const std::uint32_t skip = now.skip();
     const std::uint32_t place = tile * kTileBodies + threadIdx.x;
     const bool live = place < bodies;
@@ -237,10 +243,7 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
     }
     if (more) {
       if (threadIdx.x == 0) fetch_entries(next, t.a, t.b, shared_at(a), shared_at(b), barrier);
-      if (next.guests > 0u) {
-        guest_rows(next);
-        guest_values();
-      }
+      guest_values(next, next_row);
     }
 #pragma unroll 2
     for (std::uint32_t j = threadIdx.x; j < now.rows; j += kThreads) {
@@ -259,6 +262,9 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
       fetch_rows(next, t.iterate, t.constants, shared_at(iterate), shared_at(constants), barrier);
     }
     now = next;
+    next = after;
+#pragma unroll
+    for (int i = 0; i < kGuests; ++i) guest_row[i] = next_row[i];
   }
   sums.reduce_to(d.partials + 5 * blockIdx.x);
 }
