@@ -215,7 +215,7 @@ class B200Backend:
                 continue
             self._check(status)
             self._capacity = max(self._capacity, int(count.value))
-            return out[: count.value].copy()
+            return out[: count.value]
 
     # -- ComputeBackend -------------------------------------------------
     def find_cell_contacts(self, world, parameters: ContactParameters | None = None) -> np.ndarray:
@@ -253,7 +253,7 @@ class B200Backend:
                 continue
             self._check(status)
             self._capacity = max(self._capacity, int(count.value))
-            return self._graph(n, contacts[: count.value].copy(), index, arrays)
+            return self._graph(n, contacts[: count.value], index, arrays)
 
     def build_contact_graph(self, contacts: np.ndarray, cell_count: int) -> ContactGraph:
         """ContactGraph(cell_count, contacts) (contact_graph.cpp:302-349) on
@@ -289,7 +289,7 @@ class B200Backend:
                 continue
             self._check(status)
             total = int(count.value)
-            return ExternalContactGraph(n, contacts[:total].copy(), offsets, indices[:total].copy())
+            return ExternalContactGraph(n, contacts[:total], offsets, indices[:total])
 
     def build_contact_graph_device(self, contacts_pointer: int, count: int, cell_count: int, index) -> int:
         """msb_build_contact_graph on device-resident contact records and

@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <optional>
@@ -779,6 +780,62 @@ void flush_downloads(Ctx& c) {
   const cudaError_t err = host_copies(c).run(c.pending);
   c.pending.clear();
   check(err, "copy back");
+}
+
+// Results for the caller's host arrays.  Large ones come through two halves
+// of pinned staging in pieces, one half's host copies running on the pool
+// while the other half is on its way (a pageable copy is one thread's, and
+// faults the caller's new pages in one by one).  The staging stays small:
+// pinning as much as the results is 10 ms of a context's first call at 40 MB.
+struct HostResult {
+  void* dst;
+  const void* device_src;
+  std::size_t bytes;
+};
+void download_results(Ctx& c, std::initializer_list<HostResult> results) {
+  constexpr std::size_t kPiece = std::size_t(1) << 19, kPieces = 12, kHalf = kPieces * kPiece;
+  constexpr std::size_t kDirect = std::size_t(1) << 18;  // up to this, plain copies cost less than waking the pool
+  std::vector<HostResult> pieces;
+  std::size_t total = 0;
+  for (const auto& r : results) total += r.bytes;
+  for (const auto& r : results) {
+    if (r.bytes == 0) continue;
+    if (total <= kDirect || pinned_host(r.dst)) {
+      check(cudaMemcpyAsync(r.dst, r.device_src, r.bytes, cudaMemcpyDeviceToHost, c.stream), "copy back");
+      continue;
+    }
+    for (std::size_t from = 0; from < r.bytes; from += kPiece) {
+      pieces.push_back({static_cast<char*>(r.dst) + from, static_cast<const char*>(r.device_src) + from,
+                        std::min(kPiece, r.bytes - from)});
+    }
+  }
+  if (!pieces.empty()) {
+    unsigned char* const staging = c.download.ensure(2 * kHalf);
+    while (c.download_events.size() < 2 * kPieces) {
+      cudaEvent_t e;
+      check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+      c.download_events.push_back(e);
+    }
+    std::vector<msb::HostCopies::Job> jobs[2];
+    std::size_t next = 0;
+    const auto queue = [&](std::size_t half) {
+      for (std::size_t k = 0; k < kPieces && next < pieces.size(); ++k, ++next) {
+        const HostResult& piece = pieces[next];
+        unsigned char* const slot = staging + half * kHalf + k * kPiece;
+        const cudaEvent_t there = c.download_events[half * kPieces + k];
+        check(cudaMemcpyAsync(slot, piece.device_src, piece.bytes, cudaMemcpyDeviceToHost, c.stream), "copy back");
+        check(cudaEventRecord(there, c.stream), "event");
+        jobs[half].push_back({piece.dst, slot, piece.bytes, there});
+      }
+    };
+    queue(0);
+    for (std::size_t half = 0; !jobs[half].empty(); half ^= 1) {
+      queue(half ^ 1);
+      check(host_copies(c).run(jobs[half]), "copy back");
+      jobs[half].clear();
+    }
+  }
+  sync(c);
 }
 
 void load_cells(Ctx& c, const msb_cell_arrays& cells, bool device_pointers) {
@@ -2309,21 +2366,16 @@ GraphArrays graph_staging(Ctx& c, std::uint64_t cell_count, std::uint64_t entrie
   return g;
 }
 
-void copy_out(Ctx& c, void* host, const void* device, std::uint64_t bytes) {
-  if (bytes == 0) return;
-  check(cudaMemcpyAsync(host, device, bytes, cudaMemcpyDeviceToHost, c.stream), "copy index");
-}
-
-// Copies a staged index to the caller's host arrays (`index` names them).
+// Copies a staged index to the caller's host arrays (`index` names them),
+// with `contacts` beside it.
 void copy_graph_out(Ctx& c, const GraphArrays& g, std::uint64_t cell_count, std::uint64_t entries,
-                    std::uint64_t neighbors, msb_contact_graph_index& index) {
-  copy_out(c, index.incidence_offsets, g.incidence_offsets, (cell_count + 1) * 8);
-  copy_out(c, index.incidence_contacts, g.incidence, entries * 8);
-  if (g.neighbor_offsets != nullptr) {
-    copy_out(c, index.neighbor_offsets, g.neighbor_offsets, (cell_count + 1) * 8);
-    copy_out(c, index.neighbor_ids, g.neighbors, neighbors * 8);
-  }
-  sync(c);
+                    std::uint64_t neighbors, msb_contact_graph_index& index, HostResult contacts = {}) {
+  const bool listed = g.neighbor_offsets != nullptr;
+  download_results(c, {contacts,
+                       {index.incidence_offsets, g.incidence_offsets, (cell_count + 1) * 8},
+                       {index.incidence_contacts, g.incidence, entries * 8},
+                       {index.neighbor_offsets, g.neighbor_offsets, listed ? (cell_count + 1) * 8 : 0},
+                       {index.neighbor_ids, g.neighbors, listed ? neighbors * 8 : 0}});
 }
 
 // The checks on a caller's index record shared by the graph calls.
@@ -2641,9 +2693,7 @@ int msb_find_cell_contacts(msb_context* context, const msb_cell_arrays* cells,
     if (contacts == nullptr) throw std::invalid_argument("null contact array");
     c.records.ensure(total * sizeof(msb_cell_contact));
     launch_touches_to_cell_contacts(c.touches.p, total, c.ids.p, c.records.p, c.stream);
-    check(cudaMemcpyAsync(contacts, c.records.p, total * sizeof(msb_cell_contact), cudaMemcpyDeviceToHost, c.stream),
-          "copy contacts");
-    sync(c);
+    download_results(c, {{contacts, c.records.p, total * sizeof(msb_cell_contact)}});
   });
 }
 
@@ -2671,14 +2721,11 @@ int msb_find_cell_contact_graph(msb_context* context, const msb_cell_arrays* cel
         index->neighbor_count = packed;
         if (packed > index->neighbor_capacity) throw CapacityError("neighbour id array is too small");
       }
-      copy_graph_out(c, g, cells->count, 2ull * total, packed, *index);
+      copy_graph_out(c, g, cells->count, 2ull * total, packed, *index,
+                     {contacts, c.records.p, total * sizeof(msb_cell_contact)});
+    } else {
+      download_results(c, {{contacts, c.records.p, total * sizeof(msb_cell_contact)}});
     }
-    if (total > 0) {
-      check(cudaMemcpyAsync(contacts, c.records.p, total * sizeof(msb_cell_contact), cudaMemcpyDeviceToHost,
-                            c.stream),
-            "copy contacts");
-    }
-    sync(c);
   });
 }
 
@@ -2704,18 +2751,15 @@ int msb_find_external_contact_graph(msb_context* context, const msb_cell_arrays*
     }
     c.records.ensure(std::max<std::uint64_t>(total, 1) * sizeof(msb_external_contact));
     if (total > 0) launch_touches_to_external_contacts(c.touches.p, total, c.ids.p, c.records.p, c.stream);
-    if (incidence_offsets != nullptr) {
-      const GraphArrays g = graph_staging(c, cells->count, total, false);
+    GraphArrays g{};
+    const bool indexed = incidence_offsets != nullptr;
+    if (indexed) {
+      g = graph_staging(c, cells->count, total, false);
       build_graph(c, c.records.p, total, cells->count, true, g);
-      copy_out(c, incidence_offsets, g.incidence_offsets, (cells->count + 1) * 8);
-      copy_out(c, incidence_contacts, g.incidence, std::uint64_t(total) * 8);
     }
-    if (total > 0) {
-      check(cudaMemcpyAsync(contacts, c.records.p, total * sizeof(msb_external_contact), cudaMemcpyDeviceToHost,
-                            c.stream),
-            "copy contacts");
-    }
-    sync(c);
+    download_results(c, {{contacts, c.records.p, total * sizeof(msb_external_contact)},
+                         {incidence_offsets, g.incidence_offsets, indexed ? (cells->count + 1) * 8 : 0},
+                         {incidence_contacts, g.incidence, indexed ? std::uint64_t(total) * 8 : 0}});
   });
 }
 
@@ -2781,10 +2825,11 @@ int msb_build_external_contact_graph(msb_context* context, const msb_external_co
     }
     build_graph(c, source, count, cell_count, true, g);
     if (device_pointers == 0) {
-      copy_out(c, incidence_offsets, g.incidence_offsets, (cell_count + 1) * 8);
-      copy_out(c, incidence_contacts, g.incidence, count * 8);
+      download_results(c, {{incidence_offsets, g.incidence_offsets, (cell_count + 1) * 8},
+                           {incidence_contacts, g.incidence, count * 8}});
+    } else {
+      sync(c);
     }
-    sync(c);
   });
 }
 
@@ -2807,10 +2852,7 @@ int msb_find_external_contacts(msb_context* context, const msb_cell_arrays* cell
     if (contacts == nullptr) throw std::invalid_argument("null contact array");
     c.records.ensure(total * sizeof(msb_external_contact));
     launch_touches_to_external_contacts(c.touches.p, total, c.ids.p, c.records.p, c.stream);
-    check(cudaMemcpyAsync(contacts, c.records.p, total * sizeof(msb_external_contact), cudaMemcpyDeviceToHost,
-                          c.stream),
-          "copy contacts");
-    sync(c);
+    download_results(c, {{contacts, c.records.p, total * sizeof(msb_external_contact)}});
   });
 }
 
