@@ -278,11 +278,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) forward_tc_kernel(const std::ui
 //
 // C (m x n) = A (m x k) B (k x n), bf16 operands through element strides.
 // A CTA computes a 128-row tile of C (rows past m zero) over its share of k
-// (grid z splits k): per 64-wide k chunk its 128 threads stage the A chunk
+// (grid z splits k): per 64-wide k chunk its threads stage the A chunk
 // (128 x 64) and the B chunk (n rounded up to 16, x 64) in the canonical
 // K-major layout, thread 0 issues four tcgen05.mma (K = 16 each) into the
 // TMEM accumulator and commits them to an mbarrier, and the chunk after
-// waits for them; the next chunk's loads are in flight meanwhile.  The four
+// waits for them; the next chunk's loads are in flight meanwhile.  The eight
 // warps then read their 32 lanes of the accumulator with tcgen05.ld and
 // store C (or the split's partial sums), or the layer's dZ.
 //
@@ -292,10 +292,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) forward_tc_kernel(const std::ui
 // weight gradients) a GEMM of a training step of 8,192 rows took 70 us, and
 // a bias sum, one block adding 8,192 rows in order, 317 us; the step went
 // from 1,166 to 223 us with the vector loads, the GELU derivative and the
-// column sums in the epilogue.  At 8,192 rows it is bound by its fourteen
-// dependent launches of 5-12 us.
+// column sums in the epilogue, and to 198 with eight warps a CTA (four
+// before).  At 8,192 rows it is bound by the latency of its chain of short
+// launches (64 tiles of C on 148 SMs).
 
-constexpr int kGemmThreads = 128;
+constexpr int kGemmThreads = 256;  // half of them stage A, half B; in the epilogue two warps share a row's columns
 constexpr std::uint32_t kGemmChunk = 64;
 constexpr std::uint32_t kGemmBytesA = 128 * kGemmChunk * 2;  // 16 KB
 constexpr std::uint32_t kGemmBytesB = 128 * kGemmChunk * 2;  // 16 KB (n <= 128)
@@ -331,13 +332,13 @@ struct Operand {
   int staging;
 
   __device__ __forceinline__ bool place(std::uint32_t& row_group, std::uint32_t& k_group) const {
-    const std::uint32_t groups = tile_rows / 8;
+    const std::uint32_t groups = tile_rows / 8, thread = threadIdx.x % 128;
     if (staging == kAlongK) {
-      k_group = threadIdx.x % 8;
-      row_group = threadIdx.x / 8;
+      k_group = thread % 8;
+      row_group = thread / 8;
     } else {
-      row_group = threadIdx.x % groups;
-      k_group = threadIdx.x / groups;
+      row_group = thread % groups;
+      k_group = thread / groups;
     }
     return row_group < groups && k_group < 8;
   }
@@ -426,11 +427,12 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, int stagi
   const std::uint32_t m0 = blockIdx.y * 128;
   const std::uint32_t k_begin = blockIdx.z * chunk_split * kGemmChunk;
   const std::uint32_t k_end = smin<std::uint32_t>(p.k, k_begin + chunk_split * kGemmChunk);
-  const Operand a{p.a, p.m, m0, 128u, p.sam, p.sak, staging_a};
-  const Operand b{p.b, p.n, 0u, nt, p.sbn, p.sbk, staging_b};
-  uint4 va[8], vb[8];
-  a.load(k_begin, k_end, va);
-  b.load(k_begin, k_end, vb);
+  const bool first = threadIdx.x < 128;
+  const Operand operand = first ? Operand{p.a, p.m, m0, 128u, p.sam, p.sak, staging_a}
+                                : Operand{p.b, p.n, 0u, nt, p.sbn, p.sbk, staging_b};
+  unsigned char* const to = first ? smem : smem + kGemmOffB;
+  uint4 chunk[8];
+  operand.load(k_begin, k_end, chunk);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(barrier), "r"(1u) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -449,8 +451,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, int stagi
   std::uint32_t phase = 0;
   std::uint32_t issued = 0;
   for (std::uint32_t k0 = k_begin; k0 < k_end; k0 += kGemmChunk) {
-    a.store(smem, va);
-    b.store(smem + kGemmOffB, vb);
+    operand.store(to, chunk);
     fence_async_smem();
     fence_before();
     __syncthreads();
@@ -464,10 +465,7 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, int stagi
       }
       commit(barrier);
     }
-    if (k0 + kGemmChunk < k_end) {
-      a.load(k0 + kGemmChunk, k_end, va);
-      b.load(k0 + kGemmChunk, k_end, vb);
-    }
+    if (k0 + kGemmChunk < k_end) operand.load(k0 + kGemmChunk, k_end, chunk);
     if (threadIdx.x == 0) {
       std::uint32_t polls = 0;
       while (!try_wait(barrier, phase)) {
@@ -484,11 +482,13 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, int stagi
     if (!ok) break;
   }
   fence_after();
-  // Epilogue: warp w holds rows 32w..32w+31 of the tile, one per lane.
-  const std::uint32_t warp = threadIdx.x >> 5;
+  // Epilogue: warps w and w + 4 hold rows 32w..32w+31 of the tile, one per
+  // lane, and take the columns below and from 64 on.
+  const std::uint32_t warp = (threadIdx.x >> 5) % 4;
   const std::uint32_t row = m0 + warp * 32 + (threadIdx.x & 31);
+  const std::uint32_t from = threadIdx.x < 128 ? 0u : 64u;
   if (ok) {
-    for (std::uint32_t c0 = 0; c0 < nt; c0 += 32) {
+    for (std::uint32_t c0 = from; c0 < smin(nt, from + 64u); c0 += 32) {
       float v[32];
       if (issued > 0) {
         load32(tmem + ((warp * 32u) << 16) + c0, v);
