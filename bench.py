@@ -169,7 +169,7 @@ def measured_peak():
 def ncu_traffic():
     """DRAM bytes of one BB iteration as a multiple of its algorithmic bytes,
     from the committed ncu capture (profiles/bb_iteration_traffic.json, the
-    1M-capsule colony's system after 2 steps: 2.2M rows, 1.04M bodies); None
+    tiled passes over a 400,000-capsule colony's system: 1.66M rows); None
     without one.  The bench scales it to its own launches by the algorithmic
     bytes, which grow with rows and bodies as the traffic does."""
     path = ROOT / "profiles" / "bb_iteration_traffic.json"
@@ -803,7 +803,7 @@ def main():
             # The timed steps' overlap re-checks by how their candidates were found.
             "rechecks": rechecks,
             "roofline": {
-                "kernel": "bb_iteration (body pass + row pass)",
+                "kernel": "bb_iteration (tile pass + boundary pass)",
                 "bound": "hbm",
                 "achieved": achieved,
                 "peak": peak,
