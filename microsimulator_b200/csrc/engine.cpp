@@ -793,11 +793,16 @@ struct HostResult {
   std::size_t bytes;
 };
 void download_results(Ctx& c, std::initializer_list<HostResult> results) {
-  constexpr std::size_t kPiece = std::size_t(1) << 19, kPieces = 12, kHalf = kPieces * kPiece;
-  constexpr std::size_t kDirect = std::size_t(1) << 18;  // up to this, plain copies cost less than waking the pool
+  constexpr std::size_t kPiece = std::size_t(1) << 19, kMostPieces = 12;
+  constexpr std::size_t kDirect = std::size_t(1) << 20;  // up to this, plain copies cost little more than waking the pool
   std::vector<HostResult> pieces;
   std::size_t total = 0;
   for (const auto& r : results) total += r.bytes;
+  // Pieces a half: 4, 8 or 16 MB of pinned memory in all (rounded up).  A new
+  // context's first call on 10 to 40 thousand bodies: 13 to 16 ms, against 21
+  // to 29 with 16 MB whatever the results; repeated calls take the same time.
+  const std::size_t half_pieces = total > (std::size_t(24) << 20) ? kMostPieces : total > (std::size_t(4) << 20) ? 6 : 3;
+  const std::size_t half_bytes = half_pieces * kPiece;
   for (const auto& r : results) {
     if (r.bytes == 0) continue;
     if (total <= kDirect || pinned_host(r.dst)) {
@@ -810,8 +815,8 @@ void download_results(Ctx& c, std::initializer_list<HostResult> results) {
     }
   }
   if (!pieces.empty()) {
-    unsigned char* const staging = c.download.ensure(2 * kHalf);
-    while (c.download_events.size() < 2 * kPieces) {
+    unsigned char* const staging = c.download.ensure(2 * half_bytes);
+    while (c.download_events.size() < 2 * kMostPieces) {
       cudaEvent_t e;
       check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
       c.download_events.push_back(e);
@@ -819,10 +824,10 @@ void download_results(Ctx& c, std::initializer_list<HostResult> results) {
     std::vector<msb::HostCopies::Job> jobs[2];
     std::size_t next = 0;
     const auto queue = [&](std::size_t half) {
-      for (std::size_t k = 0; k < kPieces && next < pieces.size(); ++k, ++next) {
+      for (std::size_t k = 0; k < half_pieces && next < pieces.size(); ++k, ++next) {
         const HostResult& piece = pieces[next];
-        unsigned char* const slot = staging + half * kHalf + k * kPiece;
-        const cudaEvent_t there = c.download_events[half * kPieces + k];
+        unsigned char* const slot = staging + half * half_bytes + k * kPiece;
+        const cudaEvent_t there = c.download_events[half * kMostPieces + k];
         check(cudaMemcpyAsync(slot, piece.device_src, piece.bytes, cudaMemcpyDeviceToHost, c.stream), "copy back");
         check(cudaEventRecord(there, c.stream), "event");
         jobs[half].push_back({piece.dst, slot, piece.bytes, there});
