@@ -412,9 +412,12 @@ int msb_advance_contact_dynamics_device(
     msb_contact_dynamics_report* report, msb_contact_dynamics_outputs* outputs);
 
 /* Measurement hook, no counterpart in the reference: runs `iterations` more
- * projected iterations of the last system this context solved, timing each
- * pass with CUDA events on the context's stream; returns the mean duration
- * of the body pass and of the row pass and the system's rows and bodies. */
+ * projected iterations of the last system this context solved (or evaluated
+ * since), timing each pass with CUDA events on the context's stream; returns
+ * the mean duration of the body pass and of the row pass (after a tiled
+ * solve: the tile pass and the boundary pass) and the system's rows and
+ * bodies.  MSB_ERR_INVALID_ARGUMENT without such a system: before the first
+ * solve, after a batch, after a step that failed. */
 int msb_profile_iterations(msb_context* context, uint32_t iterations, float* body_ms, float* row_ms,
                            uint64_t* rows, uint64_t* bodies);
 

@@ -197,7 +197,8 @@ class B200Backend:
 
     def profile_iterations(self, iterations: int = 20) -> dict:
         """Mean device time of one BB iteration's body and row passes on the
-        last solved system (CUDA events on the backend's stream)."""
+        last solved system (CUDA events on the backend's stream); after a
+        tiled solve, of its tile and boundary passes."""
         body, row = c_float(0), c_float(0)
         rows, bodies = c_uint64(0), c_uint64(0)
         self._check(self._lib.msb_profile_iterations(self._handle, iterations, ctypes.byref(body), ctypes.byref(row),

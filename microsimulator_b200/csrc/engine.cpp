@@ -600,7 +600,12 @@ struct msb_context {
 
   // solve
   int last_blocks = 0;
-  int last_tiled = 0;  // the last solved system was taken by tiles, this many blocks an SM
+  // What msb_profile_iterations may run on: whether `desc` describes a system
+  // whose arrays are as they were when it was filled, and whether that system
+  // was last solved by tiles (this many blocks an SM; 0: it was not, and
+  // desc->tiles is another system's).
+  bool desc_current = false;
+  int last_tiled = 0;
   msb::SolveDesc* desc = nullptr;
   msb::DBuf<double> partials;
   std::vector<std::unique_ptr<msb::SolveGraph>> graphs;
@@ -1306,6 +1311,8 @@ void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_
                std::uint32_t max_iterations, bool with_state = false) {
   SolveDesc& d = *c.host_desc;
   fill_problem(c, d, row_count, dt, growth, tolerance, max_iterations);
+  c.desc_current = true;
+  c.last_tiled = 0;
   if (with_state) {
     // The fused solve resets nothing itself: copy the state part too.
     d.step = 0.0f;
@@ -1394,7 +1401,6 @@ bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_r
   if (c.host_desc->gang.late != 0) throw DeviceCheckError("a wait of the resident solve ran out of time");
   if (c.host_desc->check_status != 0) throw DeviceCheckError("an index check of the resident solve failed");
   c.last_blocks = grid_for(std::max(c.rows.count, c.n), kSolveThreads, 4);
-  c.last_tiled = 0;
   return c.host_desc->gang.misfit == 0;
 }
 
@@ -1453,8 +1459,8 @@ int build_tiles(Ctx& c, TileArrays& out) {
   out = {c.tile_order.p,    c.tile_degree.p,   c.tile_slot_base.p, c.tile_group.p,     c.tile_a.p,
          c.tile_b.p,        c.tile_body_a.p,   c.tile_body_b.p,    c.tile_row_base.p,  c.tile_guest_base.p,
          c.tile_guests.p,   c.tile_row_of.p,   c.tile_constants.p, c.tile_iterate.p,   c.tile_first.p,
-         c.tile_second.p,   c.tile_boundary.p, tiles,              boundary,           max_slots,
-         max_rows,          max_locals};
+         c.tile_second.p,   c.tile_boundary.p, n,                  tiles,              boundary,
+         max_slots,         max_rows,          max_locals};
   return tile_blocks_per_sm(max_slots, max_rows, max_locals);
 }
 
@@ -1866,6 +1872,7 @@ void append_overlap_rows(Ctx& c, const Overlaps& o, const ResponseArrays& respon
   c.flagged.ensure(o.overlapping);
   launch_gather_flagged(c.found.p, o.candidates, c.flags.p, c.flag_offsets.p, c.flagged.p, c.stream);
   const std::uint32_t base_row = c.rows.count;
+  c.desc_current = false;
   c.rows.grow(std::size_t(base_row) + o.overlapping, c.stream);
   launch_make_rows(c.flagged.p, o.overlapping, c.trial.view(), build, &response, c.rows.arrays(), base_row,
                    c.rows.partner.p, c.rows.multipliers.p, c.scalars.p + kOverlapBits, c.stream, colonies_of(c));
@@ -1964,6 +1971,7 @@ void guess_forces(Ctx& c, float dt, const msb_growth_load_response& growth) {
 Attempt advance_substep(Ctx& c, float dt, const msb_contact_dynamics_parameters& p, const msb_contact_parameters& cp,
                         const msb_constraint_contact_parameters& wp, bool probe, std::uint64_t& iterations) {
   const std::uint32_t n = c.n;
+  c.desc_current = false;
   c.has_drift = false;  // no drift unless flow drift writes it below
   if (c.colonies > 0) {
     // Every colony takes part in the substep's first search and test.
@@ -2243,6 +2251,7 @@ void write_outputs(Ctx& c, msb_contact_dynamics_outputs* outputs, bool device_po
 // Uploads a ContactSystem's records as the context's rows and bodies.
 void load_system(Ctx& c, const msb_contact_system& s, const float* multipliers) {
   validate_system(s);
+  c.desc_current = false;
   c.n = std::uint32_t(s.body_count);
   c.spatial_valid = false;  // the records carry no geometry
   c.has_drift = false;
@@ -2960,7 +2969,7 @@ int msb_profile_iterations(msb_context* context, uint32_t iterations, float* bod
                            uint64_t* rows, uint64_t* bodies) {
   return guarded(context, [&] {
     auto& c = *context;
-    if (c.last_blocks == 0 || iterations == 0) throw std::invalid_argument("no solved system to time");
+    if (c.last_blocks == 0 || !c.desc_current || iterations == 0) throw std::invalid_argument("no solved system to time");
     cudaEvent_t start, between, stop;
     check(cudaEventCreate(&start), "event");
     check(cudaEventCreate(&between), "event");

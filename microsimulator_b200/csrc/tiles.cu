@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
   // A local copy: the descriptor may change under the stores below, for all
   // the compiler knows.
   const TileArrays t = d.tiles;
-  const std::uint32_t bodies = d.body_count;
+  const std::uint32_t bodies = t.bodies;
   const bool project = mode == 1;
   const float alpha = d.step;
   const float dt = d.dt;

@@ -41,6 +41,7 @@ struct TileArrays {
   float* first;                    // boundary rows' side terms
   float* second;
   const std::uint32_t* boundary;   // the boundary rows
+  std::uint32_t bodies;
   std::uint32_t tiles;
   std::uint32_t boundary_count;
   std::uint32_t max_slots;         // of any tile

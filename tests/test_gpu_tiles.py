@@ -7,8 +7,10 @@ import pytest
 
 from microsimulator_b200 import workloads
 from microsimulator_b200.backend import B200Backend
+from microsimulator_b200.sweep import ColonyBatch
 from microsimulator_b200.types import ContactDynamicsParameters, GrowthLoadResponse
 from microsimulator_b200.world import WorldState
+from tests.systems import LAWS, mixed_system, multipliers_for
 
 pytestmark = pytest.mark.gpu
 
@@ -62,3 +64,26 @@ def test_a_body_of_many_rows(forms, cells):
                   np.append(fields["direction_z"], 0.0)], axis=1),
         np.append(fields["lengths"], 120.0), 0.5, growth_rates=0.5)
     step_both(forms, long)
+
+
+def test_timing_hook_times_the_system_it_reports(forms):
+    """Systems loaded after a tiled solve are timed by slot: evaluated or
+    bounded ones with more bodies than the tiles, whose last tile is partly
+    filled.  A batch leaves no system to time."""
+    cells = 170_001
+    world = workloads.jammed(cells, seed=6)
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4)
+    forms.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+    for k, call in enumerate((forms.evaluate_contact_response, forms.evaluate_contact_gaps,
+                              lambda system, _: forms.contact_system_diagonal_bound(system))):
+        forms.advance_contact_dynamics(world.copy(), None, 0.002, p)
+        assert forms.profile_iterations(1)["bodies"] == cells
+        system = mixed_system(k, cells + 255 + k, 5000 + k, LAWS[2])
+        call(system, multipliers_for(system, k))
+        timed = forms.profile_iterations(1)
+        assert (timed["rows"], timed["bodies"]) == (5000 + k, cells + 255 + k)
+    sizes = [40, 300]
+    batch = ColonyBatch([workloads.sweep_colony(n, seed=n) for n in sizes], np.full(2, 1.0), np.full(2, 1.0e4))
+    forms.advance_contact_dynamics_batch(batch.concatenated(), batch.counts(), batch.drag, batch.stiffness, 0.002, p)
+    with pytest.raises(ValueError, match="no solved system"):
+        forms.profile_iterations(1)
