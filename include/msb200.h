@@ -467,6 +467,13 @@ int msb_set_search_reuse(msb_context* context, uint32_t mode);
  * lengths can differ in the last bits. */
 int msb_set_relaxation(msb_context* context, uint32_t form);
 
+/* Polls after which a wait inside a tiled solve's kernels gives up and the
+ * call fails with MSB_ERR_DEVICE_CHECK (the default, MSB_WAIT_POLLS: some
+ * seconds).  0: what is not there at once is not waited for, which tests use
+ * to take the failure's path. */
+#define MSB_WAIT_POLLS 8388608u
+int msb_set_wait_limit(msb_context* context, uint32_t polls);
+
 /* Warm starts of the stepper, extensions with no counterpart in the
  * reference (whose stepper starts every step from zero multipliers and keeps
  * no state between steps, contact_dynamics.cpp:725).  `mode` ORs flags:

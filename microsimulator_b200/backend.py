@@ -135,6 +135,13 @@ class B200Backend:
         cooperative kernel with grid barriers."""
         self._check(self._lib.msb_set_relaxation(self._handle, form))
 
+    WAIT_POLLS = 1 << 23
+
+    def set_wait_limit(self, polls: int = WAIT_POLLS) -> None:
+        """Polls after which a wait inside a solve's kernels gives up and the
+        call raises; 0 does not wait for what is not there at once."""
+        self._check(self._lib.msb_set_wait_limit(self._handle, polls))
+
     WARM_START_ZERO = 0
     WARM_START_CARRY = 1
     WARM_START_GUESS = 2

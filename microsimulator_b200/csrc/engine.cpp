@@ -605,6 +605,7 @@ struct msb_context {
   // was last solved by tiles (this many blocks an SM; 0: it was not, and
   // desc->tiles is another system's).
   bool desc_current = false;
+  std::uint32_t wait_polls = msb::kWaitPolls;
   int last_tiled = 0;
   msb::SolveDesc* desc = nullptr;
   msb::DBuf<double> partials;
@@ -1305,6 +1306,7 @@ void fill_problem(Ctx& c, SolveDesc& d, std::uint32_t row_count, float dt, const
   d.tolerance = tolerance;
   d.max_iterations = max_iterations;
   d.has_drift = c.has_drift ? 1u : 0u;
+  d.wait_polls = c.wait_polls;
 }
 
 void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_response& growth, float tolerance,
@@ -1525,7 +1527,10 @@ SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, flo
   sync(c);
   const SolveDesc& d = *c.host_desc;
   if (d.barrier_abort != 0) throw DeviceCheckError("a grid barrier of the relaxation ran out of time");
-  if (d.check_status != 0) throw DeviceCheckError("an index check or a bounded wait of the relaxation failed");
+  if (d.check_status != 0) {
+    throw DeviceCheckError("an index check or a bounded wait of the relaxation failed at iteration " +
+                           std::to_string(d.iterations));
+  }
   if (!fused) count_launch(SolveGraph::loop_launches(d.iterations));
   c.solve_log.push_back({rows, d.iterations, d.status, d.residual});
   if (d.status == 3) throw std::invalid_argument("contact system has no positive diagonal");
@@ -2558,6 +2563,10 @@ int msb_set_flow_field(msb_context* context, const msb_flow_field* field) {
     c.flow_travel_limit = 0.25f * std::min({field->spacing.x, field->spacing.y, field->spacing.z});
     c.has_flow = true;
   });
+}
+
+int msb_set_wait_limit(msb_context* context, uint32_t polls) {
+  return guarded(context, [&] { context->wait_polls = polls; });
 }
 
 int msb_set_relaxation(msb_context* context, uint32_t form) {

@@ -71,6 +71,10 @@ struct ResidentGang {
   std::uint32_t late;
 };
 
+// The ordinary SolveDesc::wait_polls: some seconds of trips to L2 at half a
+// microsecond each.
+constexpr std::uint32_t kWaitPolls = 1u << 23;
+
 // Everything one solve reads and writes, in device memory at a fixed address
 // so that the captured solve graph can be replayed for any system.
 struct SolveDesc {
@@ -95,6 +99,7 @@ struct SolveDesc {
   float tolerance;
   std::uint32_t max_iterations;
   std::uint32_t has_drift;  // 0: every drift is zero and the drift arrays are not read
+  std::uint32_t wait_polls;  // polls after which a device-side wait gives up
   TileArrays tiles;         // of a tiled solve
   // solver state
   float step;
@@ -112,7 +117,7 @@ struct SolveDesc {
   std::uint32_t barrier_count;
   std::uint32_t barrier_generation;
   std::uint32_t barrier_abort;  // a barrier wait ran out of time: every block stops
-  std::uint32_t check_status;   // checked build: the first index check that failed (0: none)
+  std::uint32_t check_status;   // the first failed check (0: none): a wait that ran out; checked build: an index
   ResidentGang gang;            // the resident solve's
 };
 

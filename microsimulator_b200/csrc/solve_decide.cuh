@@ -128,6 +128,9 @@ __device__ __forceinline__ std::uint32_t decide(SolveDesc& d, std::uint32_t mode
       proceed = iteration < d.max_iterations ? 1u : 0u;
     }
   }
+  // A failed check ends the solve: the sums may lack a block's, and every
+  // further iteration could wait as long again.
+  if (__ldcg(&d.check_status) != 0u) proceed = 0;
   d.proceed = proceed;
   return proceed;
 }

@@ -46,7 +46,6 @@ constexpr int kThreads = kSolveThreads;
 static_assert(kThreads == int(kTileBodies), "one thread per body of a tile");
 constexpr int kRowBatch = 4;  // rows of a thread whose loads are in flight together
 constexpr int kGuests = 2;    // guests of a thread fetched ahead
-constexpr std::uint32_t kWaitPolls = 1u << 24;
 
 extern __shared__ __align__(128) unsigned char tile_memory[];
 
@@ -95,8 +94,8 @@ __device__ __forceinline__ void fetch_rows(const Tile& tile, const float2* itera
   bulk_copy(to_iterate, iterate + (tile.r0 - tile.skip()), bytes, barrier);
   bulk_copy(to_constants, constants + (tile.r0 - tile.skip()), bytes, barrier);
 }
-__device__ __forceinline__ bool entries_there(std::uint32_t barrier, std::uint32_t phase) {
-  for (std::uint32_t polls = 0; polls < kWaitPolls; ++polls) {
+__device__ __forceinline__ bool entries_there(std::uint32_t barrier, std::uint32_t phase, std::uint32_t limit) {
+  for (std::uint32_t polls = 0; polls < limit; ++polls) {
     std::uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
@@ -189,8 +188,7 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
     for (std::uint32_t g = threadIdx.x + kGuests * kThreads; g < now.guests; g += kThreads) {
       multiplier[now.rows + g] = projected(t.iterate[t.guests[now.g0 + g]]);
     }
-    const bool there = entries_there(barrier, phase);
-    phase ^= 1u;
+    const bool there = entries_there(barrier, phase, d.wait_polls);
     // The multipliers of the tile's rows, projected; a constraint row's
     // second side adds nothing.
     for (std::uint32_t j = threadIdx.x; j < now.rows; j += kThreads) {
@@ -198,9 +196,14 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
       side[j].y = -0.0f;
     }
     if (__syncthreads_or(!there) != 0) {
-      if (threadIdx.x == 0) raise_status(check, kStatusIterations);
+      if (threadIdx.x == 0) {
+        raise_status(check, kStatusIterations);  // ends the solve (decide)
+        // The block keeps its shared memory until the copies into it are done.
+        entries_there(barrier, phase, kWaitPolls);
+      }
       return;
     }
+    phase ^= 1u;
     if (live) {
       const std::uint32_t locals = now.rows + now.guests;
       float w[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};

@@ -5,7 +5,7 @@ tolerances (two solves of one system may differ by that)."""
 import numpy as np
 import pytest
 
-from microsimulator_b200 import workloads
+from microsimulator_b200 import abi, workloads
 from microsimulator_b200.backend import B200Backend
 from microsimulator_b200.sweep import ColonyBatch
 from microsimulator_b200.types import ContactDynamicsParameters, GrowthLoadResponse
@@ -64,6 +64,26 @@ def test_a_body_of_many_rows(forms, cells):
                   np.append(fields["direction_z"], 0.0)], axis=1),
         np.append(fields["lengths"], 120.0), 0.5, growth_rates=0.5)
     step_both(forms, long)
+
+
+def test_a_copy_that_is_late_ends_the_solve(forms):
+    """With no polls allowed the tiles' copies count as late: the solve ends
+    with its first pass (not after max_iterations of them, on sums that the
+    blocks never wrote), its copies drained, and the next call is sound."""
+    world = workloads.jammed(170_001, seed=6)
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4)
+    forms.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+    expected = world.copy()
+    forms.advance_contact_dynamics(expected, None, 0.002, p)
+    forms.set_wait_limit(0)
+    try:
+        with pytest.raises(abi.NativeError, match="wait of the relaxation failed at iteration 0$"):
+            forms.advance_contact_dynamics(world.copy(), None, 0.002, p)
+    finally:
+        forms.set_wait_limit()
+    again = world.copy()
+    forms.advance_contact_dynamics(again, None, 0.002, p)
+    assert np.array_equal(again.geometry(), expected.geometry())
 
 
 def test_timing_hook_times_the_system_it_reports(forms):
