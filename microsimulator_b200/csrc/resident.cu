@@ -20,7 +20,10 @@
 // is one 64-bit word (round, value) in that CTA's global inbox, which its
 // owner polls; the sums are words of the same kind that every CTA reads and
 // adds in CTA order, so no CTA waits for another's decision and no grid
-// barrier is needed.  Every wait is bounded (kWaitPolls).
+// barrier is needed.  Every wait for a word is bounded (SolveDesc::wait_polls:
+// seconds), and so is a gang's wait for its CTAs to arrive and to leave, which
+// may have to finish other systems first (wait_count: minutes, or until
+// another CTA has given up).
 #include "resident.h"
 
 #include <cooperative_groups.h>
@@ -117,9 +120,6 @@ __device__ __forceinline__ void pad_slot(const Layout& l, std::uint32_t j) {
   l.own(j) = l.inbox(j) = 0.0f;
 }
 
-// A wait gives up after this many polls (each a trip to L2, about half a
-// microsecond: some seconds).
-constexpr std::uint32_t kWaitPolls = 1u << 23;
 __device__ __forceinline__ void put_word(unsigned long long* p, std::uint32_t tag, std::uint32_t value) {
   const unsigned long long w = (static_cast<unsigned long long>(tag) << 32) | value;
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
@@ -146,20 +146,28 @@ __device__ __forceinline__ ulonglong2 get_wide(const ulonglong2* p) {
   return w;
 }
 // Waits until *p carries `tag`; false once the wait has run out.
-__device__ __forceinline__ bool wait_word(const unsigned long long* p, std::uint32_t tag, unsigned long long& word) {
+__device__ __forceinline__ bool wait_word(const unsigned long long* p, std::uint32_t tag, unsigned long long& word,
+                                          std::uint32_t limit) {
   for (std::uint32_t polls = 0; std::uint32_t(word >> 32) != tag; ++polls) {
-    if (polls == kWaitPolls) return false;
+    if (polls == limit) return false;
     word = get_word(p);
   }
   return true;
 }
 
-// Waits until *p has reached `count`, a gang's CTAs having arrived: they may
-// first finish other systems.
-__device__ __forceinline__ bool wait_count(const std::uint32_t* p, std::uint32_t count) {
-  for (std::uint32_t polls = 0; *static_cast<const volatile std::uint32_t*>(p) < count; ++polls) {
-    if (polls == (1u << 28)) return false;
-    if (polls > 1024u) __nanosleep(500);
+// Waits until *p has reached `count`, a gang's CTAs having arrived or left:
+// they may first finish other systems, so the limit is 32 times a word's
+// (2^28 polls of half a microsecond: about two minutes).  False once it has
+// run out or another CTA has set *late.
+__device__ __forceinline__ bool wait_count(const std::uint32_t* p, std::uint32_t count, std::uint32_t limit,
+                                           const std::uint32_t* late) {
+  const auto read = [](const std::uint32_t* from) { return *static_cast<const volatile std::uint32_t*>(from); };
+  for (std::uint64_t polls = 0; read(p) < count; ++polls) {
+    if (polls >= 32ull * limit) return false;
+    if (polls > 1024u) {
+      if (read(late) != 0u) return false;
+      __nanosleep(500);
+    }
   }
   return true;
 }
@@ -204,6 +212,8 @@ struct Comm {
   std::uint32_t first = 0;  // grid form: the first of the gang's CTAs
   std::uint32_t round = 0;  // grid form: tags words, never falls within a launch
   ResidentGang* gang = nullptr;
+  std::uint32_t* late = nullptr;   // grid form: set once a CTA has given up a wait
+  std::uint32_t wait_polls = 0;
 
   __device__ void sync_all() const {
     if constexpr (kForm == kCluster) {
@@ -250,7 +260,7 @@ struct Comm {
 #pragma unroll
         for (int t = 0; t < kFlight; ++t) {
           if (x0 + t * kThreads < s.remote_count) {
-            late = !wait_word(words + slot[t], round, w[t]) || late;
+            late = !wait_word(words + slot[t], round, w[t], wait_polls) || late;
             l.inbox(slot[t]) = __uint_as_float(std::uint32_t(w[t]));
           }
         }
@@ -308,7 +318,7 @@ __device__ __forceinline__ bool get_record(const Comm<kGrid>& comm, std::uint32_
     return all;
   };
   for (std::uint32_t polls = 0; !there(); ++polls) {
-    if (polls == kWaitPolls) return false;
+    if (polls == comm.wait_polls) return false;
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) x.v[k] = __longlong_as_double(static_cast<long long>(w[k].x));
@@ -481,10 +491,13 @@ __device__ __forceinline__ Sums receive_sides(const SolveDesc& d, const Layout& 
   return s;
 }
 
-// Loads this CTA's share of bodies [b0, b1).  False (in every CTA) when some
-// CTA's share does not fit `bytes` of shared memory.
+enum Outcome { kSolved, kMisfit, kLate };
+
+// Loads this CTA's share of bodies [b0, b1).  kMisfit (in every CTA) when some
+// CTA's share does not fit `bytes` of shared memory; kLate when the other CTAs
+// did not arrive in time.
 template <int kForm>
-__device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm, Shared& s, Layout& l,
+__device__ Outcome load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm, Shared& s, Layout& l,
                            std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1, std::uint32_t* check) {
   const std::uint32_t* offsets = r.order != nullptr ? r.order_offsets : d.incidence.offsets;
   const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -654,12 +667,10 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
       atomicMax(&gang.base, comm.round);
       __threadfence();
       atomicAdd(&gang.arrived, 1u);
-      if (!wait_count(&gang.arrived, comm.size)) {
-        atomicExch(&gang.late, 1u);
-        s.misfit = 1u;
-      }
+      const bool late = !wait_count(&gang.arrived, comm.size, comm.wait_polls, comm.late);
       __threadfence();
       if (*static_cast<volatile std::uint32_t*>(&gang.misfit) != 0u) s.misfit = 1u;
+      if (late) s.misfit = 2u;
       s.round = *static_cast<volatile std::uint32_t*>(&gang.base);
     }
     __syncthreads();
@@ -676,7 +687,7 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
   } else {
     __syncthreads();
   }
-  if (s.misfit != 0) return false;
+  if (s.misfit != 0) return s.misfit == 2u ? kLate : kMisfit;
   // Where each entry's side terms go: the other entry of its row.
   for (std::uint32_t q = threadIdx.x; q < bodies; q += kThreads) {
     const std::uint32_t degree = l.degree(q);
@@ -710,14 +721,13 @@ __device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kFo
     }
   }
   __syncthreads();
-  return true;
+  return kSolved;
 }
 
 struct Report {
   float step, residual, bound;
   std::uint32_t iterations, status;
 };
-enum Outcome { kSolved, kMisfit, kLate };
 
 // The whole solve of bodies [b0, b1) by the CTAs of `comm`.
 template <int kForm, int P>
@@ -725,7 +735,8 @@ __device__ __forceinline__ Outcome resident_solve(const SolveDesc& d, const Resi
                                                   Shared& s, std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1,
                                                   float tolerance, std::uint32_t* check, Report& report) {
   Layout l{};
-  if (!load_share(d, r, comm, s, l, bytes, b0, b1, check)) return kMisfit;
+  const Outcome loaded = load_share(d, r, comm, s, l, bytes, b0, b1, check);
+  if (loaded != kSolved) return loaded;
   // Every thread takes the same decisions from the same sums.  The rounds
   // share one copy of the code: what a round executes is fetched once per
   // iteration, by few warps, so its size counts.
@@ -800,6 +811,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   Comm<kForm> comm{blockIdx.x, gridDim.x, &arrays};
   if constexpr (kForm == kGrid) {
     comm.gang = &state->gang;
+    comm.late = &state->gang.late;
+    comm.wait_polls = problem.wait_polls;
     clear_words(comm);
   }
   Report report;
@@ -844,7 +857,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       Comm<kSingle> comm{0, 1, &arrays};
       outcome = resident_solve<kSingle, 1>(problem, arrays, comm, s, bytes, b0, b1, tolerance, batch.check, report);
     } else {
-      Comm<kGrid> comm{blockIdx.x - job.first, job.size, &arrays, job.first, round, &batch.gangs[batch.lists[k]]};
+      Comm<kGrid> comm{blockIdx.x - job.first, job.size,  &arrays, job.first, round, &batch.gangs[batch.lists[k]],
+                       batch.late,             problem.wait_polls};
       outcome = resident_solve<kGrid, 1>(problem, arrays, comm, s, bytes, b0, b1, tolerance, batch.check, report);
       rank = comm.rank;
       round = comm.round;
@@ -868,7 +882,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ResidentGang& gang = batch.gangs[batch.lists[k]];
         __threadfence();
         atomicAdd(&gang.left, 1u);
-        late = !wait_count(&gang.left, job.size);
+        late = !wait_count(&gang.left, job.size, problem.wait_polls, batch.late);
       } else if (job.size > 1) {
         atomicAdd(&batch.gangs[batch.lists[k]].left, 1u);
       }

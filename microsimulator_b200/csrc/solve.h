@@ -68,7 +68,7 @@ struct ResidentGang {
   std::uint32_t left;
   std::uint32_t base;
   std::uint32_t misfit;
-  std::uint32_t late;
+  std::uint32_t late;  // of a single system; a batch's is ResidentBatch::late
 };
 
 // The ordinary SolveDesc::wait_polls: some seconds of trips to L2 at half a

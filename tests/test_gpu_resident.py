@@ -89,6 +89,37 @@ def test_empty_bodies_and_profile_hook(forms):
     assert forms.profile_iterations(2)["rows"] == 300
 
 
+def test_waits_that_run_out_fail_the_call(forms):
+    """With no polls allowed the grid's CTAs do not wait for one another: the
+    solve and a batch's gangs (whose CTAs then count as late, not as misfits)
+    fail, and the next calls are sound."""
+    system = mixed_system(1, 20000, 40000, LAWS[0])
+    initial = multipliers_for(system, 1)
+    parameters = ContactSolveParameters(1e-9, 3)
+    sizes = [300, 12000, 9000]
+    batch = ColonyBatch([workloads.sweep_colony(n, seed=n) for n in sizes], np.full(3, 1.0), np.full(3, 1.0e4))
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4)
+
+    def step():
+        cells = batch.concatenated()
+        forms.advance_contact_dynamics_batch(cells, batch.counts(), batch.drag, batch.stiffness, 0.002, p)
+        return cells.geometry()
+
+    forms.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+    step()
+    expected = forms.solve_contact_forces(system, initial, parameters).multipliers, step()
+    forms.set_wait_limit(0)
+    try:
+        with pytest.raises(abi.NativeError, match="wait of the resident solve ran out"):
+            forms.solve_contact_forces(system, initial, parameters)
+        with pytest.raises(abi.NativeError, match="wait of the batched resident solve ran out"):
+            step()
+    finally:
+        forms.set_wait_limit()
+    assert np.array_equal(forms.solve_contact_forces(system, initial, parameters).multipliers, expected[0])
+    assert np.array_equal(step(), expected[1])
+
+
 @pytest.mark.parametrize("cells", [9000, 30000])
 @pytest.mark.parametrize("flat", [True, False])
 def test_steps_in_spatial_order(forms, cells, flat):
