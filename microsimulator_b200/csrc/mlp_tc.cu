@@ -498,10 +498,15 @@ __global__ void __launch_bounds__(kGemmThreads) gemm_tc_kernel(Gemm p, int stagi
       }
       if (p.z != nullptr) {
         const std::size_t at = std::size_t(row) * p.n + c0;
+        // The caller's activations: 16 bytes a load where they allow it.
+        const bool wide = reinterpret_cast<std::uintptr_t>(p.z) % 16 == 0;
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
           float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          if (row < p.m) z = *reinterpret_cast<const float4*>(p.z + at + j);
+          const float* from = p.z + at + j;
+          if (row < p.m) {
+            z = wide ? *reinterpret_cast<const float4*>(from) : make_float4(from[0], from[1], from[2], from[3]);
+          }
           v[j] = row < p.m ? v[j] * gelu_grad(z.x) : 0.0f;
           v[j + 1] = row < p.m ? v[j + 1] * gelu_grad(z.y) : 0.0f;
           v[j + 2] = row < p.m ? v[j + 2] * gelu_grad(z.z) : 0.0f;

@@ -51,11 +51,13 @@ def test_unaligned_operands_give_the_same_bits(backend):
     shifted[1:] = xt.reshape(-1)
     weights = torch.empty(net.weights.numel() + 1, dtype=torch.int16, device=DEVICE)
     weights[1:] = net.weights
+    activations = torch.empty(act.numel() + 4, dtype=torch.uint8, device=DEVICE)
+    activations[4:] = act
     scratch = torch.empty(int(lib.msb_mlp_backward_scratch_bytes(n)) + 4, dtype=torch.uint8, device=DEVICE)
     grads = torch.zeros_like(net.grads)
     stream = ctypes.c_void_p(torch.cuda.current_stream(DEVICE).cuda_stream)
     net._check(lib.msb_mlp_backward(
         ctypes.c_void_p(weights.data_ptr() + 2), ctypes.c_void_p(shifted.data_ptr() + 2), n,
-        ctypes.c_void_p(act.data_ptr()), ctypes.c_void_p(dy.data_ptr()), ctypes.c_void_p(grads.data_ptr()),
+        ctypes.c_void_p(activations.data_ptr() + 4), ctypes.c_void_p(dy.data_ptr()), ctypes.c_void_p(grads.data_ptr()),
         ctypes.c_void_p(scratch.data_ptr() + 4), stream))
     assert torch.equal(grads, expected)
