@@ -467,10 +467,11 @@ int msb_set_search_reuse(msb_context* context, uint32_t mode);
  * lengths can differ in the last bits. */
 int msb_set_relaxation(msb_context* context, uint32_t form);
 
-/* Polls after which a wait inside the kernels of a tiled or resident solve
- * gives up and the call fails with MSB_ERR_DEVICE_CHECK (the default,
- * MSB_WAIT_POLLS: some seconds; 32 times as many where the CTAs of a batch's
- * colony wait for one that still solves another).  0: what is not there at once is not waited for, which tests use
+/* Polls after which a wait inside the kernels of a tiled solve (for a copy)
+ * or a resident one (for its CTAs to arrive and to leave: 32 times as many,
+ * since one may still solve another colony of a batch) gives up and the call
+ * fails with MSB_ERR_DEVICE_CHECK.  The default, MSB_WAIT_POLLS, is some
+ * seconds.  0: what is not there at once is not waited for, which tests use
  * to take the failure's path. */
 #define MSB_WAIT_POLLS 8388608u
 int msb_set_wait_limit(msb_context* context, uint32_t polls);

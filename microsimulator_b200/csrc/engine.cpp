@@ -1461,8 +1461,8 @@ int build_tiles(Ctx& c, TileArrays& out) {
   out = {c.tile_order.p,    c.tile_degree.p,   c.tile_slot_base.p, c.tile_group.p,     c.tile_a.p,
          c.tile_b.p,        c.tile_body_a.p,   c.tile_body_b.p,    c.tile_row_base.p,  c.tile_guest_base.p,
          c.tile_guests.p,   c.tile_row_of.p,   c.tile_constants.p, c.tile_iterate.p,   c.tile_first.p,
-         c.tile_second.p,   c.tile_boundary.p, n,                  tiles,              boundary,
-         max_slots,         max_rows,          max_locals};
+         c.tile_second.p,   c.tile_boundary.p, tiles,              boundary,           max_slots,
+         max_rows,          max_locals};
   return tile_blocks_per_sm(max_slots, max_rows, max_locals);
 }
 
@@ -1509,7 +1509,7 @@ SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, flo
     auto& made = c.tile_graphs[tiled];
     if (tiled > 0 && !made) {
       auto fresh = std::make_unique<SolveGraph>();
-      check(cudaError_t(fresh->create(c.desc, kMaxPassBlocks, c.stream, tiled)), "solve graph");
+      check(cudaError_t(fresh->create(c.desc, kMaxPassBlocks, c.stream, tiled, c.wait_polls)), "solve graph");
       made = std::move(fresh);
     }
     check(cudaError_t((tiled > 0 ? *made : graph).launch(c.stream)), "solve launch");
@@ -2566,7 +2566,10 @@ int msb_set_flow_field(msb_context* context, const msb_flow_field* field) {
 }
 
 int msb_set_wait_limit(msb_context* context, uint32_t polls) {
-  return guarded(context, [&] { context->wait_polls = polls; });
+  return guarded(context, [&] {
+    context->wait_polls = polls;
+    for (auto& graph : context->tile_graphs) graph.reset();  // they hold the polls
+  });
 }
 
 int msb_set_relaxation(msb_context* context, uint32_t form) {
@@ -2986,7 +2989,7 @@ int msb_profile_iterations(msb_context* context, uint32_t iterations, float* bod
     // Warm the caches as the solve loop does.
     const auto iterate = [&](cudaEvent_t middle) {
       if (c.last_tiled > 0) {
-        launch_tile_iteration(c.desc, c.last_tiled, middle, c.stream);
+        launch_tile_iteration(c.desc, c.last_tiled, c.wait_polls, middle, c.stream);
       } else {
         launch_iteration(c.desc, c.last_blocks, middle, c.stream);
       }

@@ -20,10 +20,10 @@
 // is one 64-bit word (round, value) in that CTA's global inbox, which its
 // owner polls; the sums are words of the same kind that every CTA reads and
 // adds in CTA order, so no CTA waits for another's decision and no grid
-// barrier is needed.  Every wait for a word is bounded (SolveDesc::wait_polls:
-// seconds), and so is a gang's wait for its CTAs to arrive and to leave, which
-// may have to finish other systems first (wait_count: minutes, or until
-// another CTA has given up).
+// barrier is needed.  Every wait for a word is bounded (kWaitPolls: seconds),
+// and so is a gang's wait for its CTAs to arrive and to leave, which may have
+// to finish other systems first (wait_count: minutes, or until another CTA has
+// given up).
 #include "resident.h"
 
 #include <cooperative_groups.h>
@@ -145,19 +145,20 @@ __device__ __forceinline__ ulonglong2 get_wide(const ulonglong2* p) {
                : "memory");
   return w;
 }
-// Waits until *p carries `tag`; false once the wait has run out.
-__device__ __forceinline__ bool wait_word(const unsigned long long* p, std::uint32_t tag, unsigned long long& word,
-                                          std::uint32_t limit) {
+// Waits until *p carries `tag`; false once the wait has run out.  (A limit
+// that is no constant costs more than its comparison: a step of 60,000 cells
+// took 7.4 ms for 6.7.)
+__device__ __forceinline__ bool wait_word(const unsigned long long* p, std::uint32_t tag, unsigned long long& word) {
   for (std::uint32_t polls = 0; std::uint32_t(word >> 32) != tag; ++polls) {
-    if (polls == limit) return false;
+    if (polls == kWaitPolls) return false;
     word = get_word(p);
   }
   return true;
 }
 
 // Waits until *p has reached `count`, a gang's CTAs having arrived or left:
-// they may first finish other systems, so the limit is 32 times a word's
-// (2^28 polls of half a microsecond: about two minutes).  False once it has
+// they may first finish other systems, so the limit is 32 * `limit` polls (by
+// default 2^28 of half a microsecond: about two minutes).  False once it has
 // run out or another CTA has set *late.
 __device__ __forceinline__ bool wait_count(const std::uint32_t* p, std::uint32_t count, std::uint32_t limit,
                                            const std::uint32_t* late) {
@@ -260,7 +261,7 @@ struct Comm {
 #pragma unroll
         for (int t = 0; t < kFlight; ++t) {
           if (x0 + t * kThreads < s.remote_count) {
-            late = !wait_word(words + slot[t], round, w[t], wait_polls) || late;
+            late = !wait_word(words + slot[t], round, w[t]) || late;
             l.inbox(slot[t]) = __uint_as_float(std::uint32_t(w[t]));
           }
         }
@@ -318,7 +319,7 @@ __device__ __forceinline__ bool get_record(const Comm<kGrid>& comm, std::uint32_
     return all;
   };
   for (std::uint32_t polls = 0; !there(); ++polls) {
-    if (polls == comm.wait_polls) return false;
+    if (polls == kWaitPolls) return false;
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) x.v[k] = __longlong_as_double(static_cast<long long>(w[k].x));

@@ -643,7 +643,7 @@ SolveGraph::~SolveGraph() {
   if (graph_ != nullptr) cudaGraphDestroy(graph_);
 }
 
-int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream, int tiles_per_sm) {
+int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream, int tiles_per_sm, std::uint32_t wait_polls) {
   // At most one resident wave: a grid-stride pass whose blocks do not all
   // fit at once leaves a partly empty second wave.
   int device = 0, sms = kSmCount, body_active = 1, row_active = 1;
@@ -689,7 +689,7 @@ int SolveGraph::create(SolveDesc* desc, int blocks, cudaStream_t stream, int til
   int with_condition = 1;
   void* reset_args[] = {&d};
   void* bound_args[] = {&d};
-  void* body_args[] = {&d, &mode_auto};
+  void* body_args[] = {&d, &mode_auto, &wait_polls};  // the last: tiled only
   void* row_args[] = {&d, &mode_auto, &with_condition, &first_blocks};  // the last: tiled only
   cudaGraphNode_t reset, bound, body0, row0, loop;
   if ((err = kernel_node(graph_, &reset, nullptr, 0, (void*)solve_reset_kernel, reset_args, 1, 32)) != cudaSuccess) return err;

@@ -99,7 +99,7 @@ struct SolveDesc {
   float tolerance;
   std::uint32_t max_iterations;
   std::uint32_t has_drift;  // 0: every drift is zero and the drift arrays are not read
-  std::uint32_t wait_polls;  // polls after which a device-side wait gives up
+  std::uint32_t wait_polls;  // a 32nd of the polls after which a resident solve's CTAs are late
   TileArrays tiles;         // of a tiled solve
   // solver state
   float step;
@@ -142,8 +142,9 @@ class SolveGraph {
   SolveGraph& operator=(const SolveGraph&) = delete;
   ~SolveGraph();
   // `tiles_per_sm` > 0: the passes of tiles.cu, which read desc->tiles, with
-  // that many blocks an SM.  Returns a CUDA error code.
-  int create(SolveDesc* desc, int blocks, cudaStream_t stream, int tiles_per_sm = 0);
+  // that many blocks an SM and `wait_polls`.  Returns a CUDA error code.
+  int create(SolveDesc* desc, int blocks, cudaStream_t stream, int tiles_per_sm = 0,
+             std::uint32_t wait_polls = kWaitPolls);
   int launch(cudaStream_t stream);
   int blocks() const { return blocks_; }
   // Kernel launches of the WHILE node for a solve of `iterations`

@@ -66,6 +66,7 @@ __device__ __forceinline__ std::uint32_t decide(SolveDesc& d, std::uint32_t mode
   __shared__ double red[5][kSolveThreads / 32];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
+  const std::uint32_t failed = __ldcg(&d.check_status);
   double t[5] = {0.0, 0.0, 0.0, 0.0, 1.0};
   for (std::uint32_t p = threadIdx.x; p < blocks; p += blockDim.x) {
 #pragma unroll
@@ -130,7 +131,7 @@ __device__ __forceinline__ std::uint32_t decide(SolveDesc& d, std::uint32_t mode
   }
   // A failed check ends the solve: the sums may lack a block's, and every
   // further iteration could wait as long again.
-  if (__ldcg(&d.check_status) != 0u) proceed = 0;
+  if (failed != 0u) proceed = 0;
   d.proceed = proceed;
   return proceed;
 }

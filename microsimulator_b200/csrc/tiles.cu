@@ -108,14 +108,18 @@ __device__ __forceinline__ bool entries_there(std::uint32_t barrier, std::uint32
 }
 
 template <int Tag, int PerSm>
-__global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* desc, int fixed_mode) {
+__global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* desc, int fixed_mode,
+                                                                    std::uint32_t wait_polls) {
   const SolveDesc& d = *desc;
   const std::uint32_t mode = fixed_mode >= 0 ? std::uint32_t(fixed_mode) : d.mode;
   if (fixed_mode < 0 && mode == 1 && d.proceed == 0u) return;  // an unrolled pair after convergence
   // A local copy: the descriptor may change under the stores below, for all
   // the compiler knows.
   const TileArrays t = d.tiles;
-  const std::uint32_t bodies = t.bodies;
+  // Of the tiled system: filling the descriptor for another forgets the tiles.
+  // (Two blocks an SM leave no register over: this count among TileArrays, or
+  // the polls in a variable, took a pass of 4.15 M rows from 84 to 96 us.)
+  const std::uint32_t bodies = d.body_count;
   const bool project = mode == 1;
   const float alpha = d.step;
   const float dt = d.dt;
@@ -188,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
     for (std::uint32_t g = threadIdx.x + kGuests * kThreads; g < now.guests; g += kThreads) {
       multiplier[now.rows + g] = projected(t.iterate[t.guests[now.g0 + g]]);
     }
-    const bool there = entries_there(barrier, phase, d.wait_polls);
+    const bool there = entries_there(barrier, phase, wait_polls);
     // The multipliers of the tile's rows, projected; a constraint row's
     // second side adds nothing.
     for (std::uint32_t j = threadIdx.x; j < now.rows; j += kThreads) {
@@ -560,7 +564,7 @@ int tile_blocks_per_sm(std::uint64_t slots, std::uint64_t rows, std::uint64_t lo
 }
 
 template <int Tag>
-static void (*tile_pass(int per_sm))(SolveDesc*, int) {
+static void (*tile_pass(int per_sm))(SolveDesc*, int, std::uint32_t) {
   const auto kernel = per_sm >= 4   ? tile_pass_kernel<Tag, 4>
                       : per_sm == 3 ? tile_pass_kernel<Tag, 3>
                       : per_sm == 2 ? tile_pass_kernel<Tag, 2>
@@ -578,10 +582,11 @@ int boundary_pass_blocks() {
   return std::min(sm_count() * std::max(1, active), kMaxPassBlocks / 2);
 }
 
-void launch_tile_iteration(SolveDesc* desc, int per_sm, cudaEvent_t between, cudaStream_t stream) {
+void launch_tile_iteration(SolveDesc* desc, int per_sm, std::uint32_t wait_polls, cudaEvent_t between,
+                           cudaStream_t stream) {
   const int blocks = tile_pass_blocks(per_sm);
   const std::uint32_t bytes = tile_pass_bytes(per_sm);
-  tile_pass<1>(per_sm)<<<blocks, kThreads, bytes, stream>>>(desc, 1);
+  tile_pass<1>(per_sm)<<<blocks, kThreads, bytes, stream>>>(desc, 1, wait_polls);
   if (between != nullptr) cudaEventRecord(between, stream);
   boundary_pass_kernel<1><<<boundary_pass_blocks(), kThreads, 0, stream>>>(desc, 1, 0, blocks);
   count_launch(2);

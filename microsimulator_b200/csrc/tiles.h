@@ -41,7 +41,6 @@ struct TileArrays {
   float* first;                    // boundary rows' side terms
   float* second;
   const std::uint32_t* boundary;   // the boundary rows
-  std::uint32_t bodies;
   std::uint32_t tiles;
   std::uint32_t boundary_count;
   std::uint32_t max_slots;         // of any tile
@@ -99,8 +98,8 @@ std::uint64_t tile_shared_bytes(std::uint64_t slots, std::uint64_t rows, std::ui
 int tile_blocks_per_sm(std::uint64_t slots, std::uint64_t rows, std::uint64_t locals);
 
 // The two passes of an iteration (see tiles.cu) for a graph: kernels taking
-// (SolveDesc*, int fixed_mode) and (SolveDesc*, int fixed_mode, int
-// set_condition, int tile_blocks), their grids, and the first one's dynamic
+// (SolveDesc*, int fixed_mode, uint32_t wait_polls) and (SolveDesc*, int
+// fixed_mode, int set_condition, int tile_blocks), their grids, and the first one's dynamic
 // shared memory, for `per_sm` blocks an SM.
 void* tile_pass_function(int per_sm);
 void* boundary_pass_function();
@@ -110,7 +109,8 @@ int boundary_pass_blocks();
 
 // One more projected iteration of the last system, solved by tiles, for
 // timing (launch_iteration's counterpart).
-void launch_tile_iteration(SolveDesc* desc, int per_sm, cudaEvent_t between, cudaStream_t stream);
+void launch_tile_iteration(SolveDesc* desc, int per_sm, std::uint32_t wait_polls, cudaEvent_t between,
+                           cudaStream_t stream);
 
 // The multipliers and gaps a tiled solve reached, by row.
 void launch_unpack_tiles(SolveDesc* desc, int blocks, cudaStream_t stream);
