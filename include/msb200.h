@@ -437,6 +437,21 @@ typedef struct msb_solve_record {
 int msb_last_step_solves(const msb_context* context, msb_solve_record* records, uint32_t capacity,
                          uint32_t* count);
 
+/* Where a solve ran. */
+enum msb_solve_form {
+  MSB_FORM_SLOTS = 0,   /* the graph of two passes by slot */
+  MSB_FORM_FUSED = 1,   /* the fused kernel (msb_set_relaxation 2) */
+  MSB_FORM_ONE_CTA = 2, /* resident in one CTA, in a cluster, over the grid */
+  MSB_FORM_CLUSTER = 3,
+  MSB_FORM_GRID = 4,
+  MSB_FORM_CLUSTERS = 5, /* a batch: clusters of CTAs; gangs of CTAs; both */
+  MSB_FORM_GANGS = 6,
+  MSB_FORM_GANGS_AND_CLUSTERS = 7,
+  MSB_FORM_TILES = 16 /* + blocks an SM: tiles, after a start by slot */
+};
+/* The form of each solve of msb_last_step_solves. */
+int msb_last_step_solve_forms(const msb_context* context, uint32_t* forms, uint32_t capacity, uint32_t* count);
+
 /* The overlap re-checks of the last msb_advance_contact_dynamics(_device)
  * or batch call by how their pair candidates were found: a full contact
  * search, the substep's kept candidates (no cell moved further than their

@@ -180,6 +180,18 @@ class B200Backend:
         self._check(status)
         return out[: count.value].copy()
 
+    SOLVE_FORMS = {0: "slots", 1: "fused", 2: "one cta", 3: "cluster", 4: "grid", 5: "clusters", 6: "gangs",
+                   7: "gangs and clusters", 17: "tiles 1", 18: "tiles 2", 19: "tiles 3", 20: "tiles 4"}
+
+    def last_step_solve_forms(self) -> list[str]:
+        """Where each of ``last_step_solves`` ran (tiles: and how many blocks
+        shared an SM)."""
+        count = ctypes.c_uint32(0)
+        out = np.zeros(max(1, len(self.last_step_solves())), dtype=np.uint32)
+        self._check(self._lib.msb_last_step_solve_forms(self._handle, c_void_p(abi.ptr(out)), len(out),
+                                                        ctypes.byref(count)))
+        return [self.SOLVE_FORMS[int(form)] for form in out[: count.value]]
+
     def last_step_searches(self) -> dict:
         """The last step's overlap re-checks by how their candidates were
         found: a full search, the substep's kept candidates, or the kept

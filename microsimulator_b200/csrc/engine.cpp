@@ -569,6 +569,9 @@ struct msb_context {
   msb::DBuf<float2> tile_constants, tile_iterate;
   msb::DBuf<float> tile_first, tile_second;
   std::array<std::unique_ptr<msb::SolveGraph>, 5> tile_graphs;  // by blocks an SM
+  int tiles_built = 0;         // the tiles are those of the rows at hand, this many blocks an SM
+  bool tiles_refused = false;  // a system of this step did not suit tiles
+  std::uint32_t step_iterations = 0;  // of this step's last solve
   // A batch's schedule: jobs, gangs, each CTA's list.
   msb::DBuf<msb::ResidentJob> batch_jobs;
   msb::DBuf<msb::ResidentGang> batch_gangs;
@@ -629,6 +632,7 @@ struct msb_context {
   bool nvtx_open = false;  // an NVTX range of the current phase is open
   std::vector<int> phase_marks;
   std::vector<msb_solve_record> solve_log;  // the solves of the last step, in order
+  std::vector<std::uint32_t> form_log;      // and where each ran (msb_solve_form)
   std::array<double, 8> phase_ms{};
 
   // outputs staging for host calls
@@ -1310,9 +1314,10 @@ void fill_problem(Ctx& c, SolveDesc& d, std::uint32_t row_count, float dt, const
 }
 
 void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_response& growth, float tolerance,
-               std::uint32_t max_iterations, bool with_state = false) {
+               std::uint32_t max_iterations, bool with_state = false, bool resume = false) {
   SolveDesc& d = *c.host_desc;
   fill_problem(c, d, row_count, dt, growth, tolerance, max_iterations);
+  d.resume = resume ? 1u : 0u;
   c.desc_current = true;
   c.last_tiled = 0;
   if (with_state) {
@@ -1342,6 +1347,7 @@ void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_
 
 void build_system_incidence(Ctx& c, std::uint32_t row_count) {
   const std::size_t entries = 2ull * std::max<std::uint32_t>(row_count, 1);
+  c.tiles_built = 0;
   c.inc_offsets.ensure(c.n + 1ull);
   c.inc_a.ensure(entries);
   c.inc_b.ensure(entries);
@@ -1366,8 +1372,6 @@ void build_row_keys(Ctx& c, RowStore& store) {
               c.temp.p, c.stream);
 }
 
-// Runs the solve graph on c.rows (multipliers in place).  Requires the
-// incidence of c.rows and the bodies.
 SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growth, std::uint32_t max_iterations);
 
 // A resident solve's arrays; over several CTAs with words in global memory
@@ -1391,6 +1395,11 @@ ResidentArrays resident_arrays(Ctx& c, bool grid) {
           ordered ? c.spatial_offsets.p : nullptr};
 }
 
+void log_solve(Ctx& c, const msb_solve_record& record, std::uint32_t form) {
+  c.solve_log.push_back(record);
+  c.form_log.push_back(form);
+}
+
 // The solve with the system in shared memory, in one launch; c.host_desc
 // holds its report.  False, with nothing done, when a share does not fit.
 bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_response& growth, float tolerance,
@@ -1406,10 +1415,10 @@ bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_r
   return c.host_desc->gang.misfit == 0;
 }
 
-// Renumbers c.rows by tiles of c.spatial_order into `out`; returns how many
-// blocks of the tile pass share an SM, 0 when a body or a tile has too many
-// rows.
-int build_tiles(Ctx& c, TileArrays& out) {
+// Renumbers c.rows by tiles of c.spatial_order into `out`, with the iterate
+// (`resume`) or the multipliers of c.rows; returns how many blocks of the tile
+// pass share an SM, 0 when a body or a tile has too many rows.
+int build_tiles(Ctx& c, bool resume, TileArrays& out) {
   const std::uint32_t n = c.n, rows = c.rows.count;
   const std::uint32_t tiles = (n + kTileBodies - 1) / kTileBodies;
   const std::uint64_t slots = tile_slot_capacity(2ull * rows, tiles);
@@ -1451,7 +1460,7 @@ int build_tiles(Ctx& c, TileArrays& out) {
                         c.tile_report.p};
   launch_tile_build(n, rows, c.spatial_order.p, c.rows.slots.p, incidence_arrays(c),
                     {c.body_a.p, c.body_b.p, c.drift_a.p, c.drift_b.p}, c.rows.keyed_offsets.p, c.rows.keyed_rows.p,
-                    c.rows.multipliers.p, build, c.temp.p, c.stream);
+                    resume ? nullptr : c.rows.multipliers.p, c.rows.iterate.p, build, c.temp.p, c.stream);
   check(cudaMemcpyAsync(&c.host_scalars[kScalarCount + 6], c.tile_report.p, 16, cudaMemcpyDeviceToHost, c.stream),
         "read");
   const std::uint32_t boundary = read_u32(c, c.tile_positions.p + rows);
@@ -1466,10 +1475,97 @@ int build_tiles(Ctx& c, TileArrays& out) {
   return tile_blocks_per_sm(max_slots, max_rows, max_locals);
 }
 
-// Systems too large to be resident take the tiled passes where the substep
-// has a spatial order (per iteration against the two passes by slot: 1M
-// capsules in tracks, 4.15M rows, 97 against 187 us; 1M at random, 2.65M
-// rows, 80 against 104; 300k at random, 782,000 rows, 31 against 37).
+// Systems too large to be resident run by slot or by tiles.  Measured on B200,
+// us per iteration by slot and by tiles:
+//   1M capsules in tracks, 4.15M rows    194 and 98
+//   1M at random, 2.65M rows             112 and 84
+//   1M at random, 2.17M rows              92 and 79
+//   1M at random, 1.58M rows              73 and 72
+//   1M at random, 0.96M rows              52 and 56
+//   300k at random, 782,000 rows          46 and 37
+// Renumbering a system takes 0.5 (2.65M rows) to 0.7 ms (4.15M), the gain of
+// 19 and 7 iterations, so a step of 1M sparse capsules (0.94M or 1.55M rows)
+// took 18.3 and 38.9 ms by tiles where it takes 16.5 and 37.0 by slot.  Hence:
+//   - only systems of two rows a body and more take tiles;
+//   - with one block an SM (a crowded tile) three rows a body: at 2.65 an
+//     iteration is 118 us against 112 by slot, at 4.15 138 against 194;
+//   - a solve starts by slot and goes on by tiles, from the iterate it has
+//     reached, when it needs more than kTiledAfter iterations, so that a short
+//     one costs what it did; the solves that follow a long one in the same
+//     step (kLongSolve) are likely to be long and start by tiles;
+//   - a second solve of the same rows (a probe's) finds the tiles in place.
+constexpr std::uint32_t kTiledAfter = 8;
+constexpr std::uint32_t kLongSolve = 64;
+bool tiles_pay(std::uint64_t rows, std::uint64_t bodies) { return rows >= 2 * bodies; }
+
+// The tiles of c.rows in `c.host_desc`, starting from c.rows.iterate with
+// `resume` and from c.rows.multipliers otherwise.  False when the system runs
+// better by slot, or not at all by tiles; the rest of the step then goes by
+// slot.
+bool use_tiles(Ctx& c, bool resume) {
+  if (c.tiles_refused) return false;
+  if (c.tiles_built > 0 && !resume) return true;  // the last solve's: its multipliers are these
+  c.tiles_built = build_tiles(c, resume, c.host_desc->tiles);
+  if (c.tiles_built == 1 && c.rows.count < 3ull * c.n) c.tiles_built = 0;
+  c.tiles_refused = c.tiles_built == 0;
+  return c.tiles_built > 0;
+}
+
+// The final multipliers and gaps of a solve, and their response (the passes
+// of a solve write only the rows' side terms).
+void finish_solve(Ctx& c) {
+  if (c.last_tiled > 0) {
+    launch_unpack_tiles(c.desc, c.last_blocks, c.stream);
+  } else {
+    launch_unpack_iterate(c.desc, c.last_blocks, c.stream);
+  }
+  launch_evaluate(c.desc, c.last_blocks, false, c.stream);
+}
+
+// One launch of the solve graph (over tiles: c.host_desc->tiles) or of the
+// fused kernel on c.rows, and its report in c.host_desc; with `resume` it goes
+// on with the solve that the descriptor holds, and without `finish` the
+// solution stays in the iterate.
+enum class SolveForm { kSlots, kTiles, kFused };
+void run_solve(Ctx& c, SolveForm form, bool resume, bool finish, float dt, const msb_growth_load_response& growth,
+               float tolerance, std::uint32_t max_iterations) {
+  const std::uint32_t rows = c.rows.count;
+  const std::uint32_t before = resume ? c.host_desc->iterations : 0;
+  const bool tiled = form == SolveForm::kTiles;
+  if (form == SolveForm::kFused) {
+    // One cooperative launch runs the whole solve (relax_kernel).
+    const std::uint32_t wanted = (std::max(rows, c.n) + kSolveThreads - 1) / kSolveThreads;
+    const int blocks = std::max(1, std::min({int(wanted), c.relax_blocks, 1184}));
+    c.last_blocks = blocks;
+    fill_desc(c, rows, dt, growth, tolerance, max_iterations, true);
+    check(cudaError_t(launch_relax(*c.host_desc, c.desc, blocks, c.stream)), "solve launch");
+  } else {
+    auto& graph = graph_for(c, std::max(rows, c.n));
+    c.last_blocks = graph.blocks();
+    fill_desc(c, rows, dt, growth, tolerance, max_iterations, false, resume);
+    auto& made = c.tile_graphs[tiled ? c.tiles_built : 0];
+    if (tiled && !made) {
+      auto fresh = std::make_unique<SolveGraph>();
+      check(cudaError_t(fresh->create(c.desc, kMaxPassBlocks, c.stream, c.tiles_built, c.wait_polls)), "solve graph");
+      made = std::move(fresh);
+    }
+    check(cudaError_t((tiled ? *made : graph).launch(c.stream)), "solve launch");
+  }
+  c.last_tiled = tiled ? c.tiles_built : 0;
+  if (finish) finish_solve(c);
+  check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
+  sync(c);
+  const SolveDesc& d = *c.host_desc;
+  if (d.barrier_abort != 0) throw DeviceCheckError("a grid barrier of the relaxation ran out of time");
+  if (d.check_status != 0) {
+    throw DeviceCheckError("an index check or a bounded wait of the relaxation failed at iteration " +
+                           std::to_string(d.iterations));
+  }
+  if (form != SolveForm::kFused) count_launch(SolveGraph::loop_launches(d.iterations - before));
+}
+
+// The solve of c.rows (multipliers in place), with its response in
+// c.resp_a/b.  Requires the incidence of c.rows and the bodies.
 SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, float tolerance,
                    std::uint32_t max_iterations) {
   if (c.colonies > 0) return solve_batch(c, dt, growth, max_iterations);
@@ -1482,57 +1578,35 @@ SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, flo
     return {};
   }
   c.partials.ensure(5ull * kMaxPassBlocks);
+  bool solved = false;
+  std::uint32_t form = 0;
   if (c.relaxation == 0) {
     if (!c.resident_limits) c.resident_limits = resident_limits();
     const ResidentPlan plan = resident_plan(*c.resident_limits, rows, c.n);
-    if (plan.ctas > 0 && solve_resident(c, plan, dt, growth, tolerance, max_iterations)) {
-      const SolveDesc& d = *c.host_desc;
-      c.solve_log.push_back({rows, d.iterations, d.status, d.residual});
-      if (d.status == 3) throw std::invalid_argument("contact system has no positive diagonal");
-      return {d.status, d.iterations, d.residual};
+    solved = plan.ctas > 0 && solve_resident(c, plan, dt, growth, tolerance, max_iterations);
+    form = plan.grid ? MSB_FORM_GRID : plan.ctas > 1 ? MSB_FORM_CLUSTER : MSB_FORM_ONE_CTA;
+  }
+  if (!solved) {
+    const SolveForm plain = use_fused_relaxation(c, std::max(rows, c.n)) ? SolveForm::kFused : SolveForm::kSlots;
+    const bool tileable =
+        plain == SolveForm::kSlots && c.relaxation == 0 && c.spatial_valid && tiles_pay(rows, c.n) && !c.tiles_refused;
+    if (tileable && c.step_iterations >= kLongSolve && use_tiles(c, false)) {
+      run_solve(c, SolveForm::kTiles, false, true, dt, growth, tolerance, max_iterations);
+    } else {
+      const bool first = tileable && !c.tiles_refused && max_iterations > kTiledAfter;
+      run_solve(c, plain, false, !first, dt, growth, tolerance, first ? kTiledAfter : max_iterations);
+      if (first && c.host_desc->status == MSB_SOLVE_ITERATION_LIMIT) {
+        run_solve(c, use_tiles(c, true) ? SolveForm::kTiles : plain, true, true, dt, growth, tolerance, max_iterations);
+      } else if (first) {
+        finish_solve(c);
+      }
     }
+    form = plain == SolveForm::kFused ? MSB_FORM_FUSED
+                                      : (c.last_tiled > 0 ? MSB_FORM_TILES + std::uint32_t(c.last_tiled) : MSB_FORM_SLOTS);
   }
-  const bool fused = use_fused_relaxation(c, std::max(rows, c.n));
-  int tiled = 0;
-  if (fused) {
-    // One cooperative launch runs the whole solve (relax_kernel).
-    const std::uint32_t wanted = (std::max(rows, c.n) + kSolveThreads - 1) / kSolveThreads;
-    const int blocks = std::max(1, std::min({int(wanted), c.relax_blocks, 1184}));
-    c.last_blocks = blocks;
-    fill_desc(c, rows, dt, growth, tolerance, max_iterations, true);
-    check(cudaError_t(launch_relax(*c.host_desc, c.desc, blocks, c.stream)), "solve launch");
-  } else {
-    auto& graph = graph_for(c, std::max(rows, c.n));
-    c.last_blocks = graph.blocks();
-    if (c.relaxation == 0 && c.spatial_valid) tiled = build_tiles(c, c.host_desc->tiles);
-    fill_desc(c, rows, dt, growth, tolerance, max_iterations);
-    auto& made = c.tile_graphs[tiled];
-    if (tiled > 0 && !made) {
-      auto fresh = std::make_unique<SolveGraph>();
-      check(cudaError_t(fresh->create(c.desc, kMaxPassBlocks, c.stream, tiled, c.wait_polls)), "solve graph");
-      made = std::move(fresh);
-    }
-    check(cudaError_t((tiled > 0 ? *made : graph).launch(c.stream)), "solve launch");
-  }
-  // The final multipliers and gaps, and their response (the passes of a
-  // solve write only the rows' side terms).
-  c.last_tiled = tiled;
-  if (tiled > 0) {
-    launch_unpack_tiles(c.desc, c.last_blocks, c.stream);
-  } else {
-    launch_unpack_iterate(c.desc, c.last_blocks, c.stream);
-  }
-  launch_evaluate(c.desc, c.last_blocks, false, c.stream);
-  check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
-  sync(c);
   const SolveDesc& d = *c.host_desc;
-  if (d.barrier_abort != 0) throw DeviceCheckError("a grid barrier of the relaxation ran out of time");
-  if (d.check_status != 0) {
-    throw DeviceCheckError("an index check or a bounded wait of the relaxation failed at iteration " +
-                           std::to_string(d.iterations));
-  }
-  if (!fused) count_launch(SolveGraph::loop_launches(d.iterations));
-  c.solve_log.push_back({rows, d.iterations, d.status, d.residual});
+  c.step_iterations = d.iterations;
+  log_solve(c, {rows, d.iterations, d.status, d.residual}, form);
   if (d.status == 3) throw std::invalid_argument("contact system has no positive diagonal");
   return {d.status, d.iterations, d.residual};
 }
@@ -1740,6 +1814,7 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
   // The colonies that gangs of CTAs hold in shared memory, then the others.
   if (!c.resident_limits) c.resident_limits = resident_limits();
   bool all = false;
+  std::uint32_t form = MSB_FORM_CLUSTERS;
   std::vector<std::uint32_t> left = c.host_colony_active;  // the colonies still to solve
   if (c.relaxation == 0 && c.resident_limits->grid > 0 && k <= kResidentColonies && c.batch_tuned) {
     const auto rest = solve_batch_resident(c, c.host_colony_active, row_counts, dt, growth, max_iterations);
@@ -1747,6 +1822,7 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
     std::fill(left.begin(), left.end(), 0u);
     for (const std::uint32_t i : rest) left[i] = 1u;
     active = std::uint32_t(rest.size());
+    form = all ? MSB_FORM_GANGS : MSB_FORM_GANGS_AND_CLUSTERS;
     c.colony_rest.ensure(k);
     if (!all) {
       check(cudaMemcpyAsync(c.colony_rest.p, left.data(), k * 4ull, cudaMemcpyHostToDevice, c.stream), "copy colonies");
@@ -1809,7 +1885,7 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
   }
   out.status = worst == 2 ? MSB_SOLVE_BREAKDOWN : (worst == 1 ? MSB_SOLVE_ITERATION_LIMIT : MSB_SOLVE_CONVERGED);
   out.residual = residual;
-  c.solve_log.push_back({rows, out.iterations, out.status, residual});
+  log_solve(c, {rows, out.iterations, out.status, residual}, form);
   return out;
 }
 
@@ -2003,15 +2079,15 @@ Attempt advance_substep(Ctx& c, float dt, const msb_contact_dynamics_parameters&
   const std::uint32_t found = find_touches(c, c.state, cp, wp, p.candidate_margin, c.touches,
                                            p.candidate_margin + (c.colonies > 0 ? kBatchRecheckReach : kRecheckReach), true);
   mark(c, kPhaseRows);
-  // Systems that take the resident solve's grid form, and those too large
-  // for it, get their cells' spatial order from the grid of the search just
+  // Systems that take the resident solve's grid form, and those that may take
+  // tiles, get their cells' spatial order from the grid of the search just
   // made.
   c.spatial_valid = false;
   if (c.relaxation == 0 && found > 0 && n > 1) {
     if (!c.resident_limits) c.resident_limits = resident_limits();
     if (c.colonies > 0 ? c.resident_limits->grid > 0 && c.colonies <= kResidentColonies
                        : resident_plan(*c.resident_limits, found, n).grid ||
-                             resident_plan(*c.resident_limits, found, n).ctas == 0) {
+                             (resident_plan(*c.resident_limits, found, n).ctas == 0 && tiles_pay(found, n))) {
       c.spatial_keys.ensure(n);
       c.spatial_order.ensure(n);
       c.temp.ensure(sort_temp_words(n) + 64);
@@ -2151,6 +2227,8 @@ StepOutcome advance(Ctx& c, float dt, const msb_contact_dynamics_parameters& p, 
     c.memory.count = 0;
   }
 
+  c.step_iterations = 0;
+  c.tiles_refused = false;
   reset_scalars(c);
   launch_growth_bound(n, c.state.view(), c.growth.p, dt, c.scalars.p + kGrowthBits, c.stream);
   read_scalars(c);
@@ -2488,6 +2566,14 @@ int msb_last_step_solves(const msb_context* context, msb_solve_record* records, 
   const auto& log = context->solve_log;
   *count = std::uint32_t(log.size());
   for (std::size_t k = 0; k < log.size() && k < capacity; ++k) records[k] = log[k];
+  return log.size() > capacity ? MSB_ERR_CAPACITY : MSB_OK;
+}
+
+int msb_last_step_solve_forms(const msb_context* context, uint32_t* forms, uint32_t capacity, uint32_t* count) {
+  if (context == nullptr || count == nullptr || (capacity > 0 && forms == nullptr)) return MSB_ERR_INVALID_ARGUMENT;
+  const auto& log = context->form_log;
+  *count = std::uint32_t(log.size());
+  for (std::size_t k = 0; k < log.size() && k < capacity; ++k) forms[k] = log[k];
   return log.size() > capacity ? MSB_ERR_CAPACITY : MSB_OK;
 }
 
@@ -3037,6 +3123,7 @@ static int advance_entry(msb_context* context, msb_cell_arrays* cells, const msb
     auto& c = *context;
     c.phase_marks.clear();
     c.solve_log.clear();
+    c.form_log.clear();
     std::fill(std::begin(c.searches), std::end(c.searches), 0u);
     mark(c, kPhaseLoad);
     load_cells(c, *cells, device_pointers);
@@ -3143,6 +3230,7 @@ int msb_advance_contact_dynamics_batch(msb_context* context, msb_cell_arrays* ce
     c.box_scale = c.batch_box_scale;
     c.phase_marks.clear();
     c.solve_log.clear();
+    c.form_log.clear();
     std::fill(std::begin(c.searches), std::end(c.searches), 0u);
     mark(c, kPhaseLoad);
     load_cells(c, *cells, device_pointers != 0);

@@ -389,6 +389,7 @@ __global__ void __launch_bounds__(kSolveThreads, MSB_RELAX_MIN_BLOCKS)
 
 __global__ void __launch_bounds__(kSolveThreads) bound_kernel(SolveDesc* desc) {
   SolveDesc& d = *desc;
+  if (d.resume != 0u) return;
   float bound = 0.0f;
   for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < d.row_count; i += gridDim.x * blockDim.x) {
     d.iterate[i] = make_float2(d.multipliers[i], 0.0f);  // the solve's starting multipliers
@@ -415,7 +416,9 @@ __global__ void unpack_iterate_kernel(const SolveDesc* desc) {
 }
 
 __global__ void solve_reset_kernel(SolveDesc* desc) {
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && desc->resume != 0u) {
+    desc->proceed = 1;  // the first pair of passes is an iteration
+  } else if (threadIdx.x == 0) {
     desc->mode = 0;
     desc->ticket = 0;
     desc->iterations = 0;

@@ -99,6 +99,7 @@ struct SolveDesc {
   float tolerance;
   std::uint32_t max_iterations;
   std::uint32_t has_drift;  // 0: every drift is zero and the drift arrays are not read
+  std::uint32_t resume;      // the graph goes on from the state below instead of resetting it
   std::uint32_t wait_polls;  // a 32nd of the polls after which a resident solve's CTAs are late
   TileArrays tiles;         // of a tiled solve
   // solver state

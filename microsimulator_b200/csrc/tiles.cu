@@ -404,7 +404,8 @@ __global__ void __launch_bounds__(kThreads) tile_rows_kernel(std::uint32_t n, st
                                                              const float2* __restrict__ constants,
                                                              const std::uint32_t* __restrict__ keyed_offsets,
                                                              const std::uint32_t* __restrict__ keyed_rows,
-                                                             const float* __restrict__ multipliers, TileBuild out) {
+                                                             const float* __restrict__ multipliers,
+                                                             const float2* __restrict__ iterate, TileBuild out) {
   __shared__ std::uint32_t warp_sums[2][kThreads / 32];
   const std::uint32_t tile = blockIdx.x, place = tile * kTileBodies + threadIdx.x;
   const std::uint32_t r0 = out.row_start[tile * kTileBodies];
@@ -446,7 +447,7 @@ __global__ void __launch_bounds__(kThreads) tile_rows_kernel(std::uint32_t n, st
     out.row_of[at] = row;
     out.new_of[row] = at;
     out.constants[at] = make_float2(c.x, boundary ? -c.y : c.y);
-    out.iterate[at] = make_float2(multipliers[row], 0.0f);
+    out.iterate[at] = multipliers != nullptr ? make_float2(multipliers[row], 0.0f) : iterate[row];
     out.flags[at] = boundary ? 1u : 0u;
   }
   if (threadIdx.x == 0) {
@@ -527,8 +528,8 @@ int sm_count() {
 
 void launch_tile_build(std::uint32_t n, std::uint32_t rows, const std::uint32_t* spatial_order, const uint2* slots,
                        const IncidenceArrays& incidence, const BodyArrays& bodies, const std::uint32_t* keyed_offsets,
-                       const std::uint32_t* keyed_rows, const float* multipliers, const TileBuild& out,
-                       std::uint32_t* temp, cudaStream_t stream) {
+                       const std::uint32_t* keyed_rows, const float* multipliers, const float2* iterate,
+                       const TileBuild& out, std::uint32_t* temp, cudaStream_t stream) {
   const std::uint32_t tiles = (n + kTileBodies - 1) / kTileBodies;
   cudaMemsetAsync(out.report, 0, 4 * sizeof(std::uint32_t), stream);
   tile_order_kernel<<<tiles, kThreads, 0, stream>>>(n, spatial_order, incidence.offsets, keyed_offsets, bodies, out);
@@ -536,7 +537,7 @@ void launch_tile_build(std::uint32_t n, std::uint32_t rows, const std::uint32_t*
   exclusive_scan(out.tile_slots, out.slot_base, tiles + 1, temp, stream);
   exclusive_scan(out.row_counts, out.row_start, n + 1ull, temp, stream);
   tile_rows_kernel<<<tiles, kThreads, 0, stream>>>(n, rows, slots, incidence.constants, keyed_offsets, keyed_rows,
-                                                   multipliers, out);
+                                                   multipliers, iterate, out);
   count_launch();
   tile_guests_kernel<<<grid_for(n + 1ull, 256), 256, 0, stream>>>(n, incidence, out);
   count_launch();

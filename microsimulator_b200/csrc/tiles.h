@@ -84,11 +84,13 @@ inline std::uint64_t tile_slot_capacity(std::uint64_t entries, std::uint64_t til
 }
 
 // Renumbers the system of `rows` rows over `n` bodies taken along
-// `spatial_order`; `temp`: scan_temp_words(max(n, rows) + 1).  The boundary
+// `spatial_order`, with the rows' multipliers (gaps zero) or, where that is
+// null, their iterate; `temp`: scan_temp_words(max(n, rows) + 1).  The boundary
 // rows' number is then at positions[rows].
 void launch_tile_build(std::uint32_t n, std::uint32_t rows, const std::uint32_t* spatial_order, const uint2* slots,
                        const IncidenceArrays& incidence, const BodyArrays& bodies, const std::uint32_t* keyed_offsets,
-                       const std::uint32_t* keyed_rows, const float* multipliers, const TileBuild& out,
+                       const std::uint32_t* keyed_rows, const float* multipliers, const float2* iterate,
+                       const TileBuild& out,
                        std::uint32_t* temp, cudaStream_t stream);
 
 // Shared memory of a tile of at most `slots` slots, `rows` rows and `locals`

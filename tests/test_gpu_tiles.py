@@ -66,10 +66,34 @@ def test_a_body_of_many_rows(forms, cells):
     step_both(forms, long)
 
 
+def forms_of(backend, world, dt=0.002, tolerance=5e-4):
+    backend.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+    backend.advance_contact_dynamics(world.copy(), None, dt, ContactDynamicsParameters(overlap_tolerance=tolerance))
+    return list(zip(backend.last_step_solve_forms(), backend.last_step_solves()["iterations"].tolist()))
+
+
+def test_solves_that_gain_nothing_by_tiles_go_by_slot(forms):
+    """Sparse colonies (under two rows a body) and solves of up to 8
+    iterations; after a long solve the next starts by tiles."""
+    sparse = forms_of(forms, workloads.jammed(330_000, area_fraction=0.3, seed=2))
+    assert max(its for _, its in sparse) > 8
+    assert {form for form, _ in sparse} == {"slots"}
+    dense = workloads.jammed(170_001, seed=6)
+    seen = set()
+    for dt, tolerance in ((0.02, 5e-4), (0.002, 0.4)):
+        log = forms_of(forms, dense, dt, tolerance)
+        for k, (form, its) in enumerate(log):
+            tiled = its > 8 or (k > 0 and log[k - 1][1] >= 64)
+            assert form.startswith("tiles") == tiled, (k, log)
+            seen.add(tiled)
+    assert seen == {True, False}
+
+
 def test_a_copy_that_is_late_ends_the_solve(forms):
     """With no polls allowed the tiles' copies count as late: the solve ends
-    with its first pass (not after max_iterations of them, on sums that the
-    blocks never wrote), its copies drained, and the next call is sound."""
+    with its first pass by tiles, after 8 iterations by slot (not after
+    max_iterations of them, on sums that the blocks never wrote), its copies
+    drained, and the next call is sound."""
     world = workloads.jammed(170_001, seed=6)
     p = ContactDynamicsParameters(overlap_tolerance=5e-4)
     forms.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
@@ -77,7 +101,7 @@ def test_a_copy_that_is_late_ends_the_solve(forms):
     forms.advance_contact_dynamics(expected, None, 0.002, p)
     forms.set_wait_limit(0)
     try:
-        with pytest.raises(abi.NativeError, match="wait of the relaxation failed at iteration 0$"):
+        with pytest.raises(abi.NativeError, match="wait of the relaxation failed at iteration 9$"):
             forms.advance_contact_dynamics(world.copy(), None, 0.002, p)
     finally:
         forms.set_wait_limit()
