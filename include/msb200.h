@@ -620,10 +620,12 @@ int msb_set_flow_field(msb_context* context, const msb_flow_field* field);
  * Constraints (walls) are not taken.  Warm-start flags other than carry are
  * rejected.
  *
- * The first call on a context tunes the launch shape of the batched solve
- * (CTAs per cluster, threads per CTA, register form) and the box scale of the contact search
- * by timing each candidate on that call's system; msb_tune_batch asks for a
- * new tuning at the next call and msb_batch_tuning reads the choice. */
+ * The first call on a context tunes the box scale of the contact search, and
+ * the first solve that needs it (one of more colonies than 96 that gangs of
+ * CTAs do not hold in shared memory) the launch shape of the batched solve:
+ * CTAs per cluster, threads per CTA, register form.  Each is timed on the
+ * system at hand.  msb_tune_batch asks for a new tuning of both at the next
+ * call and msb_batch_tuning reads the choice. */
 typedef struct msb_colony_parameters {
   float drag;
   float contact_stiffness;

@@ -110,6 +110,10 @@ __global__ void grid_setup_kernel(const double* __restrict__ partials, std::uint
     const double box_width = smax(v[6 + a] * 1.001 * box_scale, DBL_MIN);
     const double extent = floor((v[3 + a] - v[a]) / box_width) + 1.0;
     out.low[a] = v[a];
+    if (a < 2) {
+      const double plain = smax(v[6 + a] * 1.001, DBL_MIN);
+      out.span[a] = (floor((v[3 + a] - v[a]) / plain) + 1.0) / (1.0 / plain);
+    }
     out.inv_width[a] = 1.0 / box_width;
     if (!(extent <= limit)) {
       dense = false;

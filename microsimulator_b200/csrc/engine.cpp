@@ -596,6 +596,7 @@ struct msb_context {
   msb::BatchShape batch_shape{4, 256, false};
   int batch_clusters = 0;
   bool batch_tuned = false;
+  bool tune_asked = false;  // msb_tune_batch: tune at the next batch, needed or not
   std::vector<std::uint32_t> host_colony_active;
   float box_scale = 1.0f;        // the contact search's box scale for the current call
   float batch_box_scale = 1.0f;  // the autotuner's choice for batches
@@ -1811,12 +1812,24 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
   c.host_colony_state.resize(k);
   std::uint32_t active = 0;
   for (const std::uint32_t a : c.host_colony_active) active += a != 0u ? 1u : 0u;
+  const auto group_rows = [&] {
+    exclusive_scan(c.colony_row_counts.p, c.colony_row_offsets.p, k + 1ull, c.temp.p, c.stream);
+    if (rows > 1) radix_sort_pairs(c.sort_keys.p, c.colony_rows.p, rows, std::max(1, int(std::bit_width(k))), c.temp.p,
+                                   c.stream);
+  };
+  bool grouped = false;
+  if (c.tune_asked) {
+    group_rows();
+    grouped = true;
+    tune_batch(c, batch_desc(c, dt, growth, max_iterations));
+    c.tune_asked = false;
+  }
   // The colonies that gangs of CTAs hold in shared memory, then the others.
   if (!c.resident_limits) c.resident_limits = resident_limits();
   bool all = false;
   std::uint32_t form = MSB_FORM_CLUSTERS;
   std::vector<std::uint32_t> left = c.host_colony_active;  // the colonies still to solve
-  if (c.relaxation == 0 && c.resident_limits->grid > 0 && k <= kResidentColonies && c.batch_tuned) {
+  if (c.relaxation == 0 && c.resident_limits->grid > 0 && k <= kResidentColonies) {
     const auto rest = solve_batch_resident(c, c.host_colony_active, row_counts, dt, growth, max_iterations);
     all = rest.empty();
     std::fill(left.begin(), left.end(), 0u);
@@ -1834,11 +1847,8 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
           "copy colonies");
   }
   if (!all) {
-    exclusive_scan(c.colony_row_counts.p, c.colony_row_offsets.p, k + 1ull, c.temp.p, c.stream);
-    if (rows > 1) radix_sort_pairs(c.sort_keys.p, c.colony_rows.p, rows, std::max(1, int(std::bit_width(k))), c.temp.p,
-                                   c.stream);
+    if (!grouped) group_rows();
     msb::BatchDesc d = batch_desc(c, dt, growth, max_iterations);
-    if (!c.batch_tuned) tune_batch(c, d);
     d.active = c.colony_rest.p;
     // A solve of few colonies (a step's later refinement rounds, where most
     // colonies have settled) runs them on clusters of 16 CTAs: the largest
@@ -1851,6 +1861,7 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
     if (wide_clusters > 0) {
       run_batch(c, d, wide, std::min<int>(wide_clusters, int(active)));
     } else {
+      if (!c.batch_tuned) tune_batch(c, d);
       run_batch(c, d, c.batch_shape, c.batch_clusters);
     }
     std::vector<msb::ColonyState> states(k);
@@ -3321,6 +3332,7 @@ int msb_advance_contact_dynamics_batch(msb_context* context, msb_cell_arrays* ce
 int msb_tune_batch(msb_context* context) {
   if (context == nullptr) return MSB_ERR_INVALID_ARGUMENT;
   context->batch_tuned = false;
+  context->tune_asked = true;
   context->tune_search = true;
   return MSB_OK;
 }

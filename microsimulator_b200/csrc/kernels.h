@@ -87,6 +87,7 @@ struct GridParams {
   std::uint32_t buckets;  // buckets in use
   std::uint32_t status;
   std::uint32_t colony_stride;  // z boxes per colony of a batch (0: one system)
+  double span[2];               // x and y covered by boxes of the plain scale
 };
 
 // ---- primitives.cu

@@ -894,13 +894,13 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 // Eight bits of each of x and y, interleaved; both axes at the scale of the
-// longer one.
+// longer one (the same whatever box scale the search's tuner chose: the order
+// decides how a solve's sums are grouped).
 __global__ void spatial_keys_kernel(std::uint32_t n, const float4* __restrict__ pos_len, const GridParams* grid_ptr,
                                     const std::uint32_t* __restrict__ colony, std::uint32_t* __restrict__ keys,
                                     std::uint32_t* __restrict__ order) {
-  const double wx = grid_ptr->inv_width[0], wy = grid_ptr->inv_width[1];
   const double x0 = grid_ptr->low[0], y0 = grid_ptr->low[1];
-  const double scale = 256.0 / fmax(double(grid_ptr->dims[0]) / wx, double(grid_ptr->dims[1]) / wy);
+  const double scale = 256.0 / fmax(grid_ptr->span[0], grid_ptr->span[1]);
   for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const float4 p = pos_len[i];
     const auto cell = [&](double at) { return std::uint32_t(fmin(fmax(at * scale, 0.0), 255.0)); };

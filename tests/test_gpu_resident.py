@@ -142,6 +142,26 @@ def test_steps_in_spatial_order(forms, cells, flat):
     assert np.max(np.abs(a.geometry() - b.geometry())) <= 4 * p.overlap_tolerance
 
 
+def test_first_batch_of_a_context_runs_as_the_second(backend):
+    """Gangs from the first call on, without a launch shape tuned for clusters
+    that no colony needs: the same solves and the same bits."""
+    sizes = [40, 900, 12000]
+    batch = ColonyBatch([workloads.sweep_colony(n, seed=n) for n in sizes], np.full(3, 1.0), np.full(3, 1.0e4))
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4)
+    results = []
+    with B200Backend(0) as b:
+        for call in range(3):
+            if call == 2:
+                b.tune_batch()
+            cells = batch.concatenated()
+            _, colonies = b.advance_contact_dynamics_batch(cells, batch.counts(), batch.drag, batch.stiffness, 0.002, p)
+            results.append((cells.geometry(), colonies["iterations"]))
+            assert set(b.last_step_solve_forms()) == {"gangs"}
+    for geometry, iterations in results[1:]:
+        assert np.array_equal(geometry, results[0][0])
+        assert np.array_equal(iterations, results[0][1])
+
+
 def test_batch_by_gangs_steps_as_by_clusters(backend):
     """Colonies held by one CTA, by gangs of several and (one body touching
     more than 62 rows) by none, against the clusters' solve: the same rows,
