@@ -24,6 +24,7 @@
 #include <stdexcept>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -67,6 +68,20 @@ void check(cudaError_t err, const char* what) {
   }
 }
 
+// Device memory that the call under way can do without (a context's tiles):
+// given back when an allocation fails.  Set by guarded() for its thread.
+thread_local msb_context* reclaim_from = nullptr;
+bool reclaim();
+
+cudaError_t device_malloc(void** p, std::size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (reclaim()) e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+
 template <typename T>
 struct DBuf {
   T* p = nullptr;
@@ -96,17 +111,31 @@ struct DBuf {
     if (n > cap) {
       release();
       const std::size_t c = capacity_for(n);
-      check(cudaMalloc(&p, c * sizeof(T)), "cudaMalloc");
+      check(device_malloc(reinterpret_cast<void**>(&p), c * sizeof(T)), "cudaMalloc");
       cap = c;
     }
     return p;
+  }
+  // The same with an eighth to spare; false, and empty, when the device has no
+  // room.
+  bool try_ensure(std::size_t n) {
+    if (n <= cap) return true;
+    release();
+    const std::size_t c = n + n / 8;
+    if (cudaMalloc(&p, c * sizeof(T)) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return false;
+    }
+    cap = c;
+    return true;
   }
   // Grows to at least n elements keeping the first `keep`.
   T* grow(std::size_t n, std::size_t keep, cudaStream_t stream) {
     if (n <= cap) return p;
     const std::size_t c = capacity_for(n);
     T* q = nullptr;
-    check(cudaMalloc(&q, c * sizeof(T)), "cudaMalloc");
+    check(device_malloc(reinterpret_cast<void**>(&q), c * sizeof(T)), "cudaMalloc");
     if (keep > 0) check(cudaMemcpyAsync(q, p, keep * sizeof(T), cudaMemcpyDeviceToDevice, stream), "grow copy");
     check(cudaStreamSynchronize(stream), "grow");
     release();
@@ -562,12 +591,7 @@ struct msb_context {
   msb::DBuf<std::uint32_t> spatial_keys, spatial_order, spatial_offsets;
   bool spatial_valid = false;
   // The tiled solve's renumbered system (tiles.h) and its graph.
-  msb::DBuf<std::uint32_t> tile_order, tile_place_of, tile_slots, tile_slot_base, tile_group, tile_row_counts,
-      tile_row_start, tile_row_base, tile_guest_counts, tile_guest_start, tile_guest_base, tile_guests, tile_row_of, tile_new_of, tile_flags, tile_positions, tile_boundary, tile_report;
-  msb::DBuf<std::uint8_t> tile_degree;
-  msb::DBuf<float4> tile_a, tile_b, tile_body_a, tile_body_b;
-  msb::DBuf<float2> tile_constants, tile_iterate;
-  msb::DBuf<float> tile_first, tile_second;
+  msb::DBuf<unsigned char> tiles;
   std::array<std::unique_ptr<msb::SolveGraph>, 5> tile_graphs;  // by blocks an SM
   int tiles_built = 0;         // the tiles are those of the rows at hand, this many blocks an SM
   bool tiles_refused = false;  // a system of this step did not suit tiles
@@ -1418,61 +1442,67 @@ bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_r
 
 // Renumbers c.rows by tiles of c.spatial_order into `out`, with the iterate
 // (`resume`) or the multipliers of c.rows; returns how many blocks of the tile
-// pass share an SM, 0 when a body or a tile has too many rows.
+// pass share an SM, 0 when a body or a tile has too many rows or the device no
+// room.
 int build_tiles(Ctx& c, bool resume, TileArrays& out) {
   const std::uint32_t n = c.n, rows = c.rows.count;
   const std::uint32_t tiles = (n + kTileBodies - 1) / kTileBodies;
   const std::uint64_t slots = tile_slot_capacity(2ull * rows, tiles);
   if (slots > 0xFFFFFFFFull) return 0;
-  c.tile_order.ensure(n);
-  c.tile_place_of.ensure(n);
-  c.tile_degree.ensure(n);
-  c.tile_slots.ensure(tiles + 1ull);
-  c.tile_slot_base.ensure(tiles + 1ull);
-  c.tile_group.ensure(n / 8 + 64ull);
-  c.tile_a.ensure(slots);
-  c.tile_b.ensure(slots);
-  c.tile_body_a.ensure(n);
-  c.tile_body_b.ensure(n);
-  c.tile_row_counts.ensure(n + 1ull);
-  c.tile_row_start.ensure(n + 1ull);
-  c.tile_row_base.ensure(tiles + 1ull);
-  c.tile_row_of.ensure(rows);
-  c.tile_new_of.ensure(rows);
-  c.tile_constants.ensure(rows + 2ull);  // the copies of a tile's rows start and end on 16 bytes
-  c.tile_iterate.ensure(rows + 2ull);
-  c.tile_flags.ensure(rows + 1ull);
-  c.tile_positions.ensure(rows + 1ull);
-  c.tile_boundary.ensure(rows);
-  c.tile_first.ensure(rows);
-  c.tile_second.ensure(rows);
-  c.tile_report.ensure(4);
-  c.tile_guest_counts.ensure(n + 1ull);
-  c.tile_guest_start.ensure(n + 1ull);
-  c.tile_guest_base.ensure(tiles + 1ull);
-  c.tile_guests.ensure(rows + 1ull);
   c.temp.ensure(scan_temp_words(std::max<std::uint64_t>(n, rows) + 1) + 64);
-  const TileBuild build{c.tile_order.p,      c.tile_place_of.p,  c.tile_degree.p,    c.tile_slots.p,
-                        c.tile_slot_base.p,  c.tile_group.p,     c.tile_a.p,         c.tile_b.p,
-                        c.tile_body_a.p,     c.tile_body_b.p,    c.tile_row_counts.p, c.tile_row_start.p,
-                        c.tile_row_base.p,   c.tile_guest_counts.p, c.tile_guest_start.p, c.tile_guest_base.p,
-                        c.tile_guests.p,     c.tile_row_of.p,    c.tile_new_of.p,    c.tile_constants.p,
-                        c.tile_iterate.p,    c.tile_flags.p,     c.tile_positions.p, c.tile_boundary.p,
-                        c.tile_report.p};
+  // One allocation in 256-byte aligned parts: laid out from null for its size.
+  TileBuild build{};
+  float *first = nullptr, *second = nullptr;
+  const auto lay_out = [&](unsigned char* base) {
+    std::size_t at = 0;
+    const auto part = [&](auto*& p, std::uint64_t count) {
+      p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
+      at += (count * sizeof(*p) + 255) & ~std::size_t(255);
+    };
+    part(build.order, n);
+    part(build.place_of, n);
+    part(build.degree, n);
+    part(build.tile_slots, tiles + 1ull);
+    part(build.slot_base, tiles + 1ull);
+    part(build.group, n / 8 + 64ull);
+    part(build.a, slots);
+    part(build.b, slots);
+    part(build.body_a, n);
+    part(build.body_b, n);
+    part(build.row_counts, n + 1ull);
+    part(build.row_start, n + 1ull);
+    part(build.row_base, tiles + 1ull);
+    part(build.guest_counts, n + 1ull);
+    part(build.guest_start, n + 1ull);
+    part(build.guest_base, tiles + 1ull);
+    part(build.guests, rows + 1ull);
+    part(build.row_of, rows);
+    part(build.new_of, rows);
+    part(build.constants, rows + 2ull);  // the copies of a tile's rows start and end on 16 bytes
+    part(build.iterate, rows + 2ull);
+    part(build.flags, rows + 1ull);
+    part(build.positions, rows + 1ull);
+    part(build.boundary, rows);
+    part(build.report, 4);
+    part(first, rows);
+    part(second, rows);
+    return at;
+  };
+  if (!c.tiles.try_ensure(lay_out(nullptr))) return 0;
+  lay_out(c.tiles.p);
   launch_tile_build(n, rows, c.spatial_order.p, c.rows.slots.p, incidence_arrays(c),
                     {c.body_a.p, c.body_b.p, c.drift_a.p, c.drift_b.p}, c.rows.keyed_offsets.p, c.rows.keyed_rows.p,
                     resume ? nullptr : c.rows.multipliers.p, c.rows.iterate.p, build, c.temp.p, c.stream);
-  check(cudaMemcpyAsync(&c.host_scalars[kScalarCount + 6], c.tile_report.p, 16, cudaMemcpyDeviceToHost, c.stream),
+  check(cudaMemcpyAsync(&c.host_scalars[kScalarCount + 6], build.report, 16, cudaMemcpyDeviceToHost, c.stream),
         "read");
-  const std::uint32_t boundary = read_u32(c, c.tile_positions.p + rows);
+  const std::uint32_t boundary = read_u32(c, build.positions + rows);
   if (c.host_scalars[kScalarCount + 6] != 0u) return 0;
   const std::uint32_t max_slots = c.host_scalars[kScalarCount + 7], max_rows = c.host_scalars[kScalarCount + 8],
                       max_locals = c.host_scalars[kScalarCount + 9];
-  out = {c.tile_order.p,    c.tile_degree.p,   c.tile_slot_base.p, c.tile_group.p,     c.tile_a.p,
-         c.tile_b.p,        c.tile_body_a.p,   c.tile_body_b.p,    c.tile_row_base.p,  c.tile_guest_base.p,
-         c.tile_guests.p,   c.tile_row_of.p,   c.tile_constants.p, c.tile_iterate.p,   c.tile_first.p,
-         c.tile_second.p,   c.tile_boundary.p, tiles,              boundary,           max_slots,
-         max_rows,          max_locals};
+  out = {build.order,   build.degree,   build.slot_base, build.group,      build.a,         build.b,
+         build.body_a,  build.body_b,   build.row_base,  build.guest_base, build.guests,    build.row_of,
+         build.constants, build.iterate, first,          second,           build.boundary,  tiles,
+         boundary,      max_slots,      max_rows,        max_locals};
   return tile_blocks_per_sm(max_slots, max_rows, max_locals);
 }
 
@@ -2376,9 +2406,24 @@ void load_system(Ctx& c, const msb_contact_system& s, const float* multipliers) 
   build_system_incidence(c, rows);
 }
 
+// No allocation is made while the tiles are in use (from their build to the
+// end of the solve), but the timing hook may be about to run on them.
+bool reclaim() {
+  msb_context* const c = reclaim_from;
+  if (c == nullptr || c->tiles.p == nullptr) return false;
+  c->tiles.release();
+  c->tiles_built = 0;
+  if (c->last_tiled > 0) c->desc_current = false;
+  return true;
+}
+
 template <typename Body>
 int guarded(msb_context* c, Body&& body) {
   if (c == nullptr) return MSB_ERR_INVALID_ARGUMENT;
+  reclaim_from = c;
+  struct Leave {
+    ~Leave() { reclaim_from = nullptr; }
+  } leave;
   try {
     check(cudaSetDevice(c->device), "cudaSetDevice");
     body();

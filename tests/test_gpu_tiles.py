@@ -89,6 +89,49 @@ def test_solves_that_gain_nothing_by_tiles_go_by_slot(forms):
     assert seen == {True, False}
 
 
+def hold_all_but(free_bytes):
+    torch = pytest.importorskip("torch")
+    torch.cuda.synchronize()
+    return torch.empty(torch.cuda.mem_get_info()[0] - free_bytes, dtype=torch.uint8, device="cuda")
+
+
+def test_tiles_do_without_memory_that_others_need(backend):
+    """Where the device has no room for the tiles, the solves go by slot (the
+    start's bits); the tiles that a context holds are given back when another
+    of its buffers needs the room."""
+    torch = pytest.importorskip("torch")
+    cells = 400_000
+    world = workloads.jammed(cells, seed=7)
+    p = ContactDynamicsParameters(overlap_tolerance=5e-4)
+    system = mixed_system(2, cells, cells, LAWS[0])
+    initial = multipliers_for(system, 2)
+    expected = backend.evaluate_contact_response(system, initial)
+
+    def step(b, form):
+        b.set_relaxation(form)
+        stepped = world.copy()
+        b.advance_contact_dynamics(stepped, None, 0.002, p)
+        return stepped.geometry()
+
+    with B200Backend(0) as b:
+        by_slot = step(b, B200Backend.RELAXATION_GRAPH)
+        step(b, B200Backend.RELAXATION_GRAPH)  # rows and the last step's rows have their buffers
+        held = hold_all_but(64 << 20)
+        without = step(b, B200Backend.RELAXATION_AUTOMATIC)
+        assert set(b.last_step_solve_forms()) == {"slots"}
+        assert np.array_equal(without, by_slot)
+        del held
+        torch.cuda.empty_cache()
+        tiled = step(b, B200Backend.RELAXATION_AUTOMATIC)
+        assert any(form.startswith("tiles") for form in b.last_step_solve_forms())
+        held = hold_all_but(16 << 20)
+        got = b.evaluate_contact_response(system, initial)  # 64 MB of records
+        del held
+        torch.cuda.empty_cache()
+        assert np.array_equal(got.velocities, expected.velocities) and np.array_equal(got.loads, expected.loads)
+        assert np.array_equal(step(b, B200Backend.RELAXATION_AUTOMATIC), tiled)
+
+
 def test_a_copy_that_is_late_ends_the_solve(forms):
     """With no polls allowed the tiles' copies count as late: the solve ends
     with its first pass by tiles, after 8 iterations by slot (not after
