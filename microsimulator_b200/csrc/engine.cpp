@@ -1339,10 +1339,9 @@ void fill_problem(Ctx& c, SolveDesc& d, std::uint32_t row_count, float dt, const
 }
 
 void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_response& growth, float tolerance,
-               std::uint32_t max_iterations, bool with_state = false, bool resume = false) {
+               std::uint32_t max_iterations, bool with_state = false) {
   SolveDesc& d = *c.host_desc;
   fill_problem(c, d, row_count, dt, growth, tolerance, max_iterations);
-  d.resume = resume ? 1u : 0u;
   c.desc_current = true;
   c.last_tiled = 0;
   if (with_state) {
@@ -1356,6 +1355,7 @@ void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_
     d.ticket = 0;
     d.proceed = 0;
     d.handle = 0;
+    d.resume = 0;
     d.bound_ticket = 0;
     d.bound_bits = 0;
     d.barrier_count = 0;
@@ -1523,9 +1523,10 @@ int build_tiles(Ctx& c, bool resume, TileArrays& out) {
 //   - a solve starts by slot and goes on by tiles, from the iterate it has
 //     reached, when it needs more than kTiledAfter iterations, so that a short
 //     one costs what it did; the solves that follow a long one in the same
-//     step (kLongSolve) are likely to be long and start by tiles;
+//     step (kLongSolve) are likely to be long and start by tiles (1M in tracks:
+//     8 iterations by slot in each step's first solve cost 0.75 ms of 93);
 //   - a second solve of the same rows (a probe's) finds the tiles in place.
-constexpr std::uint32_t kTiledAfter = 8;
+constexpr std::uint32_t kTiledAfter = 4;
 constexpr std::uint32_t kLongSolve = 64;
 bool tiles_pay(std::uint64_t rows, std::uint64_t bodies) { return rows >= 2 * bodies; }
 
@@ -1573,14 +1574,14 @@ void run_solve(Ctx& c, SolveForm form, bool resume, bool finish, float dt, const
   } else {
     auto& graph = graph_for(c, std::max(rows, c.n));
     c.last_blocks = graph.blocks();
-    fill_desc(c, rows, dt, growth, tolerance, max_iterations, false, resume);
+    fill_desc(c, rows, dt, growth, tolerance, max_iterations);
     auto& made = c.tile_graphs[tiled ? c.tiles_built : 0];
     if (tiled && !made) {
       auto fresh = std::make_unique<SolveGraph>();
       check(cudaError_t(fresh->create(c.desc, kMaxPassBlocks, c.stream, c.tiles_built, c.wait_polls)), "solve graph");
       made = std::move(fresh);
     }
-    check(cudaError_t((tiled ? *made : graph).launch(c.stream)), "solve launch");
+    check(cudaError_t((tiled ? *made : graph).launch(c.stream, resume)), "solve launch");
   }
   c.last_tiled = tiled ? c.tiles_built : 0;
   if (finish) finish_solve(c);

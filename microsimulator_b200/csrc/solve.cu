@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cstddef>
 #include <cstdint>
 
 #include "device.cuh"
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(kSolveThreads, MSB_RELAX_MIN_BLOCKS)
 
 __global__ void __launch_bounds__(kSolveThreads) bound_kernel(SolveDesc* desc) {
   SolveDesc& d = *desc;
-  if (d.resume != 0u) return;
+  if (d.resume != 0) return;
   float bound = 0.0f;
   for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < d.row_count; i += gridDim.x * blockDim.x) {
     d.iterate[i] = make_float2(d.multipliers[i], 0.0f);  // the solve's starting multipliers
@@ -416,7 +417,7 @@ __global__ void unpack_iterate_kernel(const SolveDesc* desc) {
 }
 
 __global__ void solve_reset_kernel(SolveDesc* desc) {
-  if (threadIdx.x == 0 && desc->resume != 0u) {
+  if (threadIdx.x == 0 && desc->resume != 0) {
     desc->proceed = 1;  // the first pair of passes is an iteration
   } else if (threadIdx.x == 0) {
     desc->mode = 0;
@@ -727,9 +728,11 @@ int SolveGraph::loop_launches(std::uint32_t iterations) {
   return int(evaluations * 2 * MSB_WHILE_UNROLL);
 }
 
-int SolveGraph::launch(cudaStream_t stream) {
+int SolveGraph::launch(cudaStream_t stream, bool resume) {
   // Each graph has its own WHILE-node handle; the row pass reads it here.
-  cudaError_t err = cudaMemcpyAsync(&desc_->handle, &handle_, sizeof(handle_), cudaMemcpyHostToDevice, stream);
+  static_assert(offsetof(SolveDesc, resume) == offsetof(SolveDesc, handle) + sizeof(handle_));
+  const unsigned long long words[2] = {handle_, resume ? 1ull : 0ull};
+  cudaError_t err = cudaMemcpyAsync(&desc_->handle, words, sizeof(words), cudaMemcpyHostToDevice, stream);
   if (err != cudaSuccess) return err;
   count_launch(4);
   return cudaGraphLaunch(exec_, stream);

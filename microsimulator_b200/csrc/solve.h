@@ -1,6 +1,7 @@
 // The device-resident Barzilai-Borwein projected-gradient contact solve.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -99,8 +100,6 @@ struct SolveDesc {
   float tolerance;
   std::uint32_t max_iterations;
   std::uint32_t has_drift;  // 0: every drift is zero and the drift arrays are not read
-  std::uint32_t resume;      // the graph goes on from the state below instead of resetting it
-  std::uint32_t wait_polls;  // a 32nd of the polls after which a resident solve's CTAs are late
   TileArrays tiles;         // of a tiled solve
   // solver state
   float step;
@@ -111,7 +110,10 @@ struct SolveDesc {
   std::uint32_t mode;    // 0: evaluate the initial multipliers; 1: iterate
   std::uint32_t ticket;
   std::uint32_t proceed;
-  unsigned long long handle;  // cudaGraphConditionalHandle of the WHILE node
+  // Written by SolveGraph::launch: the cudaGraphConditionalHandle of the WHILE
+  // node, and whether the graph goes on from this state instead of resetting it.
+  unsigned long long handle;
+  unsigned long long resume;
   std::uint32_t bound_ticket;
   std::uint32_t bound_bits;
   // grid barrier of the fused solve (relax_kernel)
@@ -120,7 +122,12 @@ struct SolveDesc {
   std::uint32_t barrier_abort;  // a barrier wait ran out of time: every block stops
   std::uint32_t check_status;   // the first failed check (0: none): a wait that ran out; checked build: an index
   ResidentGang gang;            // the resident solve's
+  std::uint32_t wait_polls;     // a 32nd of the polls after which a resident solve's CTAs are late
 };
+
+// Every pass reads the tiles' pointers and the state; 8 bytes more before them
+// cost 1 us of a 90 us iteration of 4.15 M rows by tiles.
+static_assert(offsetof(SolveDesc, tiles) % 16 == 0);
 
 // Builds the incidence of `rows` over `bodies` bodies.  Scratch: `keys` and
 // `values` hold 2 * rows words each, `counts` bodies + 1 words, `temp`
@@ -146,7 +153,8 @@ class SolveGraph {
   // that many blocks an SM and `wait_polls`.  Returns a CUDA error code.
   int create(SolveDesc* desc, int blocks, cudaStream_t stream, int tiles_per_sm = 0,
              std::uint32_t wait_polls = kWaitPolls);
-  int launch(cudaStream_t stream);
+  // With `resume` the solve in the descriptor goes on.
+  int launch(cudaStream_t stream, bool resume = false);
   int blocks() const { return blocks_; }
   // Kernel launches of the WHILE node for a solve of `iterations`
   // iterations (whole evaluations of its unrolled body).

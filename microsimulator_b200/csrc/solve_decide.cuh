@@ -66,7 +66,6 @@ __device__ __forceinline__ std::uint32_t decide(SolveDesc& d, std::uint32_t mode
   __shared__ double red[5][kSolveThreads / 32];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
-  const std::uint32_t failed = __ldcg(&d.check_status);
   double t[5] = {0.0, 0.0, 0.0, 0.0, 1.0};
   for (std::uint32_t p = threadIdx.x; p < blocks; p += blockDim.x) {
 #pragma unroll
@@ -129,9 +128,6 @@ __device__ __forceinline__ std::uint32_t decide(SolveDesc& d, std::uint32_t mode
       proceed = iteration < d.max_iterations ? 1u : 0u;
     }
   }
-  // A failed check ends the solve: the sums may lack a block's, and every
-  // further iteration could wait as long again.
-  if (failed != 0u) proceed = 0;
   d.proceed = proceed;
   return proceed;
 }

@@ -201,7 +201,10 @@ __global__ void __launch_bounds__(kThreads, PerSm) tile_pass_kernel(SolveDesc* d
     }
     if (__syncthreads_or(!there) != 0) {
       if (threadIdx.x == 0) {
-        raise_status(check, kStatusIterations);  // ends the solve (decide)
+        raise_status(check, kStatusIterations);
+        // Sums that are not finite end the solve (decide): a further iteration
+        // could wait as long again.
+        for (int k = 0; k < 5; ++k) d.partials[5 * blockIdx.x + k] = 0.0;
         // The block keeps its shared memory until the copies into it are done.
         entries_there(barrier, phase, kWaitPolls);
       }
