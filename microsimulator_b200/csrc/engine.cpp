@@ -479,9 +479,11 @@ struct PinnedBuffer {
     cap = 0;
   }
   unsigned char* ensure(std::size_t bytes) {
-    if (bytes > cap) {
+    return bytes > cap ? ensure_exact(std::bit_ceil(std::max<std::size_t>(bytes + bytes / 4, 1 << 20))) : p;
+  }
+  unsigned char* ensure_exact(std::size_t c) {
+    if (c > cap) {
       release();
-      const std::size_t c = std::bit_ceil(std::max<std::size_t>(bytes + bytes / 4, 1 << 20));
       if (cudaMallocHost(reinterpret_cast<void**>(&p), c) != cudaSuccess) {
         p = nullptr;
         throw std::runtime_error("cudaMallocHost failed for staging memory");
@@ -580,15 +582,17 @@ struct msb_context {
   msb::DBuf<float4> body_a, body_b, drift_a, drift_b;
   msb::DBuf<std::uint32_t> inc_offsets;
   msb::DBuf<float4> inc_a, inc_b, resp_a, resp_b, accepted_a, accepted_b;
-  msb::DBuf<float2> inc_constants, inc_sides;  // per row: (offset, compliance), the two side terms
-  msb::DBuf<std::uint32_t> inc_places;         // per side: its entry's place
-  // The resident solve: each entry's slot, and the grid form's words.
+  // Per row: (offset, compliance); the two side terms; and, for systems that
+  // may be resident, the two entries' places.
+  msb::DBuf<float2> inc_rows;
+  bool inc_placed = false;
   std::optional<msb::ResidentLimits> resident_limits;
-  msb::DBuf<std::uint32_t> resident_slots;
-  msb::DBuf<unsigned long long> resident_inbox;
+  msb::DBuf<unsigned char> resident;  // the resident solve's scratch
   // The cells along a curve through the substep's base geometry, for the
-  // grid form; valid within a substep of one system.
-  msb::DBuf<std::uint32_t> spatial_keys, spatial_order, spatial_offsets;
+  // grid form and tiles, their keys and the entries before each; valid within
+  // a substep of one system.
+  msb::DBuf<std::uint32_t> spatial;
+  std::uint32_t* spatial_order() { return spatial.p; }
   bool spatial_valid = false;
   // The tiled solve's renumbered system (tiles.h) and its graph.
   msb::DBuf<unsigned char> tiles;
@@ -596,11 +600,8 @@ struct msb_context {
   int tiles_built = 0;         // the tiles are those of the rows at hand, this many blocks an SM
   bool tiles_refused = false;  // a system of this step did not suit tiles
   std::uint32_t step_iterations = 0;  // of this step's last solve
-  // A batch's schedule: jobs, gangs, each CTA's list.
-  msb::DBuf<msb::ResidentJob> batch_jobs;
-  msb::DBuf<msb::ResidentGang> batch_gangs;
-  msb::DBuf<std::uint32_t> batch_lists, batch_flags, colony_rest;
-  msb::DBuf<ulonglong2> resident_records;
+  msb::DBuf<std::uint32_t> batch_schedule;  // a batch's jobs, gangs and lists
+  msb::DBuf<std::uint32_t> colony_rest;
   msb::DBuf<float> slack;
 
   // A batch of independent colonies (msb_advance_contact_dynamics_batch);
@@ -833,10 +834,9 @@ void download_results(Ctx& c, std::initializer_list<HostResult> results) {
   std::vector<HostResult> pieces;
   std::size_t total = 0;
   for (const auto& r : results) total += r.bytes;
-  // Pieces a half: 4, 8 or 16 MB of pinned memory in all (rounded up).  A new
-  // context's first call on 10 to 40 thousand bodies: 13 to 16 ms, against 21
-  // to 29 with 16 MB whatever the results; repeated calls take the same time.
-  const std::size_t half_pieces = total > (std::size_t(24) << 20) ? kMostPieces : total > (std::size_t(4) << 20) ? 6 : 3;
+  // Pieces a half: 2, 4 or 12 MB of pinned memory in all, since pinning takes
+  // 0.7 ms a MB of a context's first call.
+  const std::size_t half_pieces = total > (std::size_t(24) << 20) ? kMostPieces : total > (std::size_t(4) << 20) ? 4 : 2;
   const std::size_t half_bytes = half_pieces * kPiece;
   for (const auto& r : results) {
     if (r.bytes == 0) continue;
@@ -850,7 +850,7 @@ void download_results(Ctx& c, std::initializer_list<HostResult> results) {
     }
   }
   if (!pieces.empty()) {
-    unsigned char* const staging = c.download.ensure(2 * half_bytes);
+    unsigned char* const staging = c.download.ensure_exact(2 * half_bytes);
     while (c.download_events.size() < 2 * kMostPieces) {
       cudaEvent_t e;
       check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
@@ -1311,7 +1311,13 @@ bool use_fused_relaxation(Ctx& c, std::uint32_t items) {
 }
 
 IncidenceArrays incidence_arrays(Ctx& c) {
-  return {c.inc_offsets.p, c.inc_a.p, c.inc_b.p, c.inc_constants.p, c.inc_sides.p, c.inc_places.p};
+  const std::size_t rows = std::max<std::uint32_t>(c.rows.count, 1);
+  return {c.inc_offsets.p,
+          c.inc_a.p,
+          c.inc_b.p,
+          c.inc_rows.p,
+          c.inc_rows.p + rows,
+          c.inc_placed ? reinterpret_cast<std::uint32_t*>(c.inc_rows.p + 2 * rows) : nullptr};
 }
 
 // The problem part of a solve's descriptor.
@@ -1370,15 +1376,24 @@ void fill_desc(Ctx& c, std::uint32_t row_count, float dt, const msb_growth_load_
   check(cudaMemcpyAsync(c.desc, &d, offsetof(SolveDesc, step), cudaMemcpyHostToDevice, c.stream), "desc");
 }
 
-void build_system_incidence(Ctx& c, std::uint32_t row_count) {
+// How a system of `rows` rows over the bodies at hand would be resident; not
+// at all (no CTAs) unless the form is automatic.
+ResidentPlan plan_resident(Ctx& c, std::uint64_t rows) {
+  if (c.relaxation != 0) return {};
+  if (!c.resident_limits) c.resident_limits = resident_limits();
+  return resident_plan(*c.resident_limits, rows, c.n);
+}
+
+// The incidence of c.rows.
+void build_system_incidence(Ctx& c) {
+  const std::uint32_t row_count = c.rows.count;
   const std::size_t entries = 2ull * std::max<std::uint32_t>(row_count, 1);
   c.tiles_built = 0;
   c.inc_offsets.ensure(c.n + 1ull);
   c.inc_a.ensure(entries);
   c.inc_b.ensure(entries);
-  c.inc_constants.ensure(entries / 2);
-  c.inc_sides.ensure(entries / 2);
-  c.inc_places.ensure(entries);
+  c.inc_placed = c.colonies > 0 || plan_resident(c, row_count).ctas > 0;
+  c.inc_rows.ensure(entries / 2 * (c.inc_placed ? 3 : 2));
   c.sort_keys.ensure(entries);
   c.sort_values.ensure(entries);
   c.counts.ensure(c.n + 1ull);
@@ -1399,25 +1414,46 @@ void build_row_keys(Ctx& c, RowStore& store) {
 
 SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growth, std::uint32_t max_iterations);
 
-// A resident solve's arrays; over several CTAs with words in global memory
-// (`grid`), and in spatial order where the substep has one.
-ResidentArrays resident_arrays(Ctx& c, bool grid) {
-  c.resident_slots.ensure(2ull * std::max<std::uint32_t>(c.rows.count, 1));
-  if (grid) {
-    c.resident_inbox.ensure(std::size_t(resident_stride()) * kResidentMaxCtas);
-    c.resident_records.ensure(2ull * kResidentMaxCtas * kResidentWords);
+// Parts of one allocation, 256-byte aligned; from a null base it counts their
+// bytes.
+struct Parts {
+  unsigned char* base;
+  std::size_t at = 0;
+  template <class T>
+  void add(T*& p, std::uint64_t count) {
+    p = reinterpret_cast<T*>(reinterpret_cast<std::uintptr_t>(base) + at);
+    at += (count * sizeof(T) + 255) & ~std::size_t(255);
   }
-  const bool ordered = grid && c.spatial_valid;
-  if (ordered) {
+};
+
+// A resident solve's arrays; with words in global memory for `ctas` CTAs of
+// the grid form (0: another form), which takes the bodies in spatial order
+// where the substep has one.
+ResidentArrays resident_arrays(Ctx& c, int ctas) {
+  ResidentArrays r{};
+  const auto lay_out = [&](unsigned char* base) {
+    Parts parts{base};
+    parts.add(r.slot_of, 2ull * std::max<std::uint32_t>(c.rows.count, 1));
+    if (ctas > 0) {
+      parts.add(r.inbox, std::uint64_t(resident_stride()) * ctas);
+      parts.add(r.records, 2ull * kResidentMaxCtas * kResidentWords);
+    }
+    return parts.at;
+  };
+  const std::size_t bytes = lay_out(nullptr);
+  if (!c.resident.try_ensure(bytes)) c.resident.ensure(bytes);  // which takes the tiles' memory back, or throws
+  lay_out(c.resident.p);
+  r.places = incidence_arrays(c).places;
+  r.stride = resident_stride();
+  if (ctas > 0 && c.spatial_valid) {
+    std::uint32_t* const offsets = c.spatial_order() + c.n;  // the keys' place: they have served
     c.counts.ensure(c.n + 1ull);
-    c.spatial_offsets.ensure(c.n + 1ull);
     c.temp.ensure(scan_temp_words(c.n + 1ull) + 64);
-    launch_order_offsets(c.n, c.spatial_order.p, c.inc_offsets.p, c.counts.p, c.spatial_offsets.p, c.temp.p, c.stream);
+    launch_order_offsets(c.n, c.spatial_order(), c.inc_offsets.p, c.counts.p, offsets, c.temp.p, c.stream);
+    r.order = c.spatial_order();
+    r.order_offsets = offsets;
   }
-  return {c.inc_places.p,    c.resident_slots.p,
-          c.resident_inbox.p, c.resident_records.p,
-          resident_stride(), ordered ? c.spatial_order.p : nullptr,
-          ordered ? c.spatial_offsets.p : nullptr};
+  return r;
 }
 
 void log_solve(Ctx& c, const msb_solve_record& record, std::uint32_t form) {
@@ -1429,7 +1465,7 @@ void log_solve(Ctx& c, const msb_solve_record& record, std::uint32_t form) {
 // holds its report.  False, with nothing done, when a share does not fit.
 bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_response& growth, float tolerance,
                     std::uint32_t max_iterations) {
-  const ResidentArrays arrays = resident_arrays(c, plan.grid);
+  const ResidentArrays arrays = resident_arrays(c, plan.grid ? plan.ctas : 0);
   fill_desc(c, c.rows.count, dt, growth, tolerance, max_iterations, true);
   check(cudaError_t(launch_resident(*c.host_desc, c.desc, arrays, plan, c.stream)), "solve launch");
   check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
@@ -1450,47 +1486,43 @@ int build_tiles(Ctx& c, bool resume, TileArrays& out) {
   const std::uint64_t slots = tile_slot_capacity(2ull * rows, tiles);
   if (slots > 0xFFFFFFFFull) return 0;
   c.temp.ensure(scan_temp_words(std::max<std::uint64_t>(n, rows) + 1) + 64);
-  // One allocation in 256-byte aligned parts: laid out from null for its size.
+  // One allocation for all of it.
   TileBuild build{};
   float *first = nullptr, *second = nullptr;
   const auto lay_out = [&](unsigned char* base) {
-    std::size_t at = 0;
-    const auto part = [&](auto*& p, std::uint64_t count) {
-      p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
-      at += (count * sizeof(*p) + 255) & ~std::size_t(255);
-    };
-    part(build.order, n);
-    part(build.place_of, n);
-    part(build.degree, n);
-    part(build.tile_slots, tiles + 1ull);
-    part(build.slot_base, tiles + 1ull);
-    part(build.group, n / 8 + 64ull);
-    part(build.a, slots);
-    part(build.b, slots);
-    part(build.body_a, n);
-    part(build.body_b, n);
-    part(build.row_counts, n + 1ull);
-    part(build.row_start, n + 1ull);
-    part(build.row_base, tiles + 1ull);
-    part(build.guest_counts, n + 1ull);
-    part(build.guest_start, n + 1ull);
-    part(build.guest_base, tiles + 1ull);
-    part(build.guests, rows + 1ull);
-    part(build.row_of, rows);
-    part(build.new_of, rows);
-    part(build.constants, rows + 2ull);  // the copies of a tile's rows start and end on 16 bytes
-    part(build.iterate, rows + 2ull);
-    part(build.flags, rows + 1ull);
-    part(build.positions, rows + 1ull);
-    part(build.boundary, rows);
-    part(build.report, 4);
-    part(first, rows);
-    part(second, rows);
-    return at;
+    Parts parts{base};
+    parts.add(build.order, n);
+    parts.add(build.place_of, n);
+    parts.add(build.degree, n);
+    parts.add(build.tile_slots, tiles + 1ull);
+    parts.add(build.slot_base, tiles + 1ull);
+    parts.add(build.group, n / 8 + 64ull);
+    parts.add(build.a, slots);
+    parts.add(build.b, slots);
+    parts.add(build.body_a, n);
+    parts.add(build.body_b, n);
+    parts.add(build.row_counts, n + 1ull);
+    parts.add(build.row_start, n + 1ull);
+    parts.add(build.row_base, tiles + 1ull);
+    parts.add(build.guest_counts, n + 1ull);
+    parts.add(build.guest_start, n + 1ull);
+    parts.add(build.guest_base, tiles + 1ull);
+    parts.add(build.guests, rows + 1ull);
+    parts.add(build.row_of, rows);
+    parts.add(build.new_of, rows);
+    parts.add(build.constants, rows + 2ull);  // the copies of a tile's rows start and end on 16 bytes
+    parts.add(build.iterate, rows + 2ull);
+    parts.add(build.flags, rows + 1ull);
+    parts.add(build.positions, rows + 1ull);
+    parts.add(build.boundary, rows);
+    parts.add(build.report, 4);
+    parts.add(first, rows);
+    parts.add(second, rows);
+    return parts.at;
   };
   if (!c.tiles.try_ensure(lay_out(nullptr))) return 0;
   lay_out(c.tiles.p);
-  launch_tile_build(n, rows, c.spatial_order.p, c.rows.slots.p, incidence_arrays(c),
+  launch_tile_build(n, rows, c.spatial_order(), c.rows.slots.p, incidence_arrays(c),
                     {c.body_a.p, c.body_b.p, c.drift_a.p, c.drift_b.p}, c.rows.keyed_offsets.p, c.rows.keyed_rows.p,
                     resume ? nullptr : c.rows.multipliers.p, c.rows.iterate.p, build, c.temp.p, c.stream);
   check(cudaMemcpyAsync(&c.host_scalars[kScalarCount + 6], build.report, 16, cudaMemcpyDeviceToHost, c.stream),
@@ -1613,8 +1645,7 @@ SolveOutcome solve(Ctx& c, float dt, const msb_growth_load_response& growth, flo
   bool solved = false;
   std::uint32_t form = 0;
   if (c.relaxation == 0) {
-    if (!c.resident_limits) c.resident_limits = resident_limits();
-    const ResidentPlan plan = resident_plan(*c.resident_limits, rows, c.n);
+    const ResidentPlan plan = plan_resident(c, rows);
     solved = plan.ctas > 0 && solve_resident(c, plan, dt, growth, tolerance, max_iterations);
     form = plan.grid ? MSB_FORM_GRID : plan.ctas > 1 ? MSB_FORM_CLUSTER : MSB_FORM_ONE_CTA;
   }
@@ -1785,29 +1816,31 @@ std::vector<std::uint32_t> solve_batch_resident(Ctx& c, const std::vector<std::u
   if (plan.jobs.empty()) return plan.rest;
   SolveDesc problem{};
   fill_problem(c, problem, c.rows.count, dt, growth, 0.0f, max_iterations);
-  const ResidentArrays arrays = resident_arrays(c, true);
-  c.batch_jobs.ensure(plan.jobs.size());
-  c.batch_gangs.ensure(plan.jobs.size());
-  c.batch_lists.ensure(plan.list_offsets.size() + plan.lists.size());
-  c.batch_flags.ensure(2);
-  check(cudaMemcpyAsync(c.batch_jobs.p, plan.jobs.data(), plan.jobs.size() * sizeof(ResidentJob),
-                        cudaMemcpyHostToDevice, c.stream),
-        "copy jobs");
-  check(cudaMemcpyAsync(c.batch_lists.p, plan.list_offsets.data(), plan.list_offsets.size() * 4,
-                        cudaMemcpyHostToDevice, c.stream),
-        "copy jobs");
-  check(cudaMemcpyAsync(c.batch_lists.p + plan.list_offsets.size(), plan.lists.data(), plan.lists.size() * 4,
-                        cudaMemcpyHostToDevice, c.stream),
-        "copy jobs");
-  check(cudaMemsetAsync(c.batch_gangs.p, 0, plan.jobs.size() * sizeof(ResidentGang), c.stream), "memset");
-  check(cudaMemsetAsync(c.batch_flags.p, 0, 8, c.stream), "memset");
-  const ResidentBatch batch{c.batch_jobs.p,     c.batch_gangs.p,       c.batch_lists.p,
-                            c.batch_lists.p + plan.list_offsets.size(), c.colony_offsets.p,
-                            c.colony_row_counts.p, c.colony_solve_tolerance.p, c.colony_state.p,
-                            c.batch_flags.p,    c.batch_flags.p + 1};
+  const ResidentArrays arrays = resident_arrays(c, int(ctas));
+  // One copy brings the schedule, with the gangs and flags as they start.
+  const std::size_t jobs = plan.jobs.size();
+  constexpr std::size_t kJobWords = sizeof(ResidentJob) / 4, kGangWords = sizeof(ResidentGang) / 4;
+  std::vector<std::uint32_t> words(jobs * (kJobWords + kGangWords) + 2, 0u);
+  std::memcpy(words.data(), plan.jobs.data(), jobs * sizeof(ResidentJob));
+  const std::size_t lists_at = words.size();
+  words.insert(words.end(), plan.list_offsets.begin(), plan.list_offsets.end());
+  words.insert(words.end(), plan.lists.begin(), plan.lists.end());
+  std::uint32_t* const at = c.batch_schedule.ensure(words.size());
+  check(cudaMemcpyAsync(at, words.data(), words.size() * 4, cudaMemcpyHostToDevice, c.stream), "copy jobs");
+  std::uint32_t* const batch_flags = at + jobs * (kJobWords + kGangWords);
+  const ResidentBatch batch{reinterpret_cast<ResidentJob*>(at),
+                            reinterpret_cast<ResidentGang*>(at + jobs * kJobWords),
+                            at + lists_at,
+                            at + lists_at + plan.list_offsets.size(),
+                            c.colony_offsets.p,
+                            c.colony_row_counts.p,
+                            c.colony_solve_tolerance.p,
+                            c.colony_state.p,
+                            batch_flags,
+                            batch_flags + 1};
   check(cudaError_t(launch_resident_batch(problem, arrays, batch, int(ctas), c.stream)), "batched solve launch");
   std::uint32_t flags[2] = {0, 0};
-  check(cudaMemcpyAsync(flags, c.batch_flags.p, 8, cudaMemcpyDeviceToHost, c.stream), "read flags");
+  check(cudaMemcpyAsync(flags, batch_flags, 8, cudaMemcpyDeviceToHost, c.stream), "read flags");
   check(cudaMemcpyAsync(c.host_colony_state.data(), c.colony_state.p, c.colonies * sizeof(msb::ColonyState),
                         cudaMemcpyDeviceToHost, c.stream),
         "read colony states");
@@ -1867,8 +1900,8 @@ SolveOutcome solve_batch(Ctx& c, float dt, const msb_growth_load_response& growt
     for (const std::uint32_t i : rest) left[i] = 1u;
     active = std::uint32_t(rest.size());
     form = all ? MSB_FORM_GANGS : MSB_FORM_GANGS_AND_CLUSTERS;
-    c.colony_rest.ensure(k);
     if (!all) {
+      c.colony_rest.ensure(k);
       check(cudaMemcpyAsync(c.colony_rest.p, left.data(), k * 4ull, cudaMemcpyHostToDevice, c.stream), "copy colonies");
       sync(c);
     }
@@ -2126,15 +2159,13 @@ Attempt advance_substep(Ctx& c, float dt, const msb_contact_dynamics_parameters&
   // made.
   c.spatial_valid = false;
   if (c.relaxation == 0 && found > 0 && n > 1) {
-    if (!c.resident_limits) c.resident_limits = resident_limits();
+    const ResidentPlan plan = plan_resident(c, found);
     if (c.colonies > 0 ? c.resident_limits->grid > 0 && c.colonies <= kResidentColonies
-                       : resident_plan(*c.resident_limits, found, n).grid ||
-                             (resident_plan(*c.resident_limits, found, n).ctas == 0 && tiles_pay(found, n))) {
-      c.spatial_keys.ensure(n);
-      c.spatial_order.ensure(n);
+                       : plan.grid || (plan.ctas == 0 && tiles_pay(found, n))) {
+      c.spatial.ensure(2ull * n + 1);
       c.temp.ensure(sort_temp_words(n) + 64);
       launch_spatial_order(n, c.state.pos_len.p, c.grid.p, c.colonies > 0 ? c.colony_of_slot.p : nullptr,
-                           std::max(c.colonies, 1u), c.spatial_keys.p, c.spatial_order.p, c.temp.p, c.stream);
+                           std::max(c.colonies, 1u), c.spatial_order() + n, c.spatial_order(), c.temp.p, c.stream);
       c.spatial_valid = true;
     }
   }
@@ -2162,7 +2193,7 @@ Attempt advance_substep(Ctx& c, float dt, const msb_contact_dynamics_parameters&
   Attempt attempt;
   for (std::uint32_t refinement = 0; refinement <= p.max_refinements; ++refinement) {
     mark(c, kPhaseIncidence);
-    build_system_incidence(c, c.rows.count);
+    build_system_incidence(c);
     if (refinement == 0 && (c.warm_start_mode & (kWarmGuess | kWarmLearned)) != 0 && c.has_guess) {
       guess_forces(c, dt, p.growth);
     }
@@ -2404,7 +2435,7 @@ void load_system(Ctx& c, const msb_contact_system& s, const float* multipliers) 
     check(cudaMemcpyAsync(c.rows.multipliers.p, multipliers, rows * 4ull, cudaMemcpyHostToDevice, c.stream),
           "copy multipliers");
   }
-  build_system_incidence(c, rows);
+  build_system_incidence(c);
 }
 
 // No allocation is made while the tiles are in use (from their build to the
