@@ -1396,10 +1396,10 @@ void build_system_incidence(Ctx& c) {
   c.inc_rows.ensure(entries / 2 * (c.inc_placed ? 3 : 2));
   c.sort_keys.ensure(entries);
   c.sort_values.ensure(entries);
-  c.counts.ensure(c.n + 1ull);
+  c.counts.ensure(c.n + 2ull);
   c.temp.ensure(sort_temp_words(entries) + scan_temp_words(c.n + 1ull) + 64);
   build_incidence(c.rows.arrays(), row_count, c.n, incidence_arrays(c), c.sort_keys.p,
-                  c.sort_values.p, c.counts.p, c.temp.p, c.stream, c.scalars.p + kStatus);
+                  c.sort_values.p, c.counts.p, c.temp.p, c.stream, c.scalars.p + kStatus, c.inc_placed);
 }
 
 void build_row_keys(Ctx& c, RowStore& store) {
@@ -1444,6 +1444,7 @@ ResidentArrays resident_arrays(Ctx& c, int ctas) {
   if (!c.resident.try_ensure(bytes)) c.resident.ensure(bytes);  // which takes the tiles' memory back, or throws
   lay_out(c.resident.p);
   r.places = incidence_arrays(c).places;
+  r.crowded = c.colonies > 0 ? nullptr : c.counts.p + c.n + 1;
   r.stride = resident_stride();
   if (ctas > 0 && c.spatial_valid) {
     std::uint32_t* const offsets = c.spatial_order() + c.n;  // the keys' place: they have served

@@ -527,7 +527,8 @@ __device__ Outcome load_share(const SolveDesc& d, const ResidentArrays& r, Comm<
   l.degree_at = carve(bodies);
   for (std::uint32_t i = threadIdx.x; i < 16; i += kThreads) s.warp[i] = s.parts[i] = Sums{{0.0, 0.0, 0.0}, 0u};
   if (threadIdx.x == 0) {
-    s.misfit = at > bytes || bodies > 0xFFFFu ? 1u : 0u;
+    const bool crowded = r.crowded != nullptr && *r.crowded != 0u;
+    s.misfit = crowded || at > bytes || bodies > 0xFFFFu ? 1u : 0u;
     s.remote_count = 0;
     s.slots = 0;
   }

@@ -16,6 +16,7 @@ struct ResidentArrays {
   unsigned long long* inbox;    // grid form: (round, side term) words, `stride` per CTA
   ulonglong2* records;          // grid form: two sets of a record of sums per CTA
   std::uint32_t stride;
+  const std::uint32_t* crowded;  // not zero: a body has too many entries (null: not known)
   // Bodies in the order in which CTAs take them, and the entries before each
   // in that order (bodies + 1); null: by slot.
   const std::uint32_t* order;
@@ -73,8 +74,6 @@ std::uint32_t resident_stride();
 // error code.
 int launch_resident(const SolveDesc& problem, SolveDesc* desc, const ResidentArrays& arrays, ResidentPlan plan,
                     cudaStream_t stream);
-constexpr std::uint32_t kResidentDegree = 62;
-
 // A batch of independent colonies in one launch: each colony is the job of a
 // gang of neighbouring CTAs that holds it, and each CTA takes its jobs in the
 // order of `jobs`.  On one cluster of 16 CTAs the largest colony sets a

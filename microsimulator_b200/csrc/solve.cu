@@ -452,11 +452,17 @@ __global__ void incidence_counts_kernel(RowArrays r, std::uint32_t rows, std::ui
 // order (the counts run back to zero).
 __global__ void incidence_scatter_kernel(const uint2* __restrict__ slots, std::uint32_t rows,
                                          const std::uint32_t* __restrict__ offsets,
-                                         std::uint32_t* __restrict__ counts, std::uint32_t* __restrict__ values) {
+                                         std::uint32_t* __restrict__ counts, std::uint32_t* __restrict__ values,
+                                         std::uint32_t* crowded) {
+  const auto put = [&](std::uint32_t body, std::uint32_t side) {
+    const std::uint32_t left = atomicSub(&counts[body], 1u);  // the first sees them all
+    values[offsets[body] + left - 1u] = side;
+    if (left > kResidentDegree && crowded != nullptr) *crowded = 1u;
+  };
   for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < rows; i += gridDim.x * blockDim.x) {
     const uint2 s = slots[i];
-    values[offsets[s.x] + atomicSub(&counts[s.x], 1u) - 1u] = i << 1;
-    if (s.y != kInvalidSlot) values[offsets[s.y] + atomicSub(&counts[s.y], 1u) - 1u] = (i << 1) | 1u;
+    put(s.x, i << 1);
+    if (s.y != kInvalidSlot) put(s.y, (i << 1) | 1u);
   }
 }
 
@@ -584,10 +590,11 @@ namespace {
 
 void incidence_pass(RowArrays rows, std::uint32_t row_count, std::uint32_t body_count, IncidenceArrays incidence,
                     std::uint32_t* values, std::uint32_t* counts, std::uint32_t* temp, cudaStream_t stream,
-                    std::uint32_t* status) {
+                    std::uint32_t* status, bool mark_crowded) {
+  std::uint32_t* const crowded = mark_crowded ? counts + body_count + 1 : nullptr;
   // Counts per body, their scan, the entries scattered into their bodies'
   // ranges, each range sorted by row, then the jacobians gathered.
-  cudaMemsetAsync(counts, 0, (body_count + 1) * sizeof(std::uint32_t), stream);
+  cudaMemsetAsync(counts, 0, (body_count + (crowded != nullptr ? 2 : 1)) * sizeof(std::uint32_t), stream);
   if (row_count > 0) {
     incidence_counts_kernel<<<grid_for(row_count, 256), 256, 0, stream>>>(rows, row_count, counts,
                                                                          incidence.constants, incidence.sides);
@@ -596,7 +603,7 @@ void incidence_pass(RowArrays rows, std::uint32_t row_count, std::uint32_t body_
   exclusive_scan(counts, incidence.offsets, body_count + 1, temp, stream);
   if (row_count == 0) return;
   incidence_scatter_kernel<<<grid_for(row_count, 256), 256, 0, stream>>>(rows.slots, row_count, incidence.offsets,
-                                                                          counts, values);
+                                                                          counts, values, crowded);
   count_launch();
   incidence_order_kernel<<<grid_for(body_count, 256), 256, 0, stream>>>(incidence.offsets, body_count, values);
   count_launch();
@@ -609,9 +616,9 @@ void incidence_pass(RowArrays rows, std::uint32_t row_count, std::uint32_t body_
 
 void build_incidence(RowArrays rows, std::uint32_t row_count, std::uint32_t body_count, IncidenceArrays incidence,
                      std::uint32_t* keys, std::uint32_t* values, std::uint32_t* counts, std::uint32_t* temp,
-                     cudaStream_t stream, std::uint32_t* status) {
+                     cudaStream_t stream, std::uint32_t* status, bool mark_crowded) {
   (void)keys;
-  incidence_pass(rows, row_count, body_count, incidence, values, counts, temp, stream, status);
+  incidence_pass(rows, row_count, body_count, incidence, values, counts, temp, stream, status, mark_crowded);
 }
 
 void build_keyed(const uint2* slots, std::uint32_t row_count, std::uint32_t body_count, std::uint32_t* offsets,

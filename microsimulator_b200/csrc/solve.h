@@ -61,6 +61,9 @@ struct IncidenceArrays {
   std::uint32_t* places;
 };
 
+// Entries a body may have in a resident solve.
+constexpr std::uint32_t kResidentDegree = 62;
+
 // Where the CTAs of a resident solve meet: how many hold their shares and how
 // many are done, the round they count from (the largest of their own), and
 // whether a share did not fit (nothing was done) or a wait ran out.
@@ -131,10 +134,11 @@ static_assert(offsetof(SolveDesc, tiles) % 16 == 0);
 
 // Builds the incidence of `rows` over `bodies` bodies.  Scratch: `keys` and
 // `values` hold 2 * rows words each, `counts` bodies + 1 words, `temp`
-// sort_temp_words(2 * rows) words.
+// sort_temp_words(2 * rows) words.  With `mark_crowded`, counts[bodies + 1]
+// says whether a body has more than kResidentDegree entries.
 void build_incidence(RowArrays rows, std::uint32_t row_count, std::uint32_t body_count, IncidenceArrays incidence,
                      std::uint32_t* keys, std::uint32_t* values, std::uint32_t* counts, std::uint32_t* temp,
-                     cudaStream_t stream, std::uint32_t* status = nullptr);
+                     cudaStream_t stream, std::uint32_t* status = nullptr, bool mark_crowded = false);
 
 // Stable lists of each first slot's rows (ForceMemory's KeyedRows).
 void build_keyed(const uint2* slots, std::uint32_t row_count, std::uint32_t body_count, std::uint32_t* offsets,

@@ -26,11 +26,14 @@ def forms(backend):
     backend.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
 
 
-def solve_both(backend, system, initial, iterations):
-    out = []
+def solve_both(backend, system, initial, iterations, automatic=None):
+    """The automatic form's solve (which ran as `automatic`) and the graph's."""
+    out, ran = [], []
     for form in (B200Backend.RELAXATION_AUTOMATIC, B200Backend.RELAXATION_GRAPH):
         backend.set_relaxation(form)
         out.append(backend.solve_contact_forces(system, initial, ContactSolveParameters(1e-9, iterations)))
+        ran.append(backend.last_step_solve_forms()[-1])
+    assert ran[1] == "slots" and (automatic is None or ran[0] == automatic)
     return out
 
 
@@ -45,8 +48,9 @@ SIZES = [(3, 2), (7, 5), (8, 30), (9, 30), (300, 1100), (350, 1300), (2000, 4000
 def test_agrees_with_the_graph(forms, bodies, rows, law):
     system = mixed_system(bodies + law, bodies, rows, LAWS[law])
     initial = multipliers_for(system, rows)
+    form = "one cta" if rows <= 1300 else "cluster" if rows <= 21000 else "grid"
     for iterations in (0, 1):
-        resident, graph = solve_both(forms, system, initial, iterations)
+        resident, graph = solve_both(forms, system, initial, iterations, form)
         assert resident.report == graph.report
         assert np.array_equal(resident.multipliers, graph.multipliers)
     resident, graph = solve_both(forms, system, initial, 6)
@@ -72,7 +76,7 @@ def test_bodies_of_many_rows(forms, degree):
     # Up to 62 entries a body the system is resident; beyond it takes the graph.
     system = hub_system(degree)
     initial = multipliers_for(system, 3)
-    resident, graph = solve_both(forms, system, initial, 1)
+    resident, graph = solve_both(forms, system, initial, 1, "one cta" if degree <= 62 else "slots")
     assert resident.report == graph.report
     assert np.array_equal(resident.multipliers, graph.multipliers)
 
