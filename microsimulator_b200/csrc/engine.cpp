@@ -1399,7 +1399,7 @@ void build_system_incidence(Ctx& c) {
   c.counts.ensure(c.n + 2ull);
   c.temp.ensure(sort_temp_words(entries) + scan_temp_words(c.n + 1ull) + 64);
   build_incidence(c.rows.arrays(), row_count, c.n, incidence_arrays(c), c.sort_keys.p,
-                  c.sort_values.p, c.counts.p, c.temp.p, c.stream, c.scalars.p + kStatus, c.inc_placed);
+                  c.sort_values.p, c.counts.p, c.temp.p, c.stream, c.scalars.p + kStatus, true);
 }
 
 void build_row_keys(Ctx& c, RowStore& store) {
@@ -1479,8 +1479,8 @@ bool solve_resident(Ctx& c, ResidentPlan plan, float dt, const msb_growth_load_r
 
 // Renumbers c.rows by tiles of c.spatial_order into `out`, with the iterate
 // (`resume`) or the multipliers of c.rows; returns how many blocks of the tile
-// pass share an SM, 0 when a body or a tile has too many rows or the device no
-// room.
+// pass share an SM, 0 when a tile has too many rows or the device no room, -1
+// when a body has too many rows.
 int build_tiles(Ctx& c, bool resume, TileArrays& out) {
   const std::uint32_t n = c.n, rows = c.rows.count;
   const std::uint32_t tiles = (n + kTileBodies - 1) / kTileBodies;
@@ -1529,7 +1529,7 @@ int build_tiles(Ctx& c, bool resume, TileArrays& out) {
   check(cudaMemcpyAsync(&c.host_scalars[kScalarCount + 6], build.report, 16, cudaMemcpyDeviceToHost, c.stream),
         "read");
   const std::uint32_t boundary = read_u32(c, build.positions + rows);
-  if (c.host_scalars[kScalarCount + 6] != 0u) return 0;
+  if (c.host_scalars[kScalarCount + 6] != 0u) return -1;
   const std::uint32_t max_slots = c.host_scalars[kScalarCount + 7], max_rows = c.host_scalars[kScalarCount + 8],
                       max_locals = c.host_scalars[kScalarCount + 9];
   out = {build.order,   build.degree,   build.slot_base, build.group,      build.a,         build.b,
@@ -1560,19 +1560,22 @@ int build_tiles(Ctx& c, bool resume, TileArrays& out) {
 //     8 iterations by slot in each step's first solve cost 0.75 ms of 93);
 //   - a second solve of the same rows (a probe's) finds the tiles in place.
 constexpr std::uint32_t kTiledAfter = 4;
+constexpr int kCrowded = 12;  // where host_scalars has that a body of the system has too many rows
 constexpr std::uint32_t kLongSolve = 64;
 bool tiles_pay(std::uint64_t rows, std::uint64_t bodies) { return rows >= 2 * bodies; }
 
 // The tiles of c.rows in `c.host_desc`, starting from c.rows.iterate with
 // `resume` and from c.rows.multipliers otherwise.  False when the system runs
-// better by slot, or not at all by tiles; the rest of the step then goes by
-// slot.
+// better by slot, or not at all by tiles; unless that is for one body's rows,
+// the rest of the step then goes by slot.
 bool use_tiles(Ctx& c, bool resume) {
   if (c.tiles_refused) return false;
   if (c.tiles_built > 0 && !resume) return true;  // the last solve's: its multipliers are these
-  c.tiles_built = build_tiles(c, resume, c.host_desc->tiles);
-  if (c.tiles_built == 1 && c.rows.count < 3ull * c.n) c.tiles_built = 0;
-  c.tiles_refused = c.tiles_built == 0;
+  c.tiles_built = 0;
+  if (resume && c.host_scalars[kScalarCount + kCrowded] != 0u) return false;
+  const int per_sm = build_tiles(c, resume, c.host_desc->tiles);
+  c.tiles_refused = per_sm == 0 || (per_sm == 1 && c.rows.count < 3ull * c.n);
+  if (per_sm > 0 && !c.tiles_refused) c.tiles_built = per_sm;
   return c.tiles_built > 0;
 }
 
@@ -1617,7 +1620,13 @@ void run_solve(Ctx& c, SolveForm form, bool resume, bool finish, float dt, const
     check(cudaError_t((tiled ? *made : graph).launch(c.stream, resume)), "solve launch");
   }
   c.last_tiled = tiled ? c.tiles_built : 0;
-  if (finish) finish_solve(c);
+  if (finish) {
+    finish_solve(c);
+  } else {
+    check(cudaMemcpyAsync(&c.host_scalars[kScalarCount + kCrowded], c.counts.p + c.n + 1, 4, cudaMemcpyDeviceToHost,
+                          c.stream),
+          "read");
+  }
   check(cudaMemcpyAsync(c.host_desc, c.desc, sizeof(SolveDesc), cudaMemcpyDeviceToHost, c.stream), "read desc");
   sync(c);
   const SolveDesc& d = *c.host_desc;
