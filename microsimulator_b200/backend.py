@@ -39,6 +39,22 @@ from .types import (
 )
 
 
+# Arrays up to this size may come from the allocator's heap, where an unused
+# tail can be resident memory; larger ones are mapped, and pages that were
+# never written take none.
+_HEAP_BYTES = 32 << 20
+
+
+def _filled(array: np.ndarray, count: int) -> np.ndarray:
+    """The first ``count`` elements of a call's own array: a view, so that a
+    large result is not copied once more, unless the array is small and mostly
+    unused (a program that keeps the contacts of many steps would keep several
+    times their memory)."""
+    if array.nbytes <= _HEAP_BYTES and 4 * count < len(array):
+        return array[:count].copy()
+    return array[:count]
+
+
 def device_count() -> int:
     """cuda_backend_device_count()."""
     return int(abi.load_library().msb_device_count())
@@ -235,7 +251,7 @@ class B200Backend:
                 continue
             self._check(status)
             self._capacity = max(self._capacity, int(count.value))
-            return out[: count.value]
+            return _filled(out, int(count.value))
 
     # -- ComputeBackend -------------------------------------------------
     def find_cell_contacts(self, world, parameters: ContactParameters | None = None) -> np.ndarray:
@@ -273,7 +289,7 @@ class B200Backend:
                 continue
             self._check(status)
             self._capacity = max(self._capacity, int(count.value))
-            return self._graph(n, contacts[: count.value], index, arrays)
+            return self._graph(n, _filled(contacts, int(count.value)), index, arrays)
 
     def build_contact_graph(self, contacts: np.ndarray, cell_count: int) -> ContactGraph:
         """ContactGraph(cell_count, contacts) (contact_graph.cpp:302-349) on
@@ -309,7 +325,7 @@ class B200Backend:
                 continue
             self._check(status)
             total = int(count.value)
-            return ExternalContactGraph(n, contacts[:total], offsets, indices[:total])
+            return ExternalContactGraph(n, _filled(contacts, total), offsets, _filled(indices, total))
 
     def build_contact_graph_device(self, contacts_pointer: int, count: int, cell_count: int, index) -> int:
         """msb_build_contact_graph on device-resident contact records and
