@@ -411,6 +411,14 @@ int msb_advance_contact_dynamics_device(
     const msb_constraint_contact_parameters* constraint_parameters,
     msb_contact_dynamics_report* report, msb_contact_dynamics_outputs* outputs);
 
+/* Test hook, no counterpart in the reference: msb_solve_contact_forces by
+ * tiles, whatever the system's size, with the bodies taken along `order` (a
+ * permutation) and at most `blocks_per_sm` (1 to 4) blocks an SM.
+ * MSB_ERR_INVALID_ARGUMENT when the system has no rows or does not fit tiles. */
+int msb_solve_by_tiles(msb_context* context, const msb_contact_system* system, const uint32_t* order,
+                       uint32_t blocks_per_sm, const float* initial, const msb_contact_solve_parameters* parameters,
+                       float* multipliers, msb_contact_solve_report* report);
+
 /* Measurement hook, no counterpart in the reference: runs `iterations` more
  * projected iterations of the last system this context solved (or evaluated
  * since), timing each pass with CUDA events on the context's stream; returns

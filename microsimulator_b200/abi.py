@@ -372,6 +372,19 @@ SIGNATURES = {
             POINTER(c_uint64),
         ],
     ),
+    "msb_solve_by_tiles": (
+        c_int,
+        [
+            c_void_p,
+            POINTER(ContactSystem),
+            c_void_p,
+            c_uint32,
+            c_void_p,
+            POINTER(ContactSolveParameters),
+            c_void_p,
+            POINTER(ContactSolveReport),
+        ],
+    ),
     "msb_solve_contact_forces": (
         c_int,
         [

@@ -398,6 +398,24 @@ class B200Backend:
             out = initial.copy()
         return ContactSolveResult(out, ContactSolveReport(report.status, report.iterations, report.residual))
 
+    def solve_by_tiles(self, system: ContactSystem, order, blocks_per_sm: int, initial_multipliers,
+                       parameters: ContactSolveParameters) -> ContactSolveResult:
+        """``solve_contact_forces`` by tiles along ``order`` (a permutation of
+        the bodies) with at most ``blocks_per_sm`` blocks an SM, whatever the
+        system's size: a test hook."""
+        native = system.native()
+        order = np.ascontiguousarray(order, dtype=np.uint32)
+        initial = np.ascontiguousarray(initial_multipliers, dtype=np.float32)
+        if initial.shape[0] != len(system.rows) or order.shape[0] != len(system.bodies):
+            raise ValueError("multipliers and order must match the system's rows and bodies")
+        out = np.zeros(len(system.rows), dtype=np.float32)
+        report = abi.ContactSolveReport()
+        prm = parameters.native()
+        self._check(self._lib.msb_solve_by_tiles(
+            self._handle, ctypes.byref(native), c_void_p(abi.ptr(order)), blocks_per_sm, c_void_p(abi.ptr(initial)),
+            ctypes.byref(prm), c_void_p(abi.ptr(out)), ctypes.byref(report)))
+        return ContactSolveResult(out, ContactSolveReport(report.status, report.iterations, report.residual))
+
     def evaluate_contact_response(self, system: ContactSystem, multipliers) -> ContactResponse:
         native = system.native()
         multipliers = np.ascontiguousarray(multipliers, dtype=np.float32)

@@ -3092,6 +3092,53 @@ int msb_solve_contact_forces(msb_context* context, const msb_contact_system* sys
   });
 }
 
+int msb_solve_by_tiles(msb_context* context, const msb_contact_system* system, const uint32_t* order,
+                       uint32_t blocks_per_sm, const float* initial, const msb_contact_solve_parameters* parameters,
+                       float* multipliers, msb_contact_solve_report* report) {
+  return guarded(context, [&] {
+    if (system == nullptr || order == nullptr || initial == nullptr || parameters == nullptr ||
+        multipliers == nullptr || report == nullptr) {
+      throw std::invalid_argument("null argument");
+    }
+    if (system->row_count == 0 || blocks_per_sm < 1 || blocks_per_sm > 4) {
+      throw std::invalid_argument("tiles need rows and 1 to 4 blocks an SM");
+    }
+    if (system->rows == nullptr || (system->body_count > 0 && system->bodies == nullptr)) {
+      throw std::invalid_argument("null system array");
+    }
+    validate_system(*system);
+    require_multipliers(initial, system->row_count);
+    if (!std::isfinite(parameters->tolerance) || parameters->tolerance <= 0.0f) {
+      throw std::invalid_argument("contact solve tolerance must be finite and positive");
+    }
+    std::vector<bool> taken(system->body_count, false);
+    for (std::uint64_t i = 0; i < system->body_count; ++i) {
+      if (order[i] >= system->body_count || taken[order[i]]) throw std::invalid_argument("order is no permutation");
+      taken[order[i]] = true;
+    }
+    auto& c = *context;
+    load_system(c, *system, initial);
+    build_row_keys(c, c.rows);
+    c.resp_a.ensure(c.n);
+    c.resp_b.ensure(c.n);
+    c.partials.ensure(5ull * kMaxPassBlocks);
+    c.spatial.ensure(2ull * c.n + 1);
+    check(cudaMemcpyAsync(c.spatial_order(), order, c.n * 4ull, cudaMemcpyHostToDevice, c.stream), "copy order");
+    const int per_sm = build_tiles(c, false, c.host_desc->tiles);
+    if (per_sm <= 0) throw std::invalid_argument("the system does not fit tiles");
+    c.tiles_built = std::min(per_sm, int(blocks_per_sm));
+    run_solve(c, SolveForm::kTiles, false, true, system->dt, system->growth, parameters->tolerance,
+              parameters->max_iterations);
+    const SolveDesc& d = *c.host_desc;
+    log_solve(c, {c.rows.count, d.iterations, d.status, d.residual}, MSB_FORM_TILES + std::uint32_t(c.tiles_built));
+    if (d.status == 3) throw std::invalid_argument("contact system has no positive diagonal");
+    check(cudaMemcpyAsync(multipliers, c.rows.multipliers.p, system->row_count * 4, cudaMemcpyDeviceToHost, c.stream),
+          "copy multipliers");
+    sync(c);
+    *report = {d.status, d.iterations, d.residual};
+  });
+}
+
 int msb_evaluate_contact_response(msb_context* context, const msb_contact_system* system, const float* multipliers,
                                   float* velocities, float* loads, float* length_rates) {
   return guarded(context, [&] {

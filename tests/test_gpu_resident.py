@@ -124,7 +124,7 @@ def test_waits_that_run_out_fail_the_call(forms):
     assert np.array_equal(step(), expected[1])
 
 
-@pytest.mark.parametrize("cells", [9000, 30000])
+@pytest.mark.parametrize("cells", [13000, 30000])
 @pytest.mark.parametrize("flat", [True, False])
 def test_steps_in_spatial_order(forms, cells, flat):
     """Steps whose solves spread over the grid in spatial order (a colony in
@@ -141,6 +141,7 @@ def test_steps_in_spatial_order(forms, cells, flat):
         stepped = world.copy()
         report = forms.advance_contact_dynamics(stepped, None, 0.02, p).report
         results.append((stepped, report))
+        assert set(forms.last_step_solve_forms()) == {"slots" if form == B200Backend.RELAXATION_GRAPH else "grid"}
     (a, ra), (b, rb) = results
     assert ra.substeps == rb.substeps and ra.halvings == rb.halvings
     assert np.max(np.abs(a.geometry() - b.geometry())) <= 4 * p.overlap_tolerance
@@ -177,14 +178,15 @@ def test_batch_by_gangs_steps_as_by_clusters(backend):
     batch = ColonyBatch([*worlds, star], np.full(8, 1.0), np.full(8, 1.0e4))
     p = ContactDynamicsParameters(overlap_tolerance=5e-4)
     counts = batch.counts()
-    results = []
+    results, ran = [], []
     with B200Backend(0) as b:
-        b.advance_contact_dynamics_batch(batch.concatenated(), counts, batch.drag, batch.stiffness, 0.002, p)  # tunes
         for form in (B200Backend.RELAXATION_AUTOMATIC, B200Backend.RELAXATION_GRAPH):
             b.set_relaxation(form)
             cells = batch.concatenated()
             report, colonies = b.advance_contact_dynamics_batch(cells, counts, batch.drag, batch.stiffness, 0.002, p)
             results.append((cells.geometry(), report, colonies))
+            ran.append(set(b.last_step_solve_forms()))
+    assert "gangs and clusters" in ran[0] and ran[1] == {"clusters"}
     (a, ra, ca), (g, rg, cg) = results
     assert ra.substeps == rg.substeps
     assert np.array_equal(ca["rows"], cg["rows"])

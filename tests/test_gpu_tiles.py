@@ -1,5 +1,7 @@
 """The tiled solve of systems too large to be resident, against the solve
-graph on the same steps: the same substeps, geometry within four solve
+graph: bit for bit on the same systems after 0 and 1 iterations, which take no
+sum over rows (test_gpu_resident.py states why later ones may differ in the
+last bits); on steps the same substeps, and geometry within four solve
 tolerances (two solves of one system may differ by that)."""
 
 import numpy as np
@@ -8,7 +10,12 @@ import pytest
 from microsimulator_b200 import abi, workloads
 from microsimulator_b200.backend import B200Backend
 from microsimulator_b200.sweep import ColonyBatch
-from microsimulator_b200.types import ContactDynamicsParameters, GrowthLoadResponse
+from microsimulator_b200.types import (
+    ContactDynamicsParameters,
+    ContactSolveParameters,
+    ContactSystem,
+    GrowthLoadResponse,
+)
 from microsimulator_b200.world import WorldState
 from tests.systems import LAWS, mixed_system, multipliers_for
 
@@ -21,18 +28,81 @@ def forms(backend):
     backend.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
 
 
-def step_both(backend, world, constraints=None, dt=0.002, **parameters):
+def step_both(backend, world, constraints=None, dt=0.002, tiled=True, **parameters):
     p = ContactDynamicsParameters(overlap_tolerance=5e-4, **parameters)
     results = []
+    ran = []
     for form in (B200Backend.RELAXATION_AUTOMATIC, B200Backend.RELAXATION_GRAPH):
         backend.set_relaxation(form)
         stepped = world.copy()
         result = backend.advance_contact_dynamics(stepped, constraints, dt, p)
         results.append((stepped, result.report))
+        ran.append(set(backend.last_step_solve_forms()))
+        if form == B200Backend.RELAXATION_AUTOMATIC and tiled:
+            assert any(name.startswith("tiles") for name in ran[0])
+            # The timing hook runs on the system of the last solve, by its form.
+            timed = backend.profile_iterations(2)
+            assert timed["bodies"] == len(world) and timed["rows"] == backend.last_step_solves()["rows"][-1]
+    assert ran[1] == {"slots"}
     (a, ra), (b, rb) = results
     assert ra.substeps == rb.substeps and ra.halvings == rb.halvings
     assert np.max(np.abs(a.geometry() - b.geometry())) <= 4 * p.overlap_tolerance
     return ra
+
+
+def neighbours_system(seed: int, bodies: int, rows: int, law) -> tuple[ContactSystem, np.ndarray]:
+    """A mixed system whose pair rows join bodies at most 20 apart along a
+    hidden order (returned), so that most rows lie within a tile."""
+    system = mixed_system(seed, bodies, rows, law)
+    rng = np.random.default_rng(seed + 1)
+    order = rng.permutation(bodies)
+    pairs = system.rows["second_slot"] != abi.INVALID_SLOT
+    first = rng.integers(0, bodies, rows)
+    second = np.clip(first + rng.integers(1, 21, rows) * rng.choice([-1, 1], rows), 0, bodies - 1)
+    second = np.where(second == first, (first + 1) % bodies, second)
+    system.rows["first_slot"] = order[first]
+    system.rows["second_slot"] = np.where(pairs, order[second], abi.INVALID_SLOT)
+    return system, order
+
+
+def solve_both_ways(backend, system, order, blocks, initial, iterations):
+    parameters = ContactSolveParameters(1e-9, iterations)
+    tiled = backend.solve_by_tiles(system, order, blocks, initial, parameters)
+    form = backend.last_step_solve_forms()[-1]
+    backend.set_relaxation(B200Backend.RELAXATION_GRAPH)
+    return tiled, backend.solve_contact_forces(system, initial, parameters), form
+
+
+# One tile (its rows all within it, no boundary rows), a last tile of one body,
+# of all but one; drift and constraint rows in each.
+@pytest.mark.parametrize("bodies,rows", [(3, 2), (5, 7), (255, 500), (256, 256), (257, 260), (1000, 1000), (5119, 5000)])
+@pytest.mark.parametrize("blocks", [1, 2, 3, 4])
+@pytest.mark.parametrize("law", range(3))
+def test_agrees_with_the_graph(forms, bodies, rows, blocks, law):
+    system, order = neighbours_system(bodies + law, bodies, rows, LAWS[law])
+    initial = multipliers_for(system, rows)
+    for iterations in (0, 1):
+        tiled, graph, form = solve_both_ways(forms, system, order, blocks, initial, iterations)
+        assert form == f"tiles {blocks}"
+        assert tiled.report == graph.report
+        assert np.array_equal(tiled.multipliers, graph.multipliers)
+    tiled, graph, _ = solve_both_ways(forms, system, order, blocks, initial, 6)
+    assert tiled.report.iterations == graph.report.iterations
+    assert np.max(np.abs(tiled.multipliers - graph.multipliers)) <= 1e-5 * np.max(np.abs(graph.multipliers))
+
+
+# Rows between random bodies, nearly all of them between tiles: more guests
+# than the two that a thread fetches ahead, tiles with an odd first row.
+@pytest.mark.parametrize("bodies,rows,fit", [(2000, 2000, 4), (3001, 9000, 3), (2000, 8000, 2), (2049, 12000, 1)])
+def test_many_rows_between_tiles(forms, bodies, rows, fit):
+    system = mixed_system(bodies, bodies, rows, LAWS[1])
+    order = np.random.default_rng(rows).permutation(bodies)
+    initial = multipliers_for(system, 1)
+    for iterations in (0, 1):
+        tiled, graph, form = solve_both_ways(forms, system, order, fit, initial, iterations)
+        assert form == f"tiles {fit}"
+        assert tiled.report == graph.report
+        assert np.array_equal(tiled.multipliers, graph.multipliers)
 
 
 # A last tile of one body, of all its bodies, of all but one.
@@ -41,7 +111,6 @@ def step_both(backend, world, constraints=None, dt=0.002, **parameters):
 def test_steps_by_tiles(forms, cells, law):
     world = workloads.jammed(cells, seed=cells)
     step_both(forms, world, growth=GrowthLoadResponse(law, 0.0, 0.2, 3.0))
-    assert forms.profile_iterations(2)["bodies"] == cells
 
 
 def test_walls_by_tiles(forms):
@@ -63,7 +132,10 @@ def test_a_body_of_many_rows(forms, cells):
         np.stack([np.append(fields["direction_x"], 1.0), np.append(fields["direction_y"], 0.0),
                   np.append(fields["direction_z"], 0.0)], axis=1),
         np.append(fields["lengths"], 120.0), 0.5, growth_rates=0.5)
-    step_both(forms, long)
+    step_both(forms, long, tiled=False)
+    forms.set_relaxation(B200Backend.RELAXATION_AUTOMATIC)
+    forms.advance_contact_dynamics(long.copy(), None, 0.002, ContactDynamicsParameters(overlap_tolerance=5e-4))
+    assert "slots" in forms.last_step_solve_forms()
 
 
 def forms_of(backend, world, dt=0.002, tolerance=5e-4):
