@@ -116,19 +116,21 @@ struct DBuf {
     }
     return p;
   }
-  // The same with an eighth to spare; false, and empty, when the device has no
-  // room.
+  // The same for twice n where the device has room (a colony that grows 2 % a
+  // step regrew an eighth every few steps: 5 ms of a step of 1M cells), else for
+  // n; false, and empty, when there is none for that either.
   bool try_ensure(std::size_t n) {
     if (n <= cap) return true;
     release();
-    const std::size_t c = n + n / 8;
-    if (cudaMalloc(&p, c * sizeof(T)) != cudaSuccess) {
+    for (const std::size_t c : {2 * n, n}) {
+      if (cudaMalloc(&p, c * sizeof(T)) == cudaSuccess) {
+        cap = c;
+        return true;
+      }
       cudaGetLastError();
       p = nullptr;
-      return false;
     }
-    cap = c;
-    return true;
+    return false;
   }
   // Grows to at least n elements keeping the first `keep`.
   T* grow(std::size_t n, std::size_t keep, cudaStream_t stream) {
