@@ -13,9 +13,9 @@ the tolerance.  Divisions are input preparation and run between steps.
   e2e    the same steps through the host-buffer C-ABI call with the world in
          page-locked host arrays, host<->device copies inside the timed
          region (and, beside it, with ordinary pageable arrays)
-  roofline  the BB iteration (body pass + row pass) of the last solved
-         system, CUDA events on the backend's stream, against algorithmic
-         bytes R*96 + N*128 per iteration
+  roofline  the BB iterations of the timed steps' solves, CUDA events on the
+         backend's stream, against algorithmic bytes R*96 + N*128 per
+         iteration, with the form that most of them ran in
   cpu_baseline  the reference CPU backend (compiled from its sources) on the
          first timed steps of the same colony from the same state, about
          15 s of stepping, all host threads
@@ -166,16 +166,21 @@ def measured_peak():
     return 6650.0, "fallback"
 
 
-def ncu_traffic():
-    """DRAM bytes of one BB iteration as a multiple of its algorithmic bytes,
-    from the committed ncu capture (profiles/bb_iteration_traffic.json, the
-    tiled passes over a 400,000-capsule colony's system: 1.66M rows); None
-    without one.  The bench scales it to its own launches by the algorithmic
-    bytes, which grow with rows and bodies as the traffic does."""
+# What an iteration of a solve is, by the solve's form (B200Backend.SOLVE_FORMS);
+# the others keep their system in shared memory.
+PASSES = {"tiles": "tile pass + boundary pass", "slots": "body pass + row pass"}
+
+
+def ncu_traffic(form):
+    """DRAM bytes of one BB iteration in `form` as a multiple of its
+    algorithmic bytes, from the committed ncu captures of such a colony's
+    system (profiles/bb_iteration_traffic.json); None without one.  The bench
+    scales it to its own iterations by the algorithmic bytes, which grow with
+    rows and bodies as the traffic does."""
     path = ROOT / "profiles" / "bb_iteration_traffic.json"
     if not path.exists():
         return None
-    return json.loads(path.read_text())
+    return json.loads(path.read_text()).get(form)
 
 
 def reference_steps(args, world, first_step, seconds, steps_cap, seed):
@@ -633,6 +638,7 @@ def main():
     # solve (rows * 96 + cells * 128 per iteration) and the solve phase's
     # CUDA-event time on the backend's stream.
     live = {"bytes": 0, "iterations": 0, "solve_ms": 0.0}
+    forms = {}  # iterations by the form of their solve
     rechecks = {"full": 0, "kept": 0, "partial": 0}
 
     def timed(world, mode, record=False):
@@ -654,9 +660,10 @@ def main():
             if record:
                 # Every timed step's solves: bytes and iterations, and the
                 # solve phase's device time.
-                for solve in backend.last_step_solves():
+                for solve, form in zip(backend.last_step_solves(), backend.last_step_solve_forms()):
                     live["bytes"] += (int(solve["rows"]) * 96 + len(world) * 128) * int(solve["iterations"])
                     live["iterations"] += int(solve["iterations"])
+                    forms[form.split(" ")[0]] = forms.get(form.split(" ")[0], 0) + int(solve["iterations"])
                 live["solve_ms"] += step_phases["solve"]
                 for name, count in backend.last_step_searches().items():
                     rechecks[name] += count
@@ -673,7 +680,8 @@ def main():
         total_ms, cell_steps, iterations, phases = timed(world, 0, record=True)
     barrier()
     launches = backend.launch_count() - launches0
-    prof = backend.profile_iterations(20)
+    last_form = (backend.last_step_solve_forms() or ["slots"])[-1].split(" ")[0]
+    prof = {**backend.profile_iterations(20), "form": last_form} if last_form in PASSES else None
 
     # e2e: the same steps from the same state through the host-buffer call,
     # host<->device copies inside the timed region.  The world's arrays are
@@ -743,17 +751,18 @@ def main():
     total = replicas.max_over_ranks(total_ms, dist, f"cuda:{local}")
     value = replicas.sum_over_ranks(cell_steps, dist, f"cuda:{local}") / (total * 1e-3)
 
-    # The dominant kernel is the BB iteration (body pass + row pass), run by
-    # the solve graph.  achieved = the live algorithmic bytes of every
-    # iteration of the timed steps over the solve phase's time: the phase
-    # also holds each solve's bound and initial passes and its graph launch,
-    # so the figure is a lower bound.  The timing hook's separate launches
-    # give the two passes apart (their split, for the ncu shares).
+    # The dominant work is the BB iteration, run by the solve graph.  achieved
+    # = the live algorithmic bytes of every iteration of the timed steps over
+    # the solve phase's time: the phase also holds each solve's bound and
+    # initial passes, its preparation and its graph launch, so the figure is a
+    # lower bound.  The timing hook's separate launches give the two passes of
+    # the last solve apart (their split, for the ncu shares).
     peak, peak_kind = measured_peak()
     algorithmic = live["bytes"] / max(1, live["iterations"])
     iteration_ms = live["solve_ms"] / max(1, live["iterations"])
     achieved = live["bytes"] / (live["solve_ms"] * 1e-3) / 1e9 if live["solve_ms"] > 0 else 0.0
-    traffic = ncu_traffic()
+    form = max(forms, key=forms.get) if forms else "slots"
+    traffic = ncu_traffic(form)
     traffic_bytes = None
     if traffic is not None:
         traffic_bytes = algorithmic * traffic["ratio_to_algorithmic"]
@@ -803,7 +812,8 @@ def main():
             # The timed steps' overlap re-checks by how their candidates were found.
             "rechecks": rechecks,
             "roofline": {
-                "kernel": "bb_iteration (tile pass + boundary pass)",
+                "kernel": f"bb_iteration ({PASSES.get(form, 'resident in shared memory: ' + form)})",
+                "iterations_by_form": forms,
                 "bound": "hbm",
                 "achieved": achieved,
                 "peak": peak,
@@ -816,9 +826,10 @@ def main():
                 "iterations": live["iterations"],
                 "measured": "CUDA events on the backend stream around the solve phase of the timed steps; bytes = "
                             "sum over solves of (rows * 96 + cells * 128) * iterations",
-                "passes": {"body_ms": prof["body_ms"], "row_ms": prof["row_ms"], "rows": prof["rows"],
-                           "bodies": prof["bodies"],
-                           "how": "timing hook after the timed region: 20 iterations as separate launches"},
+                "passes": prof and {"form": prof["form"], "body_ms": prof["body_ms"], "row_ms": prof["row_ms"],
+                                    "rows": prof["rows"], "bodies": prof["bodies"],
+                                    "how": "timing hook after the timed region: 20 iterations of the last solved "
+                                           "system as separate launches"},
             },
             "cpu_baseline": cpu,
             "e2e": e2e,

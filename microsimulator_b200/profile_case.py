@@ -3,8 +3,10 @@
 --case bb (default): relaxes a jammed colony for a few contact-dynamics
 steps, then times extra projected iterations of the last solved system with
 the timing hook (msb_profile_iterations), whose launches carry their own
-kernel instance names (``body_pass_kernel<1>`` / ``row_pass_kernel<1>``) so
-that a profiler can select them apart from the solve graph's launches:
+kernel instance names (by tiles ``tile_pass_kernel<1, blocks an SM>`` /
+``boundary_pass_kernel<1>``, by slot ``body_pass_kernel<1>`` /
+``row_pass_kernel<1>``) so that a profiler can select them apart from the
+solve graph's launches; ``--relaxation 1`` keeps the solves by slot:
 
   python -m microsimulator_b200.profile_case --cells 500000 --steps 2 --iterations 3
 
@@ -18,8 +20,8 @@ keeping activations, ``gemm_tc_kernel``, ``gemm_reduce_kernel``):
 
   python -m microsimulator_b200.profile_case --case train --cells 8192 --iterations 5
 
---case batch: one step of a batch of sweep colonies (``batch_solve_kernel``;
-the first call's autotuner launches the kernel once per launch shape first):
+--case batch: one step of a batch of sweep colonies (``resident_batch_kernel``;
+``--relaxation 1``: ``batch_solve_kernel``):
 
   python -m microsimulator_b200.profile_case --case batch --colonies 64
 
@@ -119,6 +121,7 @@ def batch_case(args) -> None:
     from .types import ContactDynamicsParameters
 
     backend = B200Backend(0)
+    backend.set_relaxation(args.relaxation)
     batch = sweep.sweep_batch(count=args.colonies, seed=args.seed)
     dyn = ContactDynamicsParameters(overlap_tolerance=5e-4)
     for k in range(args.steps):
@@ -126,7 +129,8 @@ def batch_case(args) -> None:
         report, colonies = batch.step(backend, 0.02, dyn)
     torch.cuda.synchronize()
     print(json.dumps({"cells": int(batch.counts().sum()), "iterations": int(colonies["iterations"].sum()),
-                      "tuning": backend.batch_tuning(), "solves": backend.last_step_solves()["iterations"].tolist()}))
+                      "tuning": backend.batch_tuning(), "solves": backend.last_step_solves()["iterations"].tolist(),
+                      "forms": backend.last_step_solve_forms()}))
     backend.close()
 
 
@@ -273,6 +277,7 @@ def main() -> None:
     p.add_argument("--cells", type=int, default=500_000)
     p.add_argument("--steps", type=int, default=2)
     p.add_argument("--iterations", type=int, default=3)
+    p.add_argument("--relaxation", type=int, default=0)
     p.add_argument("--seed", type=int, default=42)
     args = p.parse_args()
     if args.case == "mlp":
@@ -299,6 +304,7 @@ def main() -> None:
     from .types import ContactDynamicsParameters
 
     backend = B200Backend(0)
+    backend.set_relaxation(args.relaxation)
     world = workloads.jammed(n=args.cells, seed=args.seed)
     dyn = ContactDynamicsParameters(overlap_tolerance=5e-4)
     reports = []
@@ -311,6 +317,7 @@ def main() -> None:
     timing = backend.profile_iterations(args.iterations)
     timing["algorithmic_bytes"] = timing["rows"] * 96 + timing["bodies"] * 128
     timing["iterations_per_step"] = reports
+    timing["forms"] = backend.last_step_solve_forms()
     print(json.dumps(timing))
     backend.close()
 
