@@ -1396,21 +1396,19 @@ void build_system_incidence(Ctx& c) {
   c.inc_b.ensure(entries);
   c.inc_placed = c.colonies > 0 || plan_resident(c, row_count).ctas > 0;
   c.inc_rows.ensure(entries / 2 * (c.inc_placed ? 3 : 2));
-  c.sort_keys.ensure(entries);
   c.sort_values.ensure(entries);
   c.counts.ensure(c.n + 2ull);
   c.temp.ensure(sort_temp_words(entries) + scan_temp_words(c.n + 1ull) + 64);
-  build_incidence(c.rows.arrays(), row_count, c.n, incidence_arrays(c), c.sort_keys.p,
-                  c.sort_values.p, c.counts.p, c.temp.p, c.stream, c.scalars.p + kStatus, true);
+  build_incidence(c.rows.arrays(), row_count, c.n, incidence_arrays(c), c.sort_values.p, c.counts.p, c.temp.p,
+                  c.stream, c.scalars.p + kStatus, true);
 }
 
 void build_row_keys(Ctx& c, RowStore& store) {
-  c.sort_keys.ensure(std::max<std::uint32_t>(store.count, 1));
   c.counts.ensure(c.n + 1ull);
   store.keyed_offsets.ensure(c.n + 1ull);
   store.keyed_rows.ensure(std::max<std::uint32_t>(store.count, 1));
   c.temp.ensure(sort_temp_words(store.count + 1ull) + scan_temp_words(c.n + 1ull) + 64);
-  build_keyed(store.slots.p, store.count, c.n, store.keyed_offsets.p, store.keyed_rows.p, c.sort_keys.p, c.counts.p,
+  build_keyed(store.slots.p, store.count, c.n, store.keyed_offsets.p, store.keyed_rows.p, c.counts.p,
               c.temp.p, c.stream);
 }
 

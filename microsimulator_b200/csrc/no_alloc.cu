@@ -387,7 +387,7 @@ extern "C" int msb_solve_contact_forces_no_alloc(const msb_contact_system* syste
     return MSB_ERR_CUDA;
   }
   launch_rows_from_records(records, rows, s.rows, stream);
-  build_incidence(s.rows, rows, bodies, s.incidence, nullptr, values, counts, temp, stream);
+  build_incidence(s.rows, rows, bodies, s.incidence, values, counts, temp, stream);
   small_solve_kernel<<<1, kBlock, 0, stream>>>(s);
   count_launch();
   // On a CUDA error `multipliers` may already hold part of the device copy

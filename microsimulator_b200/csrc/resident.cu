@@ -1065,7 +1065,7 @@ int launch_resident(const SolveDesc& problem, SolveDesc* desc, const ResidentArr
                     cudaStream_t stream) {
   if (plan.grid) return launch_lanes<kGrid>(problem, desc, arrays, plan, stream);
   if (plan.ctas > 1) return launch_lanes<kCluster>(problem, desc, arrays, plan, stream);
-  return launch_lanes<kSingle>(problem, desc, arrays, plan, stream);
+  return launch_form<kSingle, 1>(problem, desc, arrays, plan.ctas, stream);
 }
 
 }  // namespace msb

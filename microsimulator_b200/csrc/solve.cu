@@ -615,18 +615,15 @@ void incidence_pass(RowArrays rows, std::uint32_t row_count, std::uint32_t body_
 }  // namespace
 
 void build_incidence(RowArrays rows, std::uint32_t row_count, std::uint32_t body_count, IncidenceArrays incidence,
-                     std::uint32_t* keys, std::uint32_t* values, std::uint32_t* counts, std::uint32_t* temp,
-                     cudaStream_t stream, std::uint32_t* status, bool mark_crowded) {
-  (void)keys;
+                     std::uint32_t* values, std::uint32_t* counts, std::uint32_t* temp, cudaStream_t stream,
+                     std::uint32_t* status, bool mark_crowded) {
   incidence_pass(rows, row_count, body_count, incidence, values, counts, temp, stream, status, mark_crowded);
 }
 
 void build_keyed(const uint2* slots, std::uint32_t row_count, std::uint32_t body_count, std::uint32_t* offsets,
-                 std::uint32_t* rows_out, std::uint32_t* keys, std::uint32_t* counts, std::uint32_t* temp,
-                 cudaStream_t stream) {
+                 std::uint32_t* rows_out, std::uint32_t* counts, std::uint32_t* temp, cudaStream_t stream) {
   // Counts per first slot, their scan, the rows scattered into their lists,
   // each list sorted by row (a stable grouping, as KeyedRows keeps).
-  (void)keys;
   cudaMemsetAsync(counts, 0, (body_count + 1) * sizeof(std::uint32_t), stream);
   if (row_count > 0) {
     keyed_counts_kernel<<<grid_for(row_count, 256), 256, 0, stream>>>(slots, row_count, counts);

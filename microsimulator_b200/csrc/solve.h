@@ -132,18 +132,17 @@ struct SolveDesc {
 // cost 1 us of a 90 us iteration of 4.15 M rows by tiles.
 static_assert(offsetof(SolveDesc, tiles) % 16 == 0);
 
-// Builds the incidence of `rows` over `bodies` bodies.  Scratch: `keys` and
-// `values` hold 2 * rows words each, `counts` bodies + 1 words, `temp`
-// sort_temp_words(2 * rows) words.  With `mark_crowded`, counts[bodies + 1]
+// Builds the incidence of `rows` over `bodies` bodies.  Scratch: `values` holds
+// 2 * rows words, `counts` bodies + 1 words (+ 2 with `mark_crowded`), `temp`
+// scan_temp_words(bodies + 1) words.  With `mark_crowded`, counts[bodies + 1]
 // says whether a body has more than kResidentDegree entries.
 void build_incidence(RowArrays rows, std::uint32_t row_count, std::uint32_t body_count, IncidenceArrays incidence,
-                     std::uint32_t* keys, std::uint32_t* values, std::uint32_t* counts, std::uint32_t* temp,
-                     cudaStream_t stream, std::uint32_t* status = nullptr, bool mark_crowded = false);
+                     std::uint32_t* values, std::uint32_t* counts, std::uint32_t* temp, cudaStream_t stream,
+                     std::uint32_t* status = nullptr, bool mark_crowded = false);
 
 // Stable lists of each first slot's rows (ForceMemory's KeyedRows).
 void build_keyed(const uint2* slots, std::uint32_t row_count, std::uint32_t body_count, std::uint32_t* offsets,
-                 std::uint32_t* rows_out, std::uint32_t* keys, std::uint32_t* counts, std::uint32_t* temp,
-                 cudaStream_t stream);
+                 std::uint32_t* rows_out, std::uint32_t* counts, std::uint32_t* temp, cudaStream_t stream);
 
 // A solve graph for a fixed grid size: bound -> initial gaps -> WHILE
 // (not converged) { body pass; row pass }.
