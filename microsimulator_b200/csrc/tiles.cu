@@ -19,12 +19,16 @@
 // (Entries loaded into registers by each thread, 8 or 4 at a time, were
 // bound by latency: 250 and 197 us a pass at 4.15 M rows.)
 //
-// At 4.15 M rows over 1 M bodies the tile pass takes 85 us and the boundary
-// pass 16 (145 and 40 in the two passes by slot); 153 of the 155 MB it moves
+// At 4.15 M rows over 1 M bodies the tile pass takes 82 us and the boundary
+// pass 16 (163 and 31 in the two passes by slot); 153 of the 155 MB it moves
 // at 1.66 M rows are what it cannot do without.  Two blocks an SM, the chain
 // of each tile's copy, sums, side terms and rows bounds it, not DRAM.  Two
 // lanes a body (512 threads) measured 118 us where one measured 111: more
-// instructions, no more overlap; tiles of 128 to 248 bodies 0 to 15 % slower.
+// instructions, no more overlap.  Tiles of 256, 240, 224, 208 and 192 bodies,
+// both passes: 91, 93, 79, 81 and 82 us at 1 M random capsules (a third block
+// an SM fits from 224 on), 105, 119, 122, 126 and 132 at 1.7 M grown ones, 110,
+// 109, 112, 115 and 119 at 1 M settled, 31 to 35 at 300,000: no smaller size
+// is better for all of them.
 //
 // The arithmetic is the two passes', term by term; a body's entries are in
 // row order.  Only the FP64 sums are taken in another fixed order.
