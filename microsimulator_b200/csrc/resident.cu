@@ -492,13 +492,12 @@ __device__ __forceinline__ Sums receive_sides(const SolveDesc& d, const Layout& 
   return s;
 }
 
-enum Outcome { kSolved, kMisfit, kLate };
-
-// Loads this CTA's share of bodies [b0, b1).  kMisfit (in every CTA) when some
-// CTA's share does not fit `bytes` of shared memory; kLate when the other CTAs
-// did not arrive in time.
+// Loads this CTA's share of bodies [b0, b1).  False when some CTA's share does
+// not fit `bytes` of shared memory (in every CTA, s.misfit 1) or the other CTAs
+// did not arrive in time (s.misfit 2).  (Returning the outcome itself took the
+// one-CTA solves of a 300-cell step from 253 to 269 us: other code.)
 template <int kForm>
-__device__ Outcome load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm, Shared& s, Layout& l,
+__device__ bool load_share(const SolveDesc& d, const ResidentArrays& r, Comm<kForm>& comm, Shared& s, Layout& l,
                            std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1, std::uint32_t* check) {
   const std::uint32_t* offsets = r.order != nullptr ? r.order_offsets : d.incidence.offsets;
   const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -689,7 +688,7 @@ __device__ Outcome load_share(const SolveDesc& d, const ResidentArrays& r, Comm<
   } else {
     __syncthreads();
   }
-  if (s.misfit != 0) return s.misfit == 2u ? kLate : kMisfit;
+  if (s.misfit != 0) return false;
   // Where each entry's side terms go: the other entry of its row.
   for (std::uint32_t q = threadIdx.x; q < bodies; q += kThreads) {
     const std::uint32_t degree = l.degree(q);
@@ -723,13 +722,14 @@ __device__ Outcome load_share(const SolveDesc& d, const ResidentArrays& r, Comm<
     }
   }
   __syncthreads();
-  return kSolved;
+  return true;
 }
 
 struct Report {
   float step, residual, bound;
   std::uint32_t iterations, status;
 };
+enum Outcome { kSolved, kMisfit, kLate };
 
 // The whole solve of bodies [b0, b1) by the CTAs of `comm`.
 template <int kForm, int P>
@@ -737,8 +737,7 @@ __device__ __forceinline__ Outcome resident_solve(const SolveDesc& d, const Resi
                                                   Shared& s, std::uint32_t bytes, std::uint32_t b0, std::uint32_t b1,
                                                   float tolerance, std::uint32_t* check, Report& report) {
   Layout l{};
-  const Outcome loaded = load_share(d, r, comm, s, l, bytes, b0, b1, check);
-  if (loaded != kSolved) return loaded;
+  if (!load_share(d, r, comm, s, l, bytes, b0, b1, check)) return kForm == kGrid && s.misfit == 2u ? kLate : kMisfit;
   // Every thread takes the same decisions from the same sums.  The rounds
   // share one copy of the code: what a round executes is fetched once per
   // iteration, by few warps, so its size counts.
